@@ -42,8 +42,8 @@ __device__ __forceinline__ int exponent(double x)
   return e - 1022;
 }
 
-// Fortran SCALE(x,e) = x*2^e, correctly rounded
-__device__ __forceinline__ double scale(double x, int e)
+// Fortran SCALE(x,e) = x*2^e, correctly rounded: the integer form, for every x and e
+static __device__ __noinline__ double scale_int(double x, int e)
 {
   const unsigned long long u = (unsigned long long)__double_as_longlong(x);
   const unsigned long long s = u & 0x8000000000000000ULL;
@@ -69,9 +69,28 @@ __device__ __forceinline__ double scale(double x, int e)
   return __longlong_as_double((long long)(s | q));
 }
 
-// project-own HYPOT: exact power-of-two scaling, h = sqrt(fma(a,a,b*b)), one Newton
+// 2^k, -1022 <= k <= 1023
+__device__ __forceinline__ double pow2(int k) { return __longlong_as_double((long long)(1023 + k) << 52); }
+
+// SCALE(x,e) by IEEE multiplications.  One multiplication by a power of two rounds once, as
+// SCALE does.  A power beyond 2^1023 or below 2^-1022 is split in two: scaling up, neither
+// multiplication rounds; scaling down, the first must give a normal number (x = 0, infinity
+// and NaN pass through both), so that only the second rounds.  The integer form takes what is
+// left: |e| > 2044, and operands below about 2^-1022 / 2^e1 scaled down past 2^-1022.
+// The 2x2 HSVDs scale a block to its largest binade and back (e about 1021 + the block's own
+// exponent), eleven times per block; with the integer form inlined at every use the 2x2 kernels
+// were bound by fetching their straight-line code: k_pivots took 9.7 us for 8 blocks.
+__device__ __forceinline__ double scale(double x, int e)
+{
+  const int e1 = (e > 1023) ? e - 1023 : ((e < -1022) ? e + 1022 : 0);
+  const int bx = (int)((unsigned long long)__double_as_longlong(x) >> 52) & 0x7FF;
+  if (e > 2044 || e < -2044 || (e1 < 0 && bx + e1 < 1 && x != 0.0)) return scale_int(x, e);
+  return __dmul_rn(__dmul_rn(x, pow2(e1)), pow2(e - e1));
+}
+
+// project-own HYPOT, the integer form, for every x and y: exact power-of-two scaling, h = sqrt(fma(a,a,b*b)), one Newton
 // step with the residual a^2 + b^2 - h^2 assembled from error-free products
-__device__ __forceinline__ double hypot2(double x, double y)
+static __device__ __noinline__ double hypot2_int(double x, double y)
 {
   const double ax = fabs(x), ay = fabs(y);
   if (isinf(ax) || isinf(ay)) return __longlong_as_double(0x7FF0000000000000LL);
@@ -89,6 +108,30 @@ __device__ __forceinline__ double hypot2(double x, double y)
   const double r = __dadd_rn(__dadd_rn(__dsub_rn(aa, hh), bb), __dsub_rn(__dadd_rn(ae, be), he));
   h = __dadd_rn(h, __ddiv_rn(r, __dadd_rn(h, h)));
   return scale(h, ea);
+}
+
+// project-own HYPOT with its scalings by IEEE multiplications: for a normal larger magnitude a
+// below 2^1023, a * 2^-ea, b * 2^-ea (b >= a 2^-55) are exact and h * 2^ea is rounded once, as
+// SCALE rounds it, so every value equals the integer form's bit for bit.  The rest (subnormal a, the
+// top binade, infinities, NaN) takes the integer form.
+__device__ __forceinline__ double hypot2(double x, double y)
+{
+  const double ax = fabs(x), ay = fabs(y);
+  const double a = (ax >= ay) ? ax : ay;
+  const double b = (ax >= ay) ? ay : ax;
+  const int ea = (int)((unsigned long long)__double_as_longlong(a) >> 52) - 1022;
+  // a NaN operand: either comparison puts y first, so b is x; a NaN a has ea = 1025
+  if (ea > 1023 || ea < -1021 || b != b) return hypot2_int(x, y);
+  if (ea - exponent(b) > 54 || b == 0.0) return a;
+  const double f = (ea == 1023) ? __longlong_as_double(1LL << 51) : pow2(-ea);  // 2^-1023 is subnormal
+  const double as = __dmul_rn(a, f), bs = __dmul_rn(b, f);
+  double h = sqrt(fma(as, as, __dmul_rn(bs, bs)));
+  const double hh = __dmul_rn(h, h), he = fma(h, h, -hh);
+  const double aa = __dmul_rn(as, as), ae = fma(as, as, -aa);
+  const double bb = __dmul_rn(bs, bs), be = fma(bs, bs, -bb);
+  const double r = __dadd_rn(__dadd_rn(__dsub_rn(aa, hh), bb), __dsub_rn(__dadd_rn(ae, be), he));
+  h = __dadd_rn(h, __ddiv_rn(r, __dadd_rn(h, h)));
+  return __dmul_rn(h, pow2(ea));
 }
 
 // hypot2 with the power-of-two scalings done by multiplication where that is exact: for
