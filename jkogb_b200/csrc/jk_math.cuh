@@ -427,8 +427,9 @@ __device__ __forceinline__ void dscalea(double A[4], int &s)
     for (int k = 0; k < 4; ++k) A[k] = scale(A[k], s);
 }
 
-// DHSVD2 (argument-checking form), src/D/dtransf.F90:614-683
-__device__ __forceinline__ void dhsvd2(double A[4], const int J0, const int J1, double U[4], double Z[4], double th1, int &info)
+// DHSVD2 (argument-checking form), src/D/dtransf.F90:614-683, for every input; out of line, it
+// serves what dhsvd2_near does not take
+static __device__ __noinline__ void dhsvd2_any(double A[4], const int J0, const int J1, double U[4], double Z[4], double th1, int &info)
 {
   double G[2] = { 0.0, 0.0 }, B[4] = { 0.0, 0.0, 0.0, 0.0 }, C[4] = { 0.0, 0.0, 0.0, 0.0 };
   int s;
@@ -459,6 +460,224 @@ __device__ __forceinline__ void dhsvd2(double A[4], const int J0, const int J1, 
 }
 
 // ------------------------------------------------------------------------
+// division and square root as straight-line code, for operands far from the ends of the
+// exponent range.  The compiler's division and square root are each followed by a branch to a
+// slow path, so that independent ones run one after another (136 and about 90 cycles each, and a
+// 2x2 HSVD has twenty-four divisions and six square roots: 7300 cycles); without the branch they
+// overlap, and divisions by the same number share its reciprocal.
+// ------------------------------------------------------------------------
+
+// 1/b rounded to nearest: the hardware's approximation (relative error 2^-23), one cubic and one
+// Newton step in fused arithmetic.  The Newton step rounds correctly except for a b whose
+// significand is all ones (1/b lies just above the midpoint that the step's result ties on), where
+// the next number up is the nearest; a cosine just below 1 is such a b.
+__device__ __forceinline__ double recip(double b)
+{
+  double y;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));
+  const double e = fma(-b, y, 1.0);
+  y = fma(y, fma(e, e, e), y);
+  y = fma(y, fma(-b, y, 1.0), y);
+  const long long ones = 0xFFFFFFFFFFFFFLL;
+  return __longlong_as_double(__double_as_longlong(y) + (((__double_as_longlong(b) & ones) == ones) ? 1 : 0));
+}
+
+// a/b rounded to nearest from y = recip(b): a quotient within an ulp, its exact remainder by one
+// fma, and the correction (P. Markstein, Computation of elementary functions on the IBM RISC
+// System/6000, IBM J. Res. Dev. 34, 1990).  a, b, a/b and the remainder must be normal; a zero
+// a keeps its sign.
+__device__ __forceinline__ double quot(double a, double b, double y)
+{
+  const double q = __dmul_rn(a, y);
+  const double r = fma(-b, q, a);
+  return (a == 0.0) ? q : fma(r, y, q);
+}
+
+// sqrt(x) rounded to nearest for normal x: the coupled iteration for sqrt(x) and 1/(2 sqrt(x))
+// from the hardware's approximation, then the remainder's correction (P. Markstein, Software
+// division and square root using Goldschmidt's algorithms, RNC6, 2004)
+__device__ __forceinline__ double root(double x)
+{
+  double y;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+  double g = __dmul_rn(x, y), h = __dmul_rn(0.5, y);
+  double r = fma(-g, h, 0.5);
+  g = fma(g, r, g);
+  h = fma(h, r, h);
+  r = fma(-g, h, 0.5);
+  g = fma(g, r, g);
+  h = fma(h, r, h);
+  return fma(fma(-g, g, x), h, g);
+}
+
+// hypot2 for a nonzero operand pair far from the ends of the exponent range: the same steps
+__device__ __forceinline__ double hypot2_near(double x, double y)
+{
+  const double ax = fabs(x), ay = fabs(y);
+  const double a = (ax >= ay) ? ax : ay;
+  const double b = (ax >= ay) ? ay : ax;
+  const int ea = (int)((unsigned long long)__double_as_longlong(a) >> 52) - 1022;
+  const int eb = (int)((unsigned long long)__double_as_longlong(b) >> 52) - 1022;
+  const double f = pow2(-ea);
+  const double as = __dmul_rn(a, f), bs = __dmul_rn(b, f);
+  double h = root(fma(as, as, __dmul_rn(bs, bs)));
+  const double hh = __dmul_rn(h, h), he = fma(h, h, -hh);
+  const double aa = __dmul_rn(as, as), ae = fma(as, as, -aa);
+  const double bb = __dmul_rn(bs, bs), be = fma(bs, bs, -bb);
+  const double r = __dadd_rn(__dadd_rn(__dsub_rn(aa, hh), bb), __dsub_rn(__dadd_rn(ae, be), he));
+  const double h2 = __dadd_rn(h, h);
+  h = __dadd_rn(h, quot(r, h2, recip(h2)));
+  return (ea - eb > 54) ? a : __dmul_rn(h, pow2(ea));
+}
+
+// whether the exponents of a 2x2 block's nonzero entries allow the straight-line forms: all
+// within 2^-200 of the largest, which lies in 2^(+-300), and no zero column
+__device__ __forceinline__ bool near_block(const double A[4])
+{
+  int hi = 0, lo = 0x7FF;
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const int e = (__double2hiint(A[k]) >> 20) & 0x7FF;
+    hi = max(hi, e);
+    lo = min(lo, (A[k] == 0.0) ? 0x7FF : e);
+  }
+  return hi >= 723 && hi <= 1323 && lo >= hi - 200 && (A[M11] != 0.0 || A[M21] != 0.0) && (A[M12] != 0.0 || A[M22] != 0.0);
+}
+
+// zero or at least 2^-300
+__device__ __forceinline__ bool near_ratio(double x) { return x == 0.0 || x >= 4.909093465297727e-91; }
+
+// DHSVD2 for the blocks that near_block takes: the operations of dhsvd2_any in the same order on
+// the unscaled block.  Scaling by a power of two changes no bit of any result while every
+// result stays normal, which near_block and the test of the two ratios x, y ensure (products
+// of three entries, U and Z stay above 2^-900).  Returns false, with nothing written, when the
+// block or its ratios do not allow it.
+__device__ __forceinline__ bool dhsvd2_near(double Ain[4], const int J0, const int J1, double Uo[4], double Zo[4], double th1, int &info_o)
+{
+  if (!near_block(Ain) || abs(J0) != 1 || abs(J1) != 1) return false;
+  double A[4] = { Ain[0], Ain[1], Ain[2], Ain[3] }, U[4] = { 1.0, 0.0, 0.0, 1.0 }, Z[4] = { 1.0, 0.0, 0.0, 1.0 };
+  int info;
+  // DHSVD2T, src/D/dtransf.F90:352-532
+  {
+    const bool d = (A[M21] == 0.0) && (A[M12] == 0.0);
+    const double c = hypot2_near(A[M11], A[M21]), s = hypot2_near(A[M12], A[M22]);
+    const bool p = (c < s);
+    const double r = p ? s : c;
+    if (p) {
+      dswap(A[M11], A[M12]); dswap(A[M21], A[M22]);
+      if (J0 == J1) { dswap(Z[M11], Z[M12]); dswap(Z[M21], Z[M22]); }
+    }
+    if (neg(A[M11])) { U[M11] = -U[M11]; U[M12] = -U[M12]; A[M12] = -A[M12]; A[M11] = -A[M11]; }
+    if (neg(A[M21])) { U[M21] = -U[M21]; U[M22] = -U[M22]; A[M22] = -A[M22]; A[M21] = -A[M21]; }
+    if (A[M11] < A[M21]) {
+      dswap(U[M11], U[M21]); dswap(U[M12], U[M22]);
+      dswap(A[M11], A[M21]); dswap(A[M12], A[M22]);
+    }
+    if (!d) {
+      const double t = quot(A[M21], A[M11], recip(A[M11]));
+      const double q = root(fma(t, t, 1.0)), y = recip(q);
+      const double u11 = fma(t, U[M21], U[M11]), u21 = fma(-t, U[M11], U[M21]);
+      const double u12 = fma(t, U[M22], U[M12]), u22 = fma(-t, U[M12], U[M22]);
+      const double a1 = fma(t, A[M22], A[M12]), a2 = fma(-t, A[M12], A[M22]);
+      U[M11] = quot(u11, q, y); U[M21] = quot(u21, q, y); U[M12] = quot(u12, q, y); U[M22] = quot(u22, q, y);
+      A[M12] = quot(a1, q, y); A[M22] = quot(a2, q, y);
+    }
+    A[M11] = r;
+    A[M21] = 0.0;
+    if ((J0 != J1) && p) {
+      dswap(A[M11], A[M12]); dswap(A[M21], A[M22]);
+      dswap(U[M11], U[M21]); dswap(U[M12], U[M22]);
+      dswap(A[M11], A[M21]); dswap(A[M12], A[M22]);
+      if (neg(A[M21])) { Z[M11] = -Z[M11]; Z[M21] = -Z[M21]; A[M11] = -A[M11]; A[M21] = -A[M21]; }
+      if (neg(A[M11])) { U[M11] = -U[M11]; U[M12] = -U[M12]; A[M11] = -A[M11]; }
+    }
+    else {
+      if (neg(A[M12])) { Z[M12] = -Z[M12]; Z[M22] = -Z[M22]; A[M22] = -A[M22]; A[M12] = -A[M12]; }
+      if (neg(A[M22])) { U[M21] = -U[M21]; U[M22] = -U[M22]; A[M22] = -A[M22]; }
+    }
+    info = d ? 0 : 1;
+  }
+  if (info) {
+    // KHSVD2, src/shared/ktransf.F90:15-217, with the block unscaled.  An upper triangle
+    // [a, b; 0, c] takes T (equal signs) or U, a lower one [c, 0; b, a] (unequal signs) L.
+    const bool upper = (A[M21] == 0.0);
+    if (!upper && (A[M12] != 0.0 || J0 == J1)) return false;  // the argument errors of KHSVD2
+    const double a = upper ? A[M11] : A[M22], b = upper ? A[M12] : A[M21], c = upper ? A[M22] : A[M11];
+    const double ya = recip(a);
+    const double x = fmax(quot(b, a, ya), 0.0), y = fmax(quot(c, a, ya), 0.0);
+    if (!(a > 0.0) || !(b >= 0.0) || !(c >= 0.0) || !near_ratio(x) || !near_ratio(y)) return false;
+    const bool tg = (J0 == J1);
+    const double nu = __dmul_rn(__dmul_rn(fmin(x, y), 2.0), fmax(x, y));
+    const double de = fma(tg ? __dsub_rn(x, y) : __dsub_rn(y, x), __dadd_rn(x, y), 1.0);
+    if (!(de >= 8.881784197001252e-16)) return false;  // (unequal signs: also a vanishing or negative denominator)
+    double t2 = fmin(quot(nu, de, recip(de)), twof());
+    if (t2 > 1e100) return false;
+    const double q2 = __dadd_rn(1.0, root(fma(t2, t2, 1.0)));
+    double tu = quot(t2, q2, recip(q2));  // |tan| of the left rotation
+    double tz, cz;
+    const double cu = root(fma(tu, tu, 1.0));
+    if (tg) {
+      tz = fma(y, tu, x);
+      cz = root(fma(tz, tz, 1.0));
+    }
+    else {
+      if (upper) tu = -tu;
+      tz = fma(y, tu, upper ? x : -x);
+      if (upper) tz = -tz;
+      const double at = fabs(tz);
+      if (at >= 1.0) return false;  // INFO -10, -11
+      if (at >= th1) { tz = copysign(JK_TH1FIX, tz); info += 8; }
+      cz = root(fma(-tz, tz, 1.0));
+    }
+    const double yu = recip(cu), yz = recip(cz);
+    double g0 = 0.0, g1 = 0.0;
+    if (!(info & 8)) {
+      const double w = tg ? quot(cz, cu, yu) : quot(cu, cz, yz);
+      const double m = __dmul_rn(tg ? a : c, w), dv = quot(tg ? c : a, w, recip(w));
+      // T: G = (a w, c / w); U: (a / w, c w); L (a = A22, c = A11): (c w, a / w)
+      g0 = tg ? m : (upper ? dv : m);
+      g1 = tg ? dv : (upper ? m : dv);
+    }
+    // C2A(B, U) with B = [cu, tu; -tu, cu], A2C(Z, C) with C = [cz, C12; tz, cz]
+    const double c12 = tg ? -tz : tz;
+    const double u11 = fma(tu, U[M21], U[M11]), u21 = fma(-tu, U[M11], U[M21]);
+    const double u12 = fma(tu, U[M22], U[M12]), u22 = fma(-tu, U[M12], U[M22]);
+    U[M11] = quot(u11, cu, yu); U[M21] = quot(u21, cu, yu); U[M12] = quot(u12, cu, yu); U[M22] = quot(u22, cu, yu);
+    const double z11 = fma(Z[M12], tz, Z[M11]), z12 = fma(Z[M11], c12, Z[M12]);
+    const double z21 = fma(Z[M22], tz, Z[M21]), z22 = fma(Z[M21], c12, Z[M22]);
+    Z[M11] = quot(z11, cz, yz); Z[M12] = quot(z12, cz, yz); Z[M21] = quot(z21, cz, yz); Z[M22] = quot(z22, cz, yz);
+    if (!(info & 8)) { A[M11] = g0; A[M22] = g1; }
+    else {
+      const double a11 = fma(tu, A[M21], A[M11]), a21 = fma(-tu, A[M11], A[M21]);
+      const double a12 = fma(tu, A[M22], A[M12]), a22 = fma(-tu, A[M12], A[M22]);
+      A[M11] = quot(a11, cu, yu); A[M21] = quot(a21, cu, yu); A[M12] = quot(a12, cu, yu); A[M22] = quot(a22, cu, yu);
+      const double b11 = fma(A[M12], tz, A[M11]), b12 = fma(A[M11], c12, A[M12]);
+      const double b21 = fma(A[M22], tz, A[M21]), b22 = fma(A[M21], c12, A[M22]);
+      A[M11] = quot(b11, cz, yz); A[M12] = quot(b12, cz, yz); A[M21] = quot(b21, cz, yz); A[M22] = quot(b22, cz, yz);
+    }
+  }
+  dhsvd2s(A, J0, J1, U, Z, info);
+#pragma unroll
+  for (int k = 0; k < 4; ++k) { Ain[k] = A[k]; Uo[k] = U[k]; Zo[k] = Z[k]; }
+  info_o = info;
+  return true;
+}
+
+// DHSVD2, src/D/dtransf.F90:614-683
+__device__ __forceinline__ void dhsvd2(double A[4], const int J0, const int J1, double U[4], double Z[4], double th1, int &info)
+{
+  if (!dhsvd2_near(A, J0, J1, U, Z, th1, info)) {
+    // copies, so that the caller's arrays stay in registers beside the call
+    double a[4] = { A[0], A[1], A[2], A[3] }, u[4] = { 0.0, 0.0, 0.0, 0.0 }, z[4] = { 0.0, 0.0, 0.0, 0.0 };
+    int inf = 0;
+    dhsvd2_any(a, J0, J1, u, z, th1, inf);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) { A[k] = a[k]; U[k] = u[k]; Z[k] = z[k]; }
+    info = inf;
+  }
+}
+
+// ------------------------------------------------------------------------
 // the branch-selected scaled rotation of BA / AB / ABODNDF2
 // (src/D/dtransf.F90:121-348):  with flags c1, c2, ratios r1, r2, multipliers m1, m2,
 //   xx = c1 ? fma(r1, y, x) : fma(r1, x, y);   x' = xx * m1
@@ -469,16 +688,32 @@ struct Rot {
   int c1, c2;
 };
 
+// n1/d1 and n2/d2, as straight-line code when the operands allow it
+__device__ __forceinline__ void div2(double n1, double d1, double n2, double d2, double &r1, double &r2)
+{
+  const int e1 = (__double2hiint(d1) >> 20) & 0x7FF, e2 = (__double2hiint(d2) >> 20) & 0x7FF;
+  const double lim = 1.9010857885610293e-211;  // 2^-700
+  const bool ok = (n1 == 0.0 || fabs(n1) >= lim) && (n2 == 0.0 || fabs(n2) >= lim) && imin(e1, e2) >= 723 &&
+                  max(e1, e2) <= 1323 && fabs(n1) <= fabs(d1) && fabs(n2) <= fabs(d2);
+  if (ok) {
+    r1 = quot(n1, d1, recip(d1));
+    r2 = quot(n2, d2, recip(d2));
+  }
+  else {
+    r1 = __ddiv_rn(n1, d1);
+    r2 = __ddiv_rn(n2, d2);
+  }
+}
+
 // coefficients of BA(B, ...) (rows), src/D/dtransf.F90:140-182
 __device__ __forceinline__ Rot rot_ba(const double B[4])
 {
   Rot t;
   t.c1 = (fabs(B[M11]) >= fabs(B[M12]));
   t.c2 = (fabs(B[M22]) >= fabs(B[M21]));
-  t.r1 = t.c1 ? __ddiv_rn(B[M12], B[M11]) : __ddiv_rn(B[M11], B[M12]);
-  t.r2 = t.c2 ? __ddiv_rn(B[M21], B[M22]) : __ddiv_rn(B[M22], B[M21]);
   t.m1 = t.c1 ? B[M11] : B[M12];
   t.m2 = t.c2 ? B[M22] : B[M21];
+  div2(t.c1 ? B[M12] : B[M11], t.m1, t.c2 ? B[M21] : B[M22], t.m2, t.r1, t.r2);
   return t;
 }
 
@@ -488,10 +723,9 @@ __device__ __forceinline__ Rot rot_ab(const double B[4])
   Rot t;
   t.c1 = (fabs(B[M11]) >= fabs(B[M21]));
   t.c2 = (fabs(B[M22]) >= fabs(B[M12]));
-  t.r1 = t.c1 ? __ddiv_rn(B[M21], B[M11]) : __ddiv_rn(B[M11], B[M21]);
-  t.r2 = t.c2 ? __ddiv_rn(B[M12], B[M22]) : __ddiv_rn(B[M22], B[M12]);
   t.m1 = t.c1 ? B[M11] : B[M21];
   t.m2 = t.c2 ? B[M22] : B[M12];
+  div2(t.c1 ? B[M21] : B[M11], t.m1, t.c2 ? B[M12] : B[M22], t.m2, t.r1, t.r2);
   return t;
 }
 
