@@ -202,21 +202,6 @@ __device__ __forceinline__ void scan_rows_real(const double *xs, const double *y
   }
 }
 
-__device__ __forceinline__ void scan_rows_cplx(const double2 *xs, const double2 *ys, int rows, int i0, int p, int q, const ZRot &t, double &d)
-{
-  for (int r = 0; r < rows; ++r) {
-    double2 x = xs[r], y = ys[r];
-    const double2 x0 = x, y0 = y;
-    zrot_apply_ab(t, x, y);
-    const int i = i0 + r;
-    if (i != p && i != q) {
-      const double axi = zabs(x0), axx = zabs(x), ayi = zabs(y0), ayy = zabs(y);
-      d = fma(__dsub_rn(axi, axx), __dadd_rn(axi, axx), d);
-      d = fma(__dsub_rn(ayi, ayy), __dadd_rn(ayi, ayy), d);
-    }
-  }
-}
-
 // ---------------------------------------------------------------------------
 // the real hyperbolic weights, pipelined: a block owns 16 "+" columns x 32 "-"
 // columns; each thread owns two pairs sharing its "+" column (two independent fma
@@ -553,17 +538,31 @@ __global__ void k_absmat(const State *st, const double2 *__restrict__ A, long lo
     mag[k] = zabs(A[k]);
 }
 
+// hypot2 out of line: the rare operands hypot2_near does not take
+__device__ __noinline__ double hypot2_call(double x, double y) { return hypot2(x, y); }
+
+// whether hypot2_near takes a row's entry: the larger part within 2^(+-998) (a NaN in the
+// other part passes through), or both parts zero
+__device__ __forceinline__ bool scan_near(double2 a)
+{
+  const double u = fmax(fabs(a.x), fabs(a.y));
+  return (u >= 3.7e-301 && u <= 2.6e300) || u == 0.0;
+}
+
 // ABODNZF2's row scan (src/Z/ztransf.F90:452-637) with the magnitudes of the unrotated
-// entries taken from xa, ya: the same operations in the same order as scan_rows_cplx
+// entries taken from xa, ya: the same operations in the same order
 __device__ __forceinline__ void scan_rows_cplx_mag(const double2 *xs, const double2 *ys, const double *xa, const double *ya,
                                                    int rows, int i0, int p, int q, const ZRot &t, double &d)
 {
   for (int r = 0; r < rows; ++r) {
     double2 x = xs[r], y = ys[r];
     zrot_apply_ab(t, x, y);
+    double axx, ayy;
+    if (scan_near(x) && scan_near(y)) { axx = zabs_near(x); ayy = zabs_near(y); }
+    else { axx = hypot2_call(x.x, x.y); ayy = hypot2_call(y.x, y.y); }
     const int i = i0 + r;
     if (i != p && i != q) {
-      const double axi = xa[r], axx = zabs(x), ayi = ya[r], ayy = zabs(y);
+      const double axi = xa[r], ayi = ya[r];
       d = fma(__dsub_rn(axi, axx), __dadd_rn(axi, axx), d);
       d = fma(__dsub_rn(ayi, ayy), __dadd_rn(ayi, ayy), d);
     }
@@ -694,49 +693,50 @@ struct ZHypPar {
 };
 static_assert(ZTP * ZTM * sizeof(ZHypPar) <= kZSmem, "a tile's scan parameters must fit in the row buffer");
 
-// hypot2 out of line: the rare operands hypot2_fast does not take
-__device__ __noinline__ double hypot2_call(double x, double y) { return hypot2(x, y); }
-
-// (the range test is repeated inside hypot2_fast; a form that tests once, with the fast path
-// split out, measured 2% slower in k_hyp_z_pm: more registers spilled)
-__device__ __forceinline__ double zabs_scan(double2 a)
-{
-  const double ax = fabs(a.x), ay = fabs(a.y);
-  const double u = (ax >= ay) ? ax : ay;
-  const double v = (ax >= ay) ? ay : ax;
-  const int bu = (int)((unsigned long long)__double_as_longlong(u) >> 52);
-  const int bv = (int)((unsigned long long)__double_as_longlong(v) >> 52);
-  if (bu >= 23 && bu <= 2021 && bv >= 1 && ax == ax && ay == ay) return hypot2_fast(a.x, a.y);
-  return hypot2_call(a.x, a.y);
-}
-
 // rows 0 .. rows - 1 of a chunk for K pairs per thread (ABODNZF2, src/Z/ztransf.F90:452-637:
 // the rotation, then the magnitudes of the rotated and of the unrotated entries, rows p and
 // q skipped).  FAST: every pair of the block takes the first branch (c1, c2); otherwise
-// each pair selects its branches.  Slots without a scan compute nothing.
+// each pair selects its branches.  Slots without a scan compute garbage that is never stored.
+// The 2 K magnitudes of a row run as one straight line of code (hypot2_near), so that their
+// square roots and divisions overlap; with the compiler's, whose slow paths are branches, the
+// chains ran one after another.
 template <int K, bool FAST>
 __device__ __forceinline__ void zscan_rows(const double2 *const *xs, const double2 *const *ys, const double *const *xa,
                                            const double *const *ya, int rows, const int *pl, const int *ql,
-                                           const int *fl, const ZRot *t, double *d)
+                                           const ZRot *t, double *d)
 {
 #pragma unroll 1
   for (int r = 0; r < rows; ++r) {
+    double2 x[K], y[K];
+    double ax[K], ay[K];
+    bool near = true;
 #pragma unroll
     for (int k = 0; k < K; ++k) {
-      if (!(fl[k] & 1)) continue;
-      double2 x = xs[k][r], y = ys[k][r];
+      x[k] = xs[k][r];
+      y[k] = ys[k][r];
       if (FAST) {
-        const double2 xx = zzfma(y, t[k].r1, x), yy = zzfma(x, t[k].r2, y);
-        x = zzmul(xx, t[k].m1);
-        y = zzmul(yy, t[k].m2);
+        const double2 xx = zzfma(y[k], t[k].r1, x[k]), yy = zzfma(x[k], t[k].r2, y[k]);
+        x[k] = zzmul(xx, t[k].m1);
+        y[k] = zzmul(yy, t[k].m2);
       }
-      else zrot_apply_ab(t[k], x, y);
-      if (r != pl[k] && r != ql[k]) {
-        const double axi = xa[k][r], axx = zabs_scan(x), ayi = ya[k][r], ayy = zabs_scan(y);
-        d[k] = fma(__dsub_rn(axi, axx), __dadd_rn(axi, axx), d[k]);
-        d[k] = fma(__dsub_rn(ayi, ayy), __dadd_rn(ayi, ayy), d[k]);
-      }
+      else zrot_apply_ab(t[k], x[k], y[k]);
+      near = near && scan_near(x[k]) && scan_near(y[k]);
     }
+    if (near) {
+#pragma unroll
+      for (int k = 0; k < K; ++k) { ax[k] = zabs_near(x[k]); ay[k] = zabs_near(y[k]); }
+    }
+    else {
+#pragma unroll
+      for (int k = 0; k < K; ++k) { ax[k] = hypot2_call(x[k].x, x[k].y); ay[k] = hypot2_call(y[k].x, y[k].y); }
+    }
+#pragma unroll
+    for (int k = 0; k < K; ++k)
+      if (r != pl[k] && r != ql[k]) {
+        const double axi = xa[k][r], ayi = ya[k][r];
+        d[k] = fma(__dsub_rn(axi, ax[k]), __dadd_rn(axi, ax[k]), d[k]);
+        d[k] = fma(__dsub_rn(ayi, ay[k]), __dadd_rn(ayi, ay[k]), d[k]);
+      }
   }
 }
 
@@ -891,12 +891,12 @@ k_hyp_z_pm(const State *st, const double2 *__restrict__ A, const double *__restr
       qr[k] = qv[k] - i0;
     }
     if (allfast) {
-      if (kw == 2) zscan_rows<2, true>(xs, ys, xa, ya, rows, pr, qr, fl, t, d);
-      else if (kw == 1) zscan_rows<1, true>(xs, ys, xa, ya, rows, pr, qr, fl, t, d);
+      if (kw == 2) zscan_rows<2, true>(xs, ys, xa, ya, rows, pr, qr, t, d);
+      else if (kw == 1) zscan_rows<1, true>(xs, ys, xa, ya, rows, pr, qr, t, d);
     }
     else {
-      if (kw == 2) zscan_rows<2, false>(xs, ys, xa, ya, rows, pr, qr, fl, t, d);
-      else if (kw == 1) zscan_rows<1, false>(xs, ys, xa, ya, rows, pr, qr, fl, t, d);
+      if (kw == 2) zscan_rows<2, false>(xs, ys, xa, ya, rows, pr, qr, t, d);
+      else if (kw == 1) zscan_rows<1, false>(xs, ys, xa, ya, rows, pr, qr, t, d);
     }
     __syncthreads();  // every thread is done with chunk c before chunk c + 2 overwrites it
   }
@@ -912,60 +912,22 @@ k_hyp_z_pm(const State *st, const double2 *__restrict__ A, const double *__restr
   }
 }
 
-template <typename T, int HP, int HM>
+template <int HP, int HM>
 __global__ void __launch_bounds__(HP * HM)
-k_weights_hyp(const State *st, const T *__restrict__ A, const int *__restrict__ plus, const int *__restrict__ minus,
+k_weights_hyp(const State *st, const double *__restrict__ A, const int *__restrict__ plus, const int *__restrict__ minus,
               int n_plus, int n_minus, double *__restrict__ Wm, int n)
 {
   if (st->stop || st->learned_step) return;  // a learned step ranks these pairs by the scorer
-  __shared__ T sP[HP][HR + 1];
-  __shared__ T sM[HM][HR + 1];
+  __shared__ double sP[HP][HR + 1];
+  __shared__ double sM[HM][HR + 1];
   const int tx = threadIdx.x % HP, ty = threadIdx.x / HP;
   const int ia = blockIdx.x * HP + tx, ib = blockIdx.y * HM + ty;
   const bool valid = (ia < n_plus) && (ib < n_minus);
   int p = 0, q = 0;
   bool scan = false, a_is_p = true;
   double d = 0.0, w = nan_w();
-  typename Tr<T>::R t;
-  if (valid) {
-    const int a = plus[ia], b = minus[ib];
-    a_is_p = (a < b);
-    p = a_is_p ? a : b;
-    q = a_is_p ? b : a;
-    const T app = A[(long long)p * n + p], aqp = A[(long long)p * n + q], apq = A[(long long)q * n + p], aqq = A[(long long)q * n + q];
-    if (may_transform(app, aqp, apq, aqq)) {
-      T A2[4] = { app, aqp, apq, aqq }, U2[4], Z2[4];
-      int info = 0;
-      const int jp = a_is_p ? 1 : -1;  // "+" column a, "-" column b
-      Tr<T>::hsvd2(A2, jp, -jp, U2, Z2, JK_TH1FIX, info);
-      if (info < 0) w = nan_w();
-      else if (!(info & 1)) w = 0.0;
-      else if (!(info & 4)) w = Tr<T>::magt(aqp, apq);
-      else {
-        // the two off-diagonal terms that start ABODNDF2 / ABODNZF2
-        const T aqp2 = (info & 8) ? A2[M21] : Tr<T>::zero();
-        const T apq2 = (info & 8) ? A2[M12] : Tr<T>::zero();
-        if constexpr (sizeof(T) == sizeof(double)) {
-          const double xq = *(const double *)&aqp, yp = *(const double *)&apq;
-          const double a1 = *(const double *)&aqp2, a2 = *(const double *)&apq2;
-          d = 0.0;
-          d = fma(__dsub_rn(xq, a1), __dadd_rn(xq, a1), d);
-          d = fma(__dsub_rn(yp, a2), __dadd_rn(yp, a2), d);
-        }
-        else {
-          const double2 xq = *(const double2 *)&aqp, yp = *(const double2 *)&apq;
-          const double2 a1 = *(const double2 *)&aqp2, a2 = *(const double2 *)&apq2;
-          d = 0.0;
-          d = fma(__dsub_rn(xq.x, a1.x), __dadd_rn(xq.x, a1.x), d);
-          d = fma(__dsub_rn(xq.y, a1.y), __dadd_rn(xq.y, a1.y), d);
-          d = fma(__dsub_rn(yp.x, a2.x), __dadd_rn(yp.x, a2.x), d);
-          d = fma(__dsub_rn(yp.y, a2.y), __dadd_rn(yp.y, a2.y), d);
-        }
-        t = Tr<T>::ab(Z2);
-        scan = true;
-      }
-    }
-  }
+  Rot t;
+  if (valid) scan = hyp_pair_setup(A, n, plus[ia], minus[ib], p, q, a_is_p, w, d, t);
   // a block-uniform exit when no thread of the tile scans
   if (!__syncthreads_or(scan)) {
     if (valid) {
@@ -993,12 +955,7 @@ k_weights_hyp(const State *st, const T *__restrict__ A, const int *__restrict__ 
       }
     }
     __syncthreads();
-    if (scan) {
-      const T *xs = a_is_p ? sP[tx] : sM[ty];
-      const T *ys = a_is_p ? sM[ty] : sP[tx];
-      if constexpr (sizeof(T) == sizeof(double)) scan_rows_real((const double *)xs, (const double *)ys, rows, i0, p, q, *(const Rot *)&t, d);
-      else scan_rows_cplx((const double2 *)xs, (const double2 *)ys, rows, i0, p, q, *(const ZRot *)&t, d);
-    }
+    if (scan) scan_rows_real(a_is_p ? sP[tx] : sM[ty], a_is_p ? sM[ty] : sP[tx], rows, i0, p, q, t, d);
     __syncthreads();
   }
   if (valid) {
@@ -2014,6 +1971,19 @@ static void hyp_d_launch(Workspace &w, const double *A, cudaStream_t s)
   k_hyp_pm<<<nt, SCAN_THREADS, smem, s>>>(w.st, A, w.plus, w.minus, w.n_plus, w.n_minus, w.n, w.Wm);
 }
 
+static void hyp_small_launch(const State *st, const double *A, const int *plus, const int *minus, int n_plus, int n_minus,
+                             double *W, int n, cudaStream_t s)
+{
+  if ((long long)n_plus * n_minus >= 256LL * 148 * 4) {
+    dim3 gh((n_plus + 15) / 16, (n_minus + 15) / 16);
+    k_weights_hyp<16, 16><<<gh, 256, 0, s>>>(st, A, plus, minus, n_plus, n_minus, W, n);
+  }
+  else {
+    dim3 gh((n_plus + 7) / 8, (n_minus + 7) / 8);
+    k_weights_hyp<8, 8><<<gh, 64, 0, s>>>(st, A, plus, minus, n_plus, n_minus, W, n);
+  }
+}
+
 template <typename T>
 static cudaError_t weights_t(Workspace &w, const T *A, cudaStream_t s)
 {
@@ -2021,39 +1991,25 @@ static cudaError_t weights_t(Workspace &w, const T *A, cudaStream_t s)
   dim3 bt(32, 8), gt((n + 31) / 32, (n + 7) / 8);
   k_weights_trig<T><<<gt, bt, 0, s>>>(w.st, A, w.J, w.Wm, n);
   if (w.n_plus > 0 && w.n_minus > 0) {
-    // the pipelined real kernel once its tiles fill the GPU; 16 x 16 / 8 x 8 tiles otherwise
-    if (sizeof(T) == sizeof(double) && (long long)w.n_plus * w.n_minus >= 512LL * 148 * 2) {
-      hyp_d_launch(w, (const double *)A, s);
+    const long long nh = (long long)w.n_plus * w.n_minus;
+    if constexpr (sizeof(T) == sizeof(double)) {
+      // the pipelined kernel once its tiles fill the GPU; 16 x 16 / 8 x 8 tiles otherwise
+      if (nh >= 512LL * 148 * 2) hyp_d_launch(w, A, s);
+      else hyp_small_launch(w.st, A, w.plus, w.minus, w.n_plus, w.n_minus, w.Wm, n, s);
     }
-    else if (sizeof(T) == sizeof(double2)) {
-      // complex: the magnitudes of all entries once, then the tiles
+    else {
+      // the magnitudes of all entries once, then the tiles
       const long long nn = (long long)n * n;
-      k_absmat<<<(unsigned)((nn + 255) / 256 < 4096 ? (nn + 255) / 256 : 4096), 256, 0, s>>>(w.st, (const double2 *)A, nn,
-                                                                                              w.mag);
-      if ((long long)w.n_plus * w.n_minus >= (long long)ZTP * ZTM * 148) {
+      k_absmat<<<(unsigned)((nn + 255) / 256 < 4096 ? (nn + 255) / 256 : 4096), 256, 0, s>>>(w.st, A, nn, w.mag);
+      if (nh >= (long long)ZTP * ZTM * 148) {
         // the pipelined tiles once they fill the GPU
         const int nt = ((w.n_plus + ZTP - 1) / ZTP) * ((w.n_minus + ZTM - 1) / ZTM);
-        k_hyp_z_pm<<<nt, ZTHREADS, kZSmem, s>>>(w.st, (const double2 *)A, w.mag, w.plus, w.minus, w.n_plus, w.n_minus, n,
-                                                w.Wm);
-      }
-      else if ((long long)w.n_plus * w.n_minus >= 256LL * 148 * 4) {
-        dim3 gh((w.n_plus + 15) / 16, (w.n_minus + 15) / 16);
-        k_weights_hyp_z<16, 16><<<gh, 256, 0, s>>>(w.st, (const double2 *)A, w.mag, w.plus, w.minus, w.n_plus, w.n_minus,
-                                                  w.Wm, n);
+        k_hyp_z_pm<<<nt, ZTHREADS, kZSmem, s>>>(w.st, A, w.mag, w.plus, w.minus, w.n_plus, w.n_minus, n, w.Wm);
       }
       else {
         dim3 gh((w.n_plus + 7) / 8, (w.n_minus + 7) / 8);
-        k_weights_hyp_z<8, 8><<<gh, 64, 0, s>>>(w.st, (const double2 *)A, w.mag, w.plus, w.minus, w.n_plus, w.n_minus,
-                                               w.Wm, n);
+        k_weights_hyp_z<8, 8><<<gh, 64, 0, s>>>(w.st, A, w.mag, w.plus, w.minus, w.n_plus, w.n_minus, w.Wm, n);
       }
-    }
-    else if ((long long)w.n_plus * w.n_minus >= 256LL * 148 * 4) {
-      dim3 gh((w.n_plus + 15) / 16, (w.n_minus + 15) / 16);
-      k_weights_hyp<T, 16, 16><<<gh, 256, 0, s>>>(w.st, A, w.plus, w.minus, w.n_plus, w.n_minus, w.Wm, n);
-    }
-    else {
-      dim3 gh((w.n_plus + 7) / 8, (w.n_minus + 7) / 8);
-      k_weights_hyp<T, 8, 8><<<gh, 64, 0, s>>>(w.st, A, w.plus, w.minus, w.n_plus, w.n_minus, w.Wm, n);
     }
   }
   return cudaGetLastError();
@@ -2277,16 +2233,7 @@ cudaError_t launch_weights_noalloc(int n, const double *A, const int *J, double 
   const int *dj = (const int *)(d + kScratchState), *dp = dj + kNoallocMaxN, *dm = dp + kNoallocMaxN;
   dim3 bt(32, 8), gt((n + 31) / 32, (n + 7) / 8);
   k_weights_trig<double><<<gt, bt, 0, s>>>(st, A, dj, W, n);
-  if (np > 0 && nm > 0) {
-    if ((long long)np * nm >= 256LL * 148 * 4) {
-      dim3 gh((np + 15) / 16, (nm + 15) / 16);
-      k_weights_hyp<double, 16, 16><<<gh, 256, 0, s>>>(st, A, dp, dm, np, nm, W, n);
-    }
-    else {
-      dim3 gh((np + 7) / 8, (nm + 7) / 8);
-      k_weights_hyp<double, 8, 8><<<gh, 64, 0, s>>>(st, A, dp, dm, np, nm, W, n);
-    }
-  }
+  if (np > 0 && nm > 0) hyp_small_launch(st, A, dp, dm, np, nm, W, n, s);
   return cudaGetLastError();
 }
 

@@ -134,35 +134,6 @@ __device__ __forceinline__ double hypot2(double x, double y)
   return __dmul_rn(h, pow2(ea));
 }
 
-// hypot2 with the power-of-two scalings done by multiplication where that is exact: for
-// finite x, y whose larger magnitude a is normal with exponent in [-999, 999] and whose
-// smaller one b is normal, a * 2^-ea, b * 2^-ea and h * 2^ea are normal numbers (or, for
-// the last, h * 2^ea is rounded once, as SCALE rounds), so every value equals hypot2's bit
-// for bit; everything else goes through hypot2.  The same operations in the same order.
-__device__ __forceinline__ double hypot2_fast(double x, double y)
-{
-  const double ax = fabs(x), ay = fabs(y);
-  const double a = (ax >= ay) ? ax : ay;
-  const double b = (ax >= ay) ? ay : ax;
-  const int ba = (int)((unsigned long long)__double_as_longlong(a) >> 52);
-  const int bb = (int)((unsigned long long)__double_as_longlong(b) >> 52);
-  if (ba >= 23 && ba <= 2021 && bb >= 1 && ax == ax && ay == ay) {
-    const int ea = ba - 1022;
-    if (ea - (bb - 1022) > 54) return a;
-    const double f = __longlong_as_double((long long)(1023 - ea) << 52);
-    const double g = __longlong_as_double((long long)(1023 + ea) << 52);
-    const double as = __dmul_rn(a, f), bs = __dmul_rn(b, f);
-    double h = sqrt(fma(as, as, __dmul_rn(bs, bs)));
-    const double hh = __dmul_rn(h, h), he = fma(h, h, -hh);
-    const double aa = __dmul_rn(as, as), ae = fma(as, as, -aa);
-    const double bq = __dmul_rn(bs, bs), be = fma(bs, bs, -bq);
-    const double r = __dadd_rn(__dadd_rn(__dsub_rn(aa, hh), bq), __dsub_rn(__dadd_rn(ae, be), he));
-    h = __dadd_rn(h, __ddiv_rn(r, __dadd_rn(h, h)));
-    return __dmul_rn(h, g);
-  }
-  return hypot2(x, y);
-}
-
 // QUIET_NAN, src/shared/utils.F90:144-149
 __device__ __forceinline__ double quiet_nan(long long payload)
 {
@@ -547,6 +518,61 @@ __device__ __forceinline__ bool near_block(const double A[4])
 // zero or at least 2^-300
 __device__ __forceinline__ bool near_ratio(double x) { return x == 0.0 || x >= 4.909093465297727e-91; }
 
+// the factors of a triangle: the left rotation [cu, tu; -tu, cu] and the right one [cz, c12; tz, cz]
+// (each still to be divided by its cosine's inverse cu, cz), the reciprocals of cu, cz, the new
+// diagonal
+struct NearK {
+  double tu, tz, c12, cu, cz, yu, yz, g0, g1;
+};
+
+// KHSVD2, src/shared/ktransf.F90:15-217, on an unscaled nonnegative triangle.  An upper one
+// [a, b; 0, c] takes T (equal signs) or U, a lower one [c, 0; b, a] (unequal signs) L.  Returns
+// false for KHSVD2's argument errors, for INFO -10 and -11 and for operands that the
+// straight-line forms do not take.
+__device__ __forceinline__ bool khsvd2_near(const double A[4], const int J0, const int J1, double th1, int &info, NearK &k)
+{
+  const bool upper = (A[M21] == 0.0);
+  if (!upper && (A[M12] != 0.0 || J0 == J1)) return false;  // the argument errors of KHSVD2
+  const double a = upper ? A[M11] : A[M22], b = upper ? A[M12] : A[M21], c = upper ? A[M22] : A[M11];
+  const double ya = recip(a);
+  const double x = fmax(quot(b, a, ya), 0.0), y = fmax(quot(c, a, ya), 0.0);
+  if (!(a > 0.0) || !(b >= 0.0) || !(c >= 0.0) || !near_ratio(x) || !near_ratio(y)) return false;
+  const bool tg = (J0 == J1);
+  const double nu = __dmul_rn(__dmul_rn(fmin(x, y), 2.0), fmax(x, y));
+  const double de = fma(tg ? __dsub_rn(x, y) : __dsub_rn(y, x), __dadd_rn(x, y), 1.0);
+  if (!(de >= 8.881784197001252e-16)) return false;  // (unequal signs: also a vanishing or negative denominator)
+  double t2 = fmin(quot(nu, de, recip(de)), twof());
+  if (t2 > 1e100) return false;
+  const double q2 = __dadd_rn(1.0, root(fma(t2, t2, 1.0)));
+  double tu = quot(t2, q2, recip(q2));  // |tan| of the left rotation
+  double tz, cz;
+  const double cu = root(fma(tu, tu, 1.0));
+  if (tg) {
+    tz = fma(y, tu, x);
+    cz = root(fma(tz, tz, 1.0));
+  }
+  else {
+    if (upper) tu = -tu;
+    tz = fma(y, tu, upper ? x : -x);
+    if (upper) tz = -tz;
+    const double at = fabs(tz);
+    if (at >= 1.0) return false;  // INFO -10, -11
+    if (at >= th1) { tz = copysign(JK_TH1FIX, tz); info += 8; }
+    cz = root(fma(-tz, tz, 1.0));
+  }
+  const double yu = recip(cu), yz = recip(cz);
+  double g0 = 0.0, g1 = 0.0;
+  if (!(info & 8)) {
+    const double w = tg ? quot(cz, cu, yu) : quot(cu, cz, yz);
+    const double m = __dmul_rn(tg ? a : c, w), dv = quot(tg ? c : a, w, recip(w));
+    // T: G = (a w, c / w); U: (a / w, c w); L (a = A22, c = A11): (c w, a / w)
+    g0 = tg ? m : (upper ? dv : m);
+    g1 = tg ? dv : (upper ? m : dv);
+  }
+  k.tu = tu; k.tz = tz; k.c12 = tg ? -tz : tz; k.cu = cu; k.cz = cz; k.yu = yu; k.yz = yz; k.g0 = g0; k.g1 = g1;
+  return true;
+}
+
 // DHSVD2 for the blocks that near_block takes: the operations of dhsvd2_any in the same order on
 // the unscaled block.  Scaling by a power of two changes no bit of any result while every
 // result stays normal, which near_block and the test of the two ratios x, y ensure (products
@@ -598,55 +624,17 @@ __device__ __forceinline__ bool dhsvd2_near(double Ain[4], const int J0, const i
     info = d ? 0 : 1;
   }
   if (info) {
-    // KHSVD2, src/shared/ktransf.F90:15-217, with the block unscaled.  An upper triangle
-    // [a, b; 0, c] takes T (equal signs) or U, a lower one [c, 0; b, a] (unequal signs) L.
-    const bool upper = (A[M21] == 0.0);
-    if (!upper && (A[M12] != 0.0 || J0 == J1)) return false;  // the argument errors of KHSVD2
-    const double a = upper ? A[M11] : A[M22], b = upper ? A[M12] : A[M21], c = upper ? A[M22] : A[M11];
-    const double ya = recip(a);
-    const double x = fmax(quot(b, a, ya), 0.0), y = fmax(quot(c, a, ya), 0.0);
-    if (!(a > 0.0) || !(b >= 0.0) || !(c >= 0.0) || !near_ratio(x) || !near_ratio(y)) return false;
-    const bool tg = (J0 == J1);
-    const double nu = __dmul_rn(__dmul_rn(fmin(x, y), 2.0), fmax(x, y));
-    const double de = fma(tg ? __dsub_rn(x, y) : __dsub_rn(y, x), __dadd_rn(x, y), 1.0);
-    if (!(de >= 8.881784197001252e-16)) return false;  // (unequal signs: also a vanishing or negative denominator)
-    double t2 = fmin(quot(nu, de, recip(de)), twof());
-    if (t2 > 1e100) return false;
-    const double q2 = __dadd_rn(1.0, root(fma(t2, t2, 1.0)));
-    double tu = quot(t2, q2, recip(q2));  // |tan| of the left rotation
-    double tz, cz;
-    const double cu = root(fma(tu, tu, 1.0));
-    if (tg) {
-      tz = fma(y, tu, x);
-      cz = root(fma(tz, tz, 1.0));
-    }
-    else {
-      if (upper) tu = -tu;
-      tz = fma(y, tu, upper ? x : -x);
-      if (upper) tz = -tz;
-      const double at = fabs(tz);
-      if (at >= 1.0) return false;  // INFO -10, -11
-      if (at >= th1) { tz = copysign(JK_TH1FIX, tz); info += 8; }
-      cz = root(fma(-tz, tz, 1.0));
-    }
-    const double yu = recip(cu), yz = recip(cz);
-    double g0 = 0.0, g1 = 0.0;
-    if (!(info & 8)) {
-      const double w = tg ? quot(cz, cu, yu) : quot(cu, cz, yz);
-      const double m = __dmul_rn(tg ? a : c, w), dv = quot(tg ? c : a, w, recip(w));
-      // T: G = (a w, c / w); U: (a / w, c w); L (a = A22, c = A11): (c w, a / w)
-      g0 = tg ? m : (upper ? dv : m);
-      g1 = tg ? dv : (upper ? m : dv);
-    }
+    NearK k;
+    if (!khsvd2_near(A, J0, J1, th1, info, k)) return false;
+    const double tu = k.tu, tz = k.tz, c12 = k.c12, cu = k.cu, cz = k.cz, yu = k.yu, yz = k.yz;
     // C2A(B, U) with B = [cu, tu; -tu, cu], A2C(Z, C) with C = [cz, C12; tz, cz]
-    const double c12 = tg ? -tz : tz;
     const double u11 = fma(tu, U[M21], U[M11]), u21 = fma(-tu, U[M11], U[M21]);
     const double u12 = fma(tu, U[M22], U[M12]), u22 = fma(-tu, U[M12], U[M22]);
     U[M11] = quot(u11, cu, yu); U[M21] = quot(u21, cu, yu); U[M12] = quot(u12, cu, yu); U[M22] = quot(u22, cu, yu);
     const double z11 = fma(Z[M12], tz, Z[M11]), z12 = fma(Z[M11], c12, Z[M12]);
     const double z21 = fma(Z[M22], tz, Z[M21]), z22 = fma(Z[M21], c12, Z[M22]);
     Z[M11] = quot(z11, cz, yz); Z[M12] = quot(z12, cz, yz); Z[M21] = quot(z21, cz, yz); Z[M22] = quot(z22, cz, yz);
-    if (!(info & 8)) { A[M11] = g0; A[M22] = g1; }
+    if (!(info & 8)) { A[M11] = k.g0; A[M22] = k.g1; }
     else {
       const double a11 = fma(tu, A[M21], A[M11]), a21 = fma(-tu, A[M11], A[M21]);
       const double a12 = fma(tu, A[M22], A[M12]), a22 = fma(-tu, A[M12], A[M22]);
@@ -746,7 +734,6 @@ __device__ __forceinline__ double2 zneg(double2 a) { return make_double2(-a.x, -
 __device__ __forceinline__ bool zeq0(double2 a) { return (a.x == 0.0) && (a.y == 0.0); }
 __device__ __forceinline__ bool zne1(double2 a) { return (a.x != 1.0) || (a.y != 0.0); }
 __device__ __forceinline__ double zabs(double2 a) { return hypot2(a.x, a.y); }
-__device__ __forceinline__ double zabs_fast(double2 a) { return hypot2_fast(a.x, a.y); }
 
 // ZDFMA, src/Z/ztransf.F90:130-141
 __device__ __forceinline__ double2 zdfma(double a, double2 b, double2 c) { return zc(fma(a, b.x, c.x), fma(a, b.y, c.y)); }
@@ -783,5 +770,8 @@ __device__ __forceinline__ double2 zratio(double2 num, double2 den)
 {
   return (den.y == 0.0) ? zddiv(num, den.x) : zzdiv(num, den);
 }
+
+// zratio out of line
+static __device__ __noinline__ double2 zratio_call(double2 num, double2 den) { return zratio(num, den); }
 
 }  // namespace jk
