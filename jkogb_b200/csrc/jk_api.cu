@@ -46,11 +46,11 @@ inline int cuda_fail(cudaError_t e)
 
 int max_order(int cplx)
 {
-  // k_rotate keeps two columns of A in shared memory and k_select its matching state
-  // (227 KB per block each); the tie key packs p in 16 bits
+  // k_rotate keeps two columns of A in shared memory (227 KB per block); k_colsort sorts up to
+  // 4096 partners
   int n = (227 * 1024) / (2 * (cplx ? 16 : 8));
-  while (n > 3 && (select_smem(n) > 227 * 1024 || colsort_e(n) > 16)) --n;
-  return n < 65535 ? n : 65535;
+  while (n > 3 && colsort_e(n) > 16) --n;
+  return n;
 }
 
 // check the arguments as DSTEP_LOOP (src/D/dstep.F90:500-521) and DPROC_INIT / TRU do
@@ -103,7 +103,6 @@ int make_workspace(Guard &g, Workspace &w, int n, int cplx, const int *J, int tr
   CK(g.alloc(&w.piv, half * pivsz));
   CK(g.alloc(&w.rowrot, half * rrsz));
   CK(g.alloc(&w.list, (size_t)n * ((n + 7) & ~7) * sizeof(unsigned short)));
-  CK(g.alloc(&w.rank, (size_t)n * n * sizeof(unsigned short)));
   CK(g.alloc(&w.len, n * sizeof(int)));
   CK(g.alloc(&w.unp, (n + 1) * sizeof(int)));
   CK(g.alloc(&w.st, sizeof(State)));
@@ -291,8 +290,9 @@ int solver_advance(jk_solver *v, long long k)
     g_launches += (long long)per_sync * per_step;
     const State &h = *v->w.st_host;
     v->steps = h.steps;
-    if (h.stop == 1) { v->phase = 2; v->info = h.info; return 1; }
-    if (h.stop == 2) {
+    const int stop = h.stop ? h.stop : h.halt;
+    if (stop == 1) { v->phase = 2; v->info = h.info; return 1; }
+    if (stop == 2) {
       if (v->o.max_steps > 0 && v->steps >= v->o.max_steps) { v->phase = 2; v->info = JK_ERR_MAX_STEPS; return 1; }
       return 0;
     }

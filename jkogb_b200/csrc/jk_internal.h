@@ -11,6 +11,7 @@ namespace jk {
 // DSTEP_LOOP / DSTEP_EXEC (src/D/dstep.F90:376-604).
 struct State {
   int stop;    // 1 once the loop has ended; 2 while it waits at `limit` (resumable)
+  int halt;    // `stop` to be, known before the last step's rotations have run
   int steps;   // S: steps with effective transformations
   int info;    // final INFO (valid once stop)
   int sl;      // SL of the current step (selected pivots)
@@ -87,7 +88,6 @@ struct Workspace {
   void *piv;         // Piv<T>[n/2]
   void *rowrot;      // RowRot<T>[n/2]
   unsigned short *list;  // n x list_ld(n): the partners of every vertex, best first
-  unsigned short *rank;  // n x n: rank[v][u] = position of u in v's list
   int *len;              // valid entries of each list
   int *unp;              // columns outside the current pivot set
   State *st;         // device state
@@ -161,8 +161,7 @@ constexpr int kNoallocMaxN = 1024;
 cudaError_t launch_weights_noalloc(int n, const double *A, const int *J, double *W, cudaStream_t s);
 double fp64_peak();
 // kernel launches of one step (the graph body)
-constexpr int kStepLaunches = 6;
-size_t select_smem(int n);
+constexpr int kStepLaunches = 5;
 int colsort_e(int n);
 
 }  // namespace jk

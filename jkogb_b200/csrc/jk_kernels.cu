@@ -68,6 +68,7 @@ __global__ void k_state_init(State *st, int learned, int stall_k, int steps0)
 __global__ void k_set_limit(State *st, long long limit)
 {
   if (st->stop == 2) st->stop = 0;
+  if (st->halt == 2) st->halt = 0;
   st->limit = limit;
 }
 
@@ -149,7 +150,7 @@ __global__ void k_jztj(T *Z, const int *J, int n)
 template <typename T>
 __global__ void k_weights_trig(const State *st, const T *__restrict__ A, const int *__restrict__ J, double *__restrict__ Wm, int n)
 {
-  if (st->stop) return;
+  if (st->stop || st->halt) return;
   const int p = blockIdx.x * 32 + threadIdx.x, q = blockIdx.y * 8 + threadIdx.y;
   if (p >= n || q >= n || p >= q) return;
   const int s = J[p] + J[q];
@@ -362,7 +363,7 @@ __global__ void __launch_bounds__(SCAN_THREADS, 2)
 k_hyp_pm(const State *st, const double *__restrict__ A, const int *__restrict__ plus, const int *__restrict__ minus,
          int n_plus, int n_minus, int n, double *__restrict__ Wm)
 {
-  if (st->stop || st->learned_step) return;  // a learned step ranks these pairs by the scorer
+  if (st->stop || st->halt || st->learned_step) return;  // a learned step ranks these pairs by the scorer
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int TM = (n_minus + TW - 1) / TW;
   const int P0 = (blockIdx.x / TM) * TW, Q0 = (blockIdx.x % TM) * TW;
@@ -533,7 +534,7 @@ k_hyp_pm(const State *st, const double *__restrict__ A, const int *__restrict__ 
 // columns, and every pair of a column would otherwise compute it again
 __global__ void k_absmat(const State *st, const double2 *__restrict__ A, long long nn, double *__restrict__ mag)
 {
-  if (st->stop || st->learned_step) return;
+  if (st->stop || st->halt || st->learned_step) return;
   for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < nn; k += (long long)gridDim.x * blockDim.x)
     mag[k] = zabs(A[k]);
 }
@@ -578,7 +579,7 @@ __global__ void __launch_bounds__(HP * HM)
 k_weights_hyp_z(const State *st, const double2 *__restrict__ A, const double *__restrict__ mag, const int *__restrict__ plus,
                 const int *__restrict__ minus, int n_plus, int n_minus, double *__restrict__ Wm, int n)
 {
-  if (st->stop || st->learned_step) return;  // a learned step ranks these pairs by the scorer
+  if (st->stop || st->halt || st->learned_step) return;  // a learned step ranks these pairs by the scorer
   __shared__ double2 sP[HP][ZHR + 1];
   __shared__ double2 sM[HM][ZHR + 1];
   __shared__ double aP[HP][ZHR + 1];
@@ -750,7 +751,7 @@ __global__ void __launch_bounds__(ZTHREADS, 2)
 k_hyp_z_pm(const State *st, const double2 *__restrict__ A, const double *__restrict__ mag, const int *__restrict__ plus,
            const int *__restrict__ minus, int n_plus, int n_minus, int n, double *__restrict__ Wm)
 {
-  if (st->stop || st->learned_step) return;  // a learned step ranks these pairs by the scorer
+  if (st->stop || st->halt || st->learned_step) return;  // a learned step ranks these pairs by the scorer
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int TM = (n_minus + ZTM - 1) / ZTM;
   const int P0 = (blockIdx.x / TM) * ZTP, Q0 = (blockIdx.x % TM) * ZTM;
@@ -917,7 +918,7 @@ __global__ void __launch_bounds__(HP * HM)
 k_weights_hyp(const State *st, const double *__restrict__ A, const int *__restrict__ plus, const int *__restrict__ minus,
               int n_plus, int n_minus, double *__restrict__ Wm, int n)
 {
-  if (st->stop || st->learned_step) return;  // a learned step ranks these pairs by the scorer
+  if (st->stop || st->halt || st->learned_step) return;  // a learned step ranks these pairs by the scorer
   __shared__ double sP[HP][HR + 1];
   __shared__ double sM[HM][HR + 1];
   const int tx = threadIdx.x % HP, ty = threadIdx.x / HP;
@@ -985,14 +986,7 @@ k_weights_hyp(const State *st, const double *__restrict__ A, const int *__restri
 // in registers, shuffles and shared memory), so a round only moves each free
 // vertex's list pointer past partners matched meanwhile (k_select, one block).
 // ---------------------------------------------------------------------------
-#ifndef SEL_THREADS
-#define SEL_THREADS 1024  // threads of the one-block selection (a tuning knob)
-#endif
 #define SORT_THREADS 256
-#ifndef JK_SEL_CLUSTER_MIN_N
-#define JK_SEL_CLUSTER_MIN_N 512  // the cluster matching from this order on (a tuning knob)
-#endif
-constexpr int kSelClusterMinN = JK_SEL_CLUSTER_MIN_N;
 
 // descending bitonic sort of s2 (a power of two) records (k, t, i) in shared memory
 __device__ __forceinline__ void bitonic_desc(unsigned long long *k, unsigned *t, int *ix, int s2)
@@ -1026,7 +1020,7 @@ __host__ __device__ __forceinline__ int pow2ceil(int x)
 __host__ __device__ __forceinline__ int list_ld(int n) { return (n + 7) & ~7; }
 
 // rank the partners of vertex v = blockIdx.x: list[v][r] = r-th best partner,
-// rank[v][u] = position of u in that list, len[v] = number of partners.
+// len[v] = number of partners.
 // One 64-bit key per partner: the top 48 bits of the weight key, then the 16-bit
 // tie code (band << 1 | (u > v)), which orders the partners of v as (band, p) do
 // and also names u.  Partners whose keys agree in the top 48 bits are re-ordered by
@@ -1101,9 +1095,9 @@ __device__ __forceinline__ void block_sort_desc(unsigned long long (&k)[E], unsi
 
 template <int E>
 __global__ void __launch_bounds__(SORT_THREADS)
-k_colsort(const State *st, const double *__restrict__ Wm, int n, unsigned short *list, unsigned short *rank, int *len)
+k_colsort(const State *st, const double *__restrict__ Wm, int n, unsigned short *list, int *len)
 {
-  if (st->stop) return;
+  if (st->stop || st->halt) return;
   __shared__ unsigned long long sk[SORT_THREADS * E];
   __shared__ unsigned short slo[SORT_THREADS * E];  // low 16 bits of the sorted keys' weight keys
   __shared__ int s_cnt, s_warp[SORT_THREADS / 32];
@@ -1184,24 +1178,22 @@ k_colsort(const State *st, const double *__restrict__ Wm, int n, unsigned short 
     __syncthreads();
   }
   unsigned short *lv = list + (long long)v * list_ld(n);
-  unsigned short *rv = rank + (long long)v * n;
   for (int r = tid; r < cnt; r += blockDim.x) {
-    const int u = ckey_u(sk[r], v);
-    lv[r] = (unsigned short)u;
-    rv[u] = (unsigned short)r;
+    lv[r] = (unsigned short)ckey_u(sk[r], v);
   }
   if (tid == 0) len[v] = cnt;
 }
 
-// the end of the previous step: SL := MIN(SL, NL) and the loop test
-// (src/D/dstep.F90:442, 564-583), with the statistics of DSTEP_TRANSF
-// (src/D/dstep.F90:349-370) when tracing
+// the end of a step: SL := MIN(SL, NL) and the loop test (src/D/dstep.F90:442, 564-583), with
+// the statistics of DSTEP_TRANSF (src/D/dstep.F90:349-370) when tracing.  The outcome goes to
+// `stop`: the state's own, or its `halt` when the step's rotations are still to run.
 template <typename T>
-__device__ void end_of_step(State *st, const Piv<T> *piv, const int *J, Trace &tr)
+__device__ void end_of_step(State *st, const Piv<T> *piv, const int *J, Trace &tr, int *stop)
 {
   if (!st->pending || st->stop) return;
   st->pending = 0;
-  const int sl = st->sl, nl = st->nl, err = st->err;
+  // other blocks of the cluster counted NL and the error minimum
+  const int sl = st->sl, nl = *(volatile int *)&st->nl, err = *(volatile int *)&st->err;
   if (st->trace_on) {
     double tw = -0.0;
     int tg = 0, hy = 0;
@@ -1221,334 +1213,26 @@ __device__ void end_of_step(State *st, const Piv<T> *piv, const int *J, Trace &t
     for (int i = 0; i < sl; ++i)
       if (st->trace_npiv < st->trace_cap_piv) tr.piv[st->trace_npiv++] = make_int2(piv[i].p, piv[i].q);
   }
-  if (err < 0) { st->info = err; st->stop = 1; }
+  if (err < 0) { st->info = err; *stop = 1; }
   else if (((sl < nl) ? sl : nl) <= 0) {
     // only a step ranked by the exact weights ends the loop; a learned step without an
     // effective pivot is followed by an exact one
     if (st->retry) st->retry = 0;
-    else { st->info = st->steps; st->stop = 1; }
+    else { st->info = st->steps; *stop = 1; }
   }
   else {
     st->steps += 1;
     // the caller's step limit: the loop waits here, between two steps, and can go on
-    if (st->limit > 0 && st->steps >= st->limit) st->stop = 2;
+    if (st->limit > 0 && st->steps >= st->limit) *stop = 2;
   }
 }
 
-// The walk of one free vertex's ranked partner list from its pointer to the first free
-// partner (-1: none left).  The vertex's window holds list entries wbase .. wbase + 15 in
-// shared memory, two 8-entry segments; once the pointer leaves the first segment, the
-// window slides by one segment and the segment after it is fetched with cp.async (it lands
-// while the round's barriers pass).  A pointer that runs past the window reads 8 G entries
-// at a time with G independent 16-byte loads (a round takes as long as its longest walk, so
-// the round trips to memory count).  lv indexes the vertex's own state.
-template <int G>
-__device__ __forceinline__ int walk_list(const unsigned short *__restrict__ row, int lv, uint4 *win, unsigned short *ptr,
-                                         unsigned short *wbase, const unsigned short *slen, const unsigned char *ms)
-{
-  int p = ptr[lv], wb = wbase[lv];
-  const int L = slen[lv];
-  int found = -1;
-  while (p < L && found < 0) {
-    if (p < wb + 16) {
-      const int sg = (p - wb) >> 3;
-      const uint4 q4 = win[2 * lv + sg];
-      const unsigned w4[4] = { q4.x, q4.y, q4.z, q4.w };
-      const int a = wb + 8 * sg;
-#pragma unroll
-      for (int e = 0; e < 8; ++e) {
-        const int idx = a + e;
-        const int u = (int)((w4[e >> 1] >> ((e & 1) * 16)) & 0xFFFFu);
-        if (found < 0 && idx >= p && idx < L && !ms[u]) { found = u; p = idx; }
-      }
-      if (found < 0) p = a + 8;
-      continue;
-    }
-    // past the window: fetch the next 8 G entries with G independent loads
-    const int a = p & ~7;
-    uint4 g4[G];
-#pragma unroll
-    for (int j = 0; j < G; ++j)
-      if (a + 8 * j < L) g4[j] = *(const uint4 *)(row + a + 8 * j);
-#pragma unroll
-    for (int j = 0; j < G; ++j) {
-      if (found >= 0 || a + 8 * j >= L) continue;
-      const unsigned w4[4] = { g4[j].x, g4[j].y, g4[j].z, g4[j].w };
-#pragma unroll
-      for (int e = 0; e < 8; ++e) {
-        const int idx = a + 8 * j + e;
-        const int u = (int)((w4[e >> 1] >> ((e & 1) * 16)) & 0xFFFFu);
-        if (found < 0 && idx >= p && idx < L && !ms[u]) { found = u; p = idx; }
-      }
-      if (found >= 0) {
-        // the window restarts at the segment of the find
-        wb = a + 8 * j;
-        win[2 * lv] = g4[j];
-        if (j < G - 1 && wb + 8 < L) win[2 * lv + 1] = g4[j + 1];
-        else if (wb + 8 < L) cp_async16(&win[2 * lv + 1], row + wb + 8);
-      }
-    }
-    if (found < 0) p = a + 8 * G;
-  }
-  if (found < 0) p = L;
-  else if (p >= wb + 8 && p < wb + 16) {
-    // the first segment is used up: slide the window and fetch the segment after it
-    win[2 * lv] = win[2 * lv + 1];
-    wb += 8;
-    if (wb + 8 < L) cp_async16(&win[2 * lv + 1], row + wb + 8);
-  }
-  cp_async_commit();
-  ptr[lv] = (unsigned short)p;
-  wbase[lv] = (unsigned short)wb;
-  return found;
-}
-
-// a vertex's list state at the start of the matching
-__device__ __forceinline__ void walk_init(const unsigned short *__restrict__ row, int L, int lv, uint4 *win, unsigned short *ptr,
-                                          unsigned short *wbase, unsigned short *slen)
-{
-  ptr[lv] = 0;
-  wbase[lv] = 0;
-  slen[lv] = (unsigned short)L;
-  win[2 * lv] = ((const uint4 *)row)[0];
-  if (L > 8) win[2 * lv + 1] = ((const uint4 *)row)[1];
-}
-
-// By one block, after the matching: the matched pairs ranked by (weight key, tie key),
-// descending; the first N_2 are this step's pivots (the STEP array, rank order); the
-// columns outside them; the step's scalars.  ms is free scratch here.
+// one pivot: the 2x2 HSVD of DSTEP_TRANSF's first loop (src/D/dstep.F90:301-326), INFO, NL
+// (src/D/dstep.F90:337) and the BA coefficients every rotating block reads
 template <typename T>
-__device__ void select_finish(State *st, const double *__restrict__ Wm, int n, int n_2, int np, int rounds,
-                              const int2 *pairs, unsigned long long *skey, unsigned *stie, int *sidx, unsigned char *ms,
-                              Piv<T> *piv, int *unp, Trace &tr, int *s_nunp)
+__device__ __forceinline__ void pivot_hsvd(State *st, const T *__restrict__ A, const int *__restrict__ J, int n, int p, int q,
+                                           Piv<T> &pv, RowRot<T> &rr, int quirk)
 {
-  const int tid = threadIdx.x, nth = blockDim.x;
-  const int s2 = pow2ceil(n / 2 > 0 ? n / 2 : 1);
-  for (int i = tid; i < s2; i += nth) {
-    if (i < np) {
-      const int2 pr = pairs[i];
-      skey[i] = wkey(Wm[(long long)pr.x * n + pr.y]);
-      stie[i] = tkey(pr.x, pr.y);
-      sidx[i] = i;
-    }
-    else { skey[i] = 0ULL; stie[i] = 0u; sidx[i] = -1; }
-  }
-  __syncthreads();
-  bitonic_desc(skey, stie, sidx, s2);
-  const int sl = (np < n_2) ? np : n_2;
-  for (int v = tid; v < n; v += nth) ms[v] = 0;
-  __syncthreads();
-  for (int r = tid; r < sl; r += nth) {
-    const int2 pr = pairs[sidx[r]];
-    ms[pr.x] = 1;
-    ms[pr.y] = 1;
-    Piv<T> &pv = piv[r];
-    pv.p = pr.x;
-    pv.q = pr.y;
-    pv.w = Wm[(long long)pr.x * n + pr.y];
-  }
-  __syncthreads();
-  for (int v = tid; v < n; v += nth)
-    if (!ms[v]) unp[atomicAdd(s_nunp, 1)] = v;
-  __syncthreads();
-  if (tid == 0) {
-    st->sl = sl;
-    st->nl = 0;
-    st->err = 0;
-    st->nunp = *s_nunp;
-    st->rounds = rounds;
-    if (sl <= 0) {
-      // DSTEP_EXEC returns with SL = 0: the loop ends with INFO = S (src/D/dstep.F90:421, 575-582)
-      st->info = st->steps;
-      st->stop = 1;
-      if (st->trace_on && st->trace_steps < st->trace_cap_steps) {
-        const int s = st->trace_steps++;
-        tr.sl[s] = 0; tr.nl[s] = -1; tr.tw[s] = -0.0; tr.trig[s] = 0; tr.hyp[s] = 0; tr.rounds[s] = rounds;
-      }
-    }
-    else st->pending = 1;
-  }
-}
-
-// one block: the end of the previous step, the matching rounds, the ranking of the
-// matched pairs and the first N_2 of them (the pivots of this step, rank order),
-// and the columns outside the pivot set.
-// A round is two barriers: (A) every free vertex finds its best free partner, the first
-// free entry of its ranked list from its pointer on (walk_list); (B) mutual proposals
-// are matched.
-template <typename T>
-__global__ void __launch_bounds__(SEL_THREADS, 1)
-k_select(State *st, const double *__restrict__ Wm, const int *__restrict__ J, int n, int n_2,
-         const unsigned short *__restrict__ list, const int *__restrict__ len, Piv<T> *piv, int *unp, Trace tr)
-{
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  const int s2 = pow2ceil(n / 2 > 0 ? n / 2 : 1);
-  unsigned long long *skey = (unsigned long long *)smem_raw;  // [s2]
-  unsigned *stie = (unsigned *)(skey + s2);                   // [s2]
-  int *sidx = (int *)(stie + s2);                             // [s2]
-  int2 *pairs = (int2 *)(sidx + s2);                          // [n/2 + 1]
-  uint4 *win = (uint4 *)(pairs + (n / 2 + 1) + ((n / 2 + 1) & 1)); // [n][2]: list entries wbase .. wbase + 15
-  int *best = (int *)(win + 2 * n);                           // [n]
-  unsigned short *ptr = (unsigned short *)(best + n);         // [n]
-  unsigned short *wbase = ptr + n;                            // [n]
-  unsigned short *slen = wbase + n;                           // [n]
-  unsigned char *ms = (unsigned char *)(slen + n);            // [n]: 0 free, 1 matched, 2 retired
-  __shared__ int s_stop, s_cnt, s_nunp, s_rounds;
-
-  const int tid = threadIdx.x, nth = blockDim.x, ld = list_ld(n);
-  if (tid == 0) {
-    end_of_step<T>(st, piv, J, tr);
-    s_stop = st->stop;
-    s_cnt = 0; s_nunp = 0; s_rounds = 0;
-  }
-  __syncthreads();
-  if (s_stop) return;
-  for (int v = tid; v < n; v += nth) {
-    ms[v] = 0;
-    walk_init(list + (long long)v * ld, len[v], v, win, ptr, wbase, slen);
-  }
-  __syncthreads();
-
-  for (int round = 0; round <= n / 2 + 1; ++round) {
-    cp_async_wait<0>();  // this thread's window refills of the last round
-    // phase A: the best free partner of every free vertex
-    for (int v = tid; v < n; v += nth)
-      if (!ms[v]) best[v] = walk_list<4>(list + (long long)v * ld, v, win, ptr, wbase, slen, ms);
-    __syncthreads();
-    // phase B: mutual proposals are matched; a vertex without a candidate retires
-    int got = 0;
-    for (int v = tid; v < n; v += nth) {
-      if (ms[v]) continue;
-      const int u = best[v];
-      if (u < 0) { ms[v] = 2; continue; }
-      if (v < u && best[u] == v) {
-        ms[v] = 1;
-        ms[u] = 1;
-        pairs[atomicAdd(&s_cnt, 1)] = make_int2(v, u);
-        got = 1;
-      }
-    }
-    if (tid == 0) s_rounds = round + 1;
-    if (!__syncthreads_or(got)) break;
-  }
-  cp_async_wait<0>();
-  select_finish<T>(st, Wm, n, n_2, s_cnt, s_rounds, pairs, skey, stie, sidx, ms, piv, unp, tr, &s_nunp);
-}
-
-// The same matching by a cluster of SEL_CLUSTER blocks sharing its state through
-// distributed shared memory (plain loads, stores and atomics; no multicast).  Block c owns
-// the vertices v = c (mod SEL_CLUSTER) and their list windows; every block keeps a replica
-// of every vertex's state (free, matched, retired), which phase B updates in all blocks.
-// A round: (A) every block walks its own free vertices' lists; cluster barrier; (B) a free
-// vertex whose best partner u proposes back (u's block holds best[u]) is matched with it,
-// the pair goes to block 0's list and both states change in every replica; cluster
-// barrier; every block reads the round's match count from block 0 and stops when it is 0.
-// Block 0 then ranks the matched pairs as the one-block kernel does.
-#define SEL_CLUSTER 8
-#define SEL_CTHREADS 256
-
-size_t select_cluster_smem(int n)
-{
-  const int s2 = pow2ceil(n / 2 > 0 ? n / 2 : 1);
-  const int np = (n / 2 + 1) + ((n / 2 + 1) & 1);
-  const int nl = (n + SEL_CLUSTER - 1) / SEL_CLUSTER;
-  return (size_t)s2 * (8 + 4 + 4) + (size_t)np * 8 + (size_t)nl * (32 + 4 + 2 + 2 + 2) + (size_t)n + 16;
-}
-
-template <typename T>
-__global__ void __cluster_dims__(SEL_CLUSTER, 1, 1) __launch_bounds__(SEL_CTHREADS, 1)
-k_select_cluster(State *st, const double *__restrict__ Wm, const int *__restrict__ J, int n, int n_2,
-                 const unsigned short *__restrict__ list, const int *__restrict__ len, Piv<T> *piv, int *unp, Trace tr)
-{
-  cg::cluster_group cluster = cg::this_cluster();
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  const int s2 = pow2ceil(n / 2 > 0 ? n / 2 : 1);
-  const int nl = (n + SEL_CLUSTER - 1) / SEL_CLUSTER;
-  unsigned long long *skey = (unsigned long long *)smem_raw;  // [s2]  (block 0)
-  unsigned *stie = (unsigned *)(skey + s2);                   // [s2]  (block 0)
-  int *sidx = (int *)(stie + s2);                             // [s2]  (block 0)
-  int2 *pairs = (int2 *)(sidx + s2);                          // [n/2 + 1]  (block 0)
-  uint4 *win = (uint4 *)(pairs + (n / 2 + 1) + ((n / 2 + 1) & 1)); // [nl][2]: own vertices' windows
-  int *best = (int *)(win + 2 * nl);                          // [nl]
-  unsigned short *ptr = (unsigned short *)(best + nl);        // [nl]
-  unsigned short *wbase = ptr + nl;                           // [nl]
-  unsigned short *slen = wbase + nl;                          // [nl]
-  unsigned char *ms = (unsigned char *)(slen + nl);           // [n]: replica of every vertex's state
-  __shared__ int s_stop, s_cnt, s_nunp, s_rounds, s_got[2];
-
-  const int tid = threadIdx.x, nth = blockDim.x, ld = list_ld(n);
-  const int c = (int)cluster.block_rank();
-  if (c == 0 && tid == 0) {
-    end_of_step<T>(st, piv, J, tr);
-    s_stop = st->stop;
-    s_cnt = 0; s_nunp = 0; s_rounds = 0; s_got[0] = 0; s_got[1] = 0;
-  }
-  for (int v = tid; v < n; v += nth) ms[v] = 0;
-  for (int lv = tid; lv * SEL_CLUSTER + c < n; lv += nth) {
-    const int v = lv * SEL_CLUSTER + c;
-    walk_init(list + (long long)v * ld, len[v], lv, win, ptr, wbase, slen);
-  }
-  int *got0 = cluster.map_shared_rank(s_got, 0);
-  int *cnt0 = cluster.map_shared_rank(&s_cnt, 0);
-  int2 *pairs0 = cluster.map_shared_rank(pairs, 0);
-  cluster.sync();
-  const int stop = *cluster.map_shared_rank(&s_stop, 0);
-  cluster.sync();  // every block has read block 0's flag
-  if (stop) return;
-
-  int rounds = 0;
-  for (int round = 0; round <= n / 2 + 1; ++round) {
-    cp_async_wait<0>();
-    // phase A: the best free partner of each own free vertex
-    for (int lv = tid; lv * SEL_CLUSTER + c < n; lv += nth) {
-      const int v = lv * SEL_CLUSTER + c;
-      if (!ms[v]) best[lv] = walk_list<16>(list + (long long)v * ld, lv, win, ptr, wbase, slen, ms);
-    }
-    cluster.sync();
-    // the next round's match count starts at zero (every block read it two barriers ago)
-    if (c == 0 && tid == 0) s_got[(round + 1) & 1] = 0;
-    // phase B: mutual proposals are matched; a vertex without a candidate retires
-    int got = 0;
-    for (int lv = tid; lv * SEL_CLUSTER + c < n; lv += nth) {
-      const int v = lv * SEL_CLUSTER + c;
-      if (ms[v]) continue;
-      const int u = best[lv];
-      if (u < 0) {
-        for (int b = 0; b < SEL_CLUSTER; ++b) *cluster.map_shared_rank(&ms[v], b) = 2;
-        continue;
-      }
-      if (v < u && *cluster.map_shared_rank(&best[u / SEL_CLUSTER], u % SEL_CLUSTER) == v) {
-        for (int b = 0; b < SEL_CLUSTER; ++b) {
-          *cluster.map_shared_rank(&ms[v], b) = 1;
-          *cluster.map_shared_rank(&ms[u], b) = 1;
-        }
-        pairs0[atomicAdd(cnt0, 1)] = make_int2(v, u);
-        got += 1;
-      }
-    }
-    if (got) atomicAdd(&got0[round & 1], got);
-    cluster.sync();
-    rounds = round + 1;
-    if (!got0[round & 1]) {
-      cluster.sync();  // every block has read the count before block 0 goes on alone
-      break;
-    }
-  }
-  cp_async_wait<0>();
-  if (c != 0) return;  // no block reads another's shared memory after the last barrier
-  select_finish<T>(st, Wm, n, n_2, s_cnt, rounds, pairs, skey, stie, sidx, ms, piv, unp, tr, &s_nunp);
-}
-
-// per pivot: the 2x2 HSVD of DSTEP_TRANSF's first loop (src/D/dstep.F90:301-326),
-// INFO, NL (src/D/dstep.F90:337) and the BA coefficients every rotating block reads
-template <typename T>
-__global__ void k_pivots(State *st, const T *__restrict__ A, const int *__restrict__ J, int n, Piv<T> *piv, RowRot<T> *rr, int quirk)
-{
-  if (st->stop) return;
-  const int r = blockIdx.x * blockDim.x + threadIdx.x;
-  if (r >= st->sl) return;
-  Piv<T> &pv = piv[r];
-  const int p = pv.p, q = pv.q;
   T B[4] = { A[(long long)p * n + p], A[(long long)p * n + q], A[(long long)q * n + p], A[(long long)q * n + q] };
   T V[4], W[4];
   int info = 0;
@@ -1570,7 +1254,254 @@ __global__ void k_pivots(State *st, const T *__restrict__ A, const int *__restri
   }
   else
     atomicMin(&st->err, info);
-  rr[r] = x;
+  rr = x;
+}
+
+// the pivots of a step by themselves (ID_NCP = 3; k_select does its own)
+template <typename T>
+__global__ void k_pivots(State *st, const T *__restrict__ A, const int *__restrict__ J, int n, Piv<T> *piv, RowRot<T> *rr, int quirk)
+{
+  if (st->stop) return;
+  const int r = blockIdx.x * blockDim.x + threadIdx.x;
+  if (r >= st->sl) return;
+  pivot_hsvd<T>(st, A, J, n, piv[r].p, piv[r].q, piv[r], rr[r], quirk);
+}
+
+// The greedy matching of one step, its first N_2 pairs and their 2x2 HSVDs, by a cluster of
+// C blocks (1 to 16) that share its state through distributed shared memory (plain loads, stores
+// and atomics; no multicast).
+//
+// Block c owns the vertices v = c (mod C); a warp owns up to 32 of them, one per lane (list
+// pointer, length and candidate in registers), and walks a list together: 64 entries per probe,
+// a ballot finds the first free partner.  The first lp entries of every own list lie in shared
+// memory (all of them up to N = 1200 or so), the rest is read from L2.  Every block keeps a replica of the
+// vertices' state (0 free, 1 matched).  A round:
+//   (A) a free vertex whose candidate is gone walks on to its best free partner, and notes it
+//       with the round's number in best[];
+//   (B) a vertex that moved in this round and whose candidate points back is matched with it
+//       (where both moved, the smaller index does it): the pair goes to block 0's list, both states
+//       to every replica.  Pairs of which neither moved were seen before.
+// A round without a match ends the matching.  Mutual best free partners are what the walk over the
+// sorted records takes, so the rounds rebuild its matching.
+//
+// What bounds it is the rounds' latency: two barriers and the longest walk.  With one
+// thread per list, 8 to 128 entries at a time (and a 16-entry window), a round cost 6.5 us at
+// N = 2048 (415 us a step on 8 blocks) and 2 us at N = 256 (43 us on one block).
+//
+// The order of the pivots matters only where the first N_2 of them are taken (np > N_2) or a
+// trace records them; otherwise they are left as matched and the sort is saved.
+constexpr int kSelThreads = 512;
+constexpr size_t kSelListBytes = 176 * 1024;  // shared memory for list prefixes
+
+// blocks per cluster: enough that a block's lists fit its shared memory and no warp walks for
+// many vertices; a larger cluster pays more per barrier
+static int select_cluster(int n)
+{
+  return (n <= 300) ? 1 : (n <= 600) ? 4 : (n <= 900) ? 8 : 16;
+}
+
+struct SelLayout {
+  int nl, lp;  // own vertices per block, list entries held in shared memory
+  size_t best, pairs, ms, total;
+  __host__ __device__ SelLayout(int n, int C)
+  {
+    nl = (n + C - 1) / C;
+    const int ld = list_ld(n);
+    const int fit = (int)(kSelListBytes / ((size_t)nl * 2)) & ~7;
+    lp = (ld < fit) ? ld : fit;
+    const size_t lists = (size_t)nl * lp * 2, sort = (size_t)pow2ceil(n / 2 > 0 ? n / 2 : 1) * 16;
+    best = (lists > sort) ? lists : sort;  // the final ranking reuses the lists' space
+    pairs = best + (((size_t)nl * 4 + 15) & ~(size_t)15);
+    ms = pairs + (size_t)(n / 2 + 1) * 8;
+    total = ms + (size_t)n + 16;
+  }
+};
+
+template <typename T>
+__global__ void __launch_bounds__(kSelThreads, 1)
+k_select(State *st, const double *__restrict__ Wm, const int *__restrict__ J, int n, int n_2,
+         const unsigned short *__restrict__ list, const int *__restrict__ len, const T *__restrict__ A, Piv<T> *piv,
+         RowRot<T> *rr, int *unp, Trace tr, int quirk, int early)
+{
+  cg::cluster_group cluster = cg::this_cluster();
+  const int C = (int)cluster.num_blocks(), c = (int)cluster.block_rank();
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const SelLayout L(n, C);
+  unsigned short *lists = (unsigned short *)smem_raw;          // [nl][lp]
+  unsigned *best = (unsigned *)(smem_raw + L.best);            // [nl]: candidate | round << 16
+  int2 *pairs = (int2 *)(smem_raw + L.pairs);                  // [n/2 + 1]  (block 0)
+  unsigned char *ms = (unsigned char *)(smem_raw + L.ms);      // [n]
+  __shared__ int s_cnt, s_nunp, s_got[3];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = kSelThreads / 32, ld = list_ld(n);
+  const bool solo = (C == 1);
+  auto sync = [&]() { if (solo) __syncthreads(); else cluster.sync(); };
+
+  // the end of the previous step, unless its own selection saw to it
+  if (!early) {
+    if (c == 0 && tid == 0) end_of_step<T>(st, piv, J, tr, &st->stop);
+    __threadfence();
+    sync();
+  }
+  if (*(volatile int *)&st->stop) return;
+  if (*(volatile int *)&st->halt) {
+    if (c == 0 && tid == 0) st->stop = st->halt;
+    return;
+  }
+  if (tid == 0) { s_cnt = 0; s_nunp = 0; s_got[0] = 0; s_got[1] = 0; s_got[2] = 0; }
+  // the lists' prefixes, 16 bytes at a time
+  {
+    const int pieces = L.lp / 8;
+    for (int k = tid; k < L.nl * pieces; k += kSelThreads) {
+      const int lv = k / pieces, e = k % pieces, v = lv * C + c;
+      if (v < n) cp_async16((uint4 *)(lists + (size_t)lv * L.lp) + e, (const uint4 *)(list + (long long)v * ld) + e);
+    }
+    cp_async_commit();
+  }
+  for (int v = tid; v < n; v += kSelThreads) ms[v] = 0;
+  // lane j of a warp owns vertex lv0 + j
+  const int K = (L.nl + nw - 1) / nw, lv0 = warp * K, mylv = lv0 + lane, myv = mylv * C + c;
+  bool active = (lane < K) && (mylv < L.nl) && (myv < n);
+  const int mylen = active ? len[myv] : 0;
+  int ptr = 0, cand = -1;
+  cp_async_wait<0>();
+  sync();
+  if (c == 0 && tid == 0) { st->nl = 0; st->err = 0; }
+
+  int rounds = 0;
+  for (int round = 0; round <= n / 2 + 1; ++round) {
+    // (A)
+    // (a slow thread may still read the last round's flag)
+    if (tid == 0) s_got[(round + 1) % 3] = 0;
+    bool moved = false;
+    if (active && ms[myv]) active = false;
+    unsigned need = __ballot_sync(0xFFFFFFFFu, active && (cand < 0 || ms[cand]));
+    while (need) {
+      const int sl = __ffs(need) - 1;
+      need &= need - 1;
+      const int p = __shfl_sync(0xFFFFFFFFu, ptr, sl), Lv = __shfl_sync(0xFFFFFFFFu, mylen, sl);
+      const unsigned short *row = lists + (size_t)(lv0 + sl) * L.lp;
+      const unsigned short *grow = list + (long long)((lv0 + sl) * C + c) * ld;
+      int found = -1, at = Lv;
+      for (int base = p & ~1; base < Lv; base += 64) {
+        const int idx = base + 2 * lane;
+        unsigned e = 0u;
+        if (idx < Lv) e = *(const unsigned *)((idx < L.lp ? row : grow) + idx);
+        const int u0 = (int)(e & 0xFFFFu), u1 = (int)(e >> 16);
+        const unsigned m0 = __ballot_sync(0xFFFFFFFFu, idx >= p && idx < Lv && !ms[u0]);
+        const unsigned m1 = __ballot_sync(0xFFFFFFFFu, idx + 1 < Lv && !ms[u1]);
+        if (m0 | m1) {
+          const int i0 = m0 ? 2 * (__ffs(m0) - 1) : 64, i1 = m1 ? 2 * (__ffs(m1) - 1) + 1 : 64;
+          const int i = (i0 < i1) ? i0 : i1;
+          found = __shfl_sync(0xFFFFFFFFu, (i & 1) ? u1 : u0, i >> 1);
+          at = base + i;
+          break;
+        }
+      }
+      if (lane == sl) {
+        ptr = at;
+        cand = found;
+        moved = (found >= 0);
+        if (found < 0) active = false;  // no free partner is left: retired
+        best[mylv] = (found < 0) ? 0xFFFFFFFFu : ((unsigned)found | ((unsigned)round << 16));
+      }
+    }
+    sync();
+    // (B)
+    if (moved) {
+      const unsigned b = solo ? best[cand] : *cluster.map_shared_rank(&best[cand / C], cand % C);
+      if ((int)(b & 0xFFFFu) == myv && ((int)(b >> 16) != round || myv < cand)) {
+        if (solo) {
+          ms[myv] = 1;
+          ms[cand] = 1;
+          s_got[round % 3] = 1;
+          pairs[atomicAdd(&s_cnt, 1)] = make_int2(min(myv, cand), max(myv, cand));
+        }
+        else {
+          for (int b2 = 0; b2 < C; ++b2) {
+            *cluster.map_shared_rank(&ms[myv], b2) = 1;
+            *cluster.map_shared_rank(&ms[cand], b2) = 1;
+            *cluster.map_shared_rank(&s_got[round % 3], b2) = 1;
+          }
+          cluster.map_shared_rank(pairs, 0)[atomicAdd(cluster.map_shared_rank(&s_cnt, 0), 1)] =
+              make_int2(min(myv, cand), max(myv, cand));
+        }
+      }
+    }
+    sync();
+    rounds = round + 1;
+    if (!s_got[round % 3]) break;
+  }
+
+  // the pairs are complete
+  const int np = solo ? s_cnt : *cluster.map_shared_rank(&s_cnt, 0);
+  const int sl = (np < n_2) ? np : n_2;
+  const bool ranked = (np > n_2) || st->trace_on || !A;
+  if (ranked) {
+    if (c == 0) {
+      const int s2 = pow2ceil(n / 2 > 0 ? n / 2 : 1);
+      unsigned long long *skey = (unsigned long long *)smem_raw;  // [s2]
+      unsigned *stie = (unsigned *)(skey + s2);                   // [s2]
+      int *sidx = (int *)(stie + s2);                             // [s2]
+      for (int i = tid; i < s2; i += kSelThreads) {
+        if (i < np) {
+          const int2 pr = pairs[i];
+          skey[i] = wkey(Wm[(long long)pr.x * n + pr.y]);
+          stie[i] = tkey(pr.x, pr.y);
+          sidx[i] = i;
+        }
+        else { skey[i] = 0ULL; stie[i] = 0u; sidx[i] = -1; }
+      }
+      __syncthreads();
+      bitonic_desc(skey, stie, sidx, s2);
+      for (int v = tid; v < n; v += kSelThreads) ms[v] = 0;
+      __syncthreads();
+      for (int r = tid; r < sl; r += kSelThreads) {
+        const int2 pr = pairs[sidx[r]];
+        ms[pr.x] = 1;
+        ms[pr.y] = 1;
+        piv[r].p = pr.x;
+        piv[r].q = pr.y;
+        piv[r].w = Wm[(long long)pr.x * n + pr.y];
+        if (A) pivot_hsvd<T>(st, A, J, n, pr.x, pr.y, piv[r], rr[r], quirk);
+      }
+      __syncthreads();
+    }
+  }
+  else {
+    const int2 *pairs0 = solo ? pairs : cluster.map_shared_rank(pairs, 0);
+    // warps of different blocks first, so that few pivots share an SM
+    for (int r = (warp * C + c) * 32 + lane; r < np; r += kSelThreads * C) {
+      const int2 pr = pairs0[r];
+      piv[r].p = pr.x;
+      piv[r].q = pr.y;
+      pivot_hsvd<T>(st, A, J, n, pr.x, pr.y, piv[r], rr[r], quirk);
+    }
+    __threadfence();
+    sync();  // every pivot is counted, and every block is done with block 0's list
+  }
+  if (c != 0) return;
+  // the columns outside the pivots
+  for (int v = tid; v < n; v += kSelThreads)
+    if (!ms[v]) unp[atomicAdd(&s_nunp, 1)] = v;
+  __syncthreads();
+  if (tid == 0) {
+    st->sl = sl;
+    st->nunp = s_nunp;
+    st->rounds = rounds;
+    if (sl <= 0) {
+      // DSTEP_EXEC returns with SL = 0: the loop ends with INFO = S (src/D/dstep.F90:421, 575-582)
+      st->info = st->steps;
+      st->stop = 1;
+      if (st->trace_on && st->trace_steps < st->trace_cap_steps) {
+        const int s = st->trace_steps++;
+        tr.sl[s] = 0; tr.nl[s] = -1; tr.tw[s] = -0.0; tr.trig[s] = 0; tr.hyp[s] = 0; tr.rounds[s] = rounds;
+      }
+    }
+    else {
+      st->pending = 1;
+      if (early) end_of_step<T>(st, piv, J, tr, &st->halt);
+    }
+  }
 }
 
 // ---------------------------------------------------------------------------
@@ -1700,7 +1631,7 @@ k_ncp3_pick(State *st, const int *__restrict__ itp, const int *__restrict__ sort
   __shared__ unsigned char ms[kNcp3MaxN];
   const int tid = threadIdx.x;
   if (tid == 0) {
-    end_of_step<T>(st, piv, J, tr);
+    end_of_step<T>(st, piv, J, tr, &st->stop);
     s_stop = st->stop;
     s_nunp = 0;
   }
@@ -1766,13 +1697,6 @@ k_ncp3_pick(State *st, const int *__restrict__ itp, const int *__restrict__ sort
     }
     else st->pending = 1;
   }
-}
-
-size_t select_smem(int n)
-{
-  const int s2 = pow2ceil(n / 2 > 0 ? n / 2 : 1);
-  const int np = (n / 2 + 1) + ((n / 2 + 1) & 1);
-  return (size_t)s2 * (8 + 4 + 4) + (size_t)np * 8 + (size_t)n * (32 + 4 + 2 + 2 + 2 + 1) + 16;
 }
 
 // k_colsort instantiations: records per thread E = pow2ceil(n) / SORT_THREADS
@@ -1913,12 +1837,12 @@ cudaError_t prepare_kernels(int n)
     e = cudaFuncSetAttribute(k_hyp_pm, cudaFuncAttributeMaxDynamicSharedMemorySize, SCAN_STAGES * (2 * TW) * SCAN_RS * (int)sizeof(double));
   if (e == cudaSuccess) e = cudaFuncSetAttribute(k_rotate<double2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 2 * n * 16);
   if (e == cudaSuccess) e = cudaFuncSetAttribute(k_hyp_z_pm, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kZSmem);
-  const int ss = (int)select_smem(n);
-  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_select<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, ss);
-  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_select<double2>, cudaFuncAttributeMaxDynamicSharedMemorySize, ss);
-  const int cs = (int)select_cluster_smem(n);
-  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_select_cluster<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, cs);
-  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_select_cluster<double2>, cudaFuncAttributeMaxDynamicSharedMemorySize, cs);
+  const int ss = (int)SelLayout(n, select_cluster(n)).total;
+  for (const void *f : { (const void *)k_select<double>, (const void *)k_select<double2> }) {
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, ss);
+    // clusters of 16
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(f, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+  }
   return e;
 }
 
@@ -2024,11 +1948,11 @@ static cudaError_t colsort(Workspace &w, cudaStream_t s)
 {
   const int n = w.n;
   switch (colsort_e(n)) {
-  case 1: k_colsort<1><<<n, SORT_THREADS, 0, s>>>(w.st, w.Wm, n, w.list, w.rank, w.len); break;
-  case 2: k_colsort<2><<<n, SORT_THREADS, 0, s>>>(w.st, w.Wm, n, w.list, w.rank, w.len); break;
-  case 4: k_colsort<4><<<n, SORT_THREADS, 0, s>>>(w.st, w.Wm, n, w.list, w.rank, w.len); break;
-  case 8: k_colsort<8><<<n, SORT_THREADS, 0, s>>>(w.st, w.Wm, n, w.list, w.rank, w.len); break;
-  case 16: k_colsort<16><<<n, SORT_THREADS, 0, s>>>(w.st, w.Wm, n, w.list, w.rank, w.len); break;
+  case 1: k_colsort<1><<<n, SORT_THREADS, 0, s>>>(w.st, w.Wm, n, w.list, w.len); break;
+  case 2: k_colsort<2><<<n, SORT_THREADS, 0, s>>>(w.st, w.Wm, n, w.list, w.len); break;
+  case 4: k_colsort<4><<<n, SORT_THREADS, 0, s>>>(w.st, w.Wm, n, w.list, w.len); break;
+  case 8: k_colsort<8><<<n, SORT_THREADS, 0, s>>>(w.st, w.Wm, n, w.list, w.len); break;
+  case 16: k_colsort<16><<<n, SORT_THREADS, 0, s>>>(w.st, w.Wm, n, w.list, w.len); break;
   default: return cudaErrorInvalidValue;
   }
   return cudaGetLastError();
@@ -2048,20 +1972,30 @@ static cudaError_t select_t(Workspace &w, const T *A, int n_2, cudaStream_t s)
                                                                                  n_2, w.n3val, w.n3len);
     k_ncp3_pick<T><<<1, 256, 0, s>>>(w.st, w.n3it, w.n3sorted, w.n3tie, w.Wm, w.J, n, n_2, w.n3val, (Piv<T> *)w.piv, w.unp,
                                      w.n3it, w.tr);
+    if (A) {
+      const int half = n / 2 > 0 ? n / 2 : 1;
+      k_pivots<T><<<(half + 127) / 128, 128, 0, s>>>(w.st, A, w.J, n, (Piv<T> *)w.piv, (RowRot<T> *)w.rowrot, w.zba_quirk);
+    }
   }
   else {
     e = colsort(w, s);
     if (e != cudaSuccess) return e;
-    if (n >= kSelClusterMinN)
-      k_select_cluster<T><<<SEL_CLUSTER, SEL_CTHREADS, select_cluster_smem(n), s>>>(w.st, w.Wm, w.J, n, n_2, w.list, w.len,
-                                                                                  (Piv<T> *)w.piv, w.unp, w.tr);
-    else
-      k_select<T><<<1, SEL_THREADS, select_smem(n), s>>>(w.st, w.Wm, w.J, n, n_2, w.list, w.len, (Piv<T> *)w.piv, w.unp,
-                                                       w.tr);
-  }
-  if (A) {
-    const int half = n / 2 > 0 ? n / 2 : 1;
-    k_pivots<T><<<(half + 127) / 128, 128, 0, s>>>(w.st, A, w.J, n, (Piv<T> *)w.piv, (RowRot<T> *)w.rowrot, w.zba_quirk);
+    const int C = select_cluster(n);
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = (unsigned)C;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    cfg.gridDim = dim3((unsigned)C);
+    cfg.blockDim = dim3(kSelThreads);
+    cfg.dynamicSmemBytes = SelLayout(n, C).total;
+    cfg.stream = s;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    e = cudaLaunchKernelEx(&cfg, k_select<T>, w.st, (const double *)w.Wm, (const int *)w.J, n, n_2,
+                           (const unsigned short *)w.list, (const int *)w.len, A, (Piv<T> *)w.piv, (RowRot<T> *)w.rowrot,
+                           w.unp, w.tr, w.zba_quirk, w.learned ? 0 : 1);
+    if (e != cudaSuccess) return e;
   }
   return cudaGetLastError();
 }
