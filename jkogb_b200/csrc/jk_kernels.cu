@@ -1181,6 +1181,8 @@ k_colsort(const State *st, const double *__restrict__ Wm, int n, unsigned short 
   for (int r = tid; r < cnt; r += blockDim.x) {
     lv[r] = (unsigned short)ckey_u(sk[r], v);
   }
+  // the last group of 8 is read whole
+  if (tid < 8 && cnt + tid < ((cnt + 7) & ~7)) lv[cnt + tid] = 0;
   if (tid == 0) len[v] = cnt;
 }
 
@@ -1271,49 +1273,70 @@ __global__ void k_pivots(State *st, const T *__restrict__ A, const int *__restri
 // C blocks (1 to 16) that share its state through distributed shared memory (plain loads, stores
 // and atomics; no multicast).
 //
-// Block c owns the vertices v = c (mod C); a warp owns up to 32 of them, one per lane (list
-// pointer, length and candidate in registers), and walks a list together: 64 entries per probe,
-// a ballot finds the first free partner.  The first lp entries of every own list lie in shared
-// memory (all of them up to N = 1200 or so), the rest is read from L2.  Every block keeps a replica of the
-// vertices' state (0 free, 1 matched).  A round:
-//   (A) a free vertex whose candidate is gone walks on to its best free partner, and notes it
-//       with the round's number in best[];
-//   (B) a vertex that moved in this round and whose candidate points back is matched with it
-//       (where both moved, the smaller index does it): the pair goes to block 0's list, both states
-//       to every replica.  Pairs of which neither moved were seen before.
+// Block c owns the vertices v = c (mod C).  Four lanes walk a list together, 64 entries per probe
+// (two 16-byte loads a lane), so that a warp walks eight lists at a time.  A ring of R entries of
+// every own list lies in shared memory, refilled by cp.async behind the pointer (the whole list
+// where it fits); what a long walk needs beyond it is read from L2.  Every block keeps a replica of
+// the vertices' state (a bit each: bytes would meet in fewer banks) and of their candidates.
+// A round:
+//   (A) a free vertex whose candidate is gone walks on to its best free partner and writes it,
+//       stamped with the round, to every replica; cluster barrier;
+//   (B) every block matches the vertices that moved in this round and whose candidate points
+//       back (where both moved, the smaller index does it): the pair goes to its owner's list, both
+//       bits to the own replica; block barrier.  Pairs of which neither moved were seen before.
 // A round without a match ends the matching.  Mutual best free partners are what the walk over the
 // sorted records takes, so the rounds rebuild its matching.
 //
-// What bounds it is the rounds' latency: two barriers and the longest walk.  With one
-// thread per list, 8 to 128 entries at a time (and a 16-entry window), a round cost 6.5 us at
-// N = 2048 (415 us a step on 8 blocks) and 2 us at N = 256 (43 us on one block).
+// One cluster barrier per round is enough because a candidate is written to the buffer of the
+// round's parity and read with its stamp.  A block that is still in (B) of round r may find
+// that a faster one has overwritten a candidate there with round r + 1's (stamp too new: ignored)
+// and left only an older one.  Such a vertex moved on because its candidate was matched with
+// another one in round r, so it has no match in round r, and an older candidate was gone before.
+//
+// What bounds it is the rounds' latency: a walk's dependent instructions, the cluster barrier (about
+// 850 cycles for 4 blocks as for 16).  On graded input nearly every free vertex moves in nearly
+// every round (50 rounds at N = 2048, walks of 30 to 200 entries): all prefer the same large
+// columns.  Measured per step at N = 2048 graded: one thread per list with a 16-entry window on 8 blocks
+// 415 us; a warp or eight lanes per list and two cluster barriers a round 214 and 195 us; this form 165 us
+// (with the 2x2 HSVDs, 6 us, in all but the first).
 //
 // The order of the pivots matters only where the first N_2 of them are taken (np > N_2) or a
 // trace records them; otherwise they are left as matched and the sort is saved.
 constexpr int kSelThreads = 512;
-constexpr size_t kSelListBytes = 176 * 1024;  // shared memory for list prefixes
+constexpr int kSelLanes = 4;                  // lanes per list
+constexpr int kSelEntries = 16;               // list entries per lane and probe
+constexpr size_t kSelListBytes = 150 * 1024;  // shared memory for the rings
 
-// blocks per cluster: enough that a block's lists fit its shared memory and no warp walks for
-// many vertices; a larger cluster pays more per barrier
+// blocks per cluster: enough that a block's rings fit its shared memory and that no lane group walks
+// for many vertices; one block while that holds, since it needs no cluster barrier
 static int select_cluster(int n)
 {
   return (n <= 300) ? 1 : (n <= 600) ? 4 : (n <= 900) ? 8 : 16;
 }
 
+constexpr unsigned kSelNone = 0xFFFFu, kSelRetired = 0xFFFEu;  // no candidate yet; no free partner left
+
 struct SelLayout {
-  int nl, lp;  // own vertices per block, list entries held in shared memory
-  size_t best, pairs, ms, total;
+  int nl, R;      // own vertices per block, ring entries (a power of two)
+  int n4;         // entries of a candidate buffer
+  size_t stride;  // bytes per ring, padded so that rings start in different banks
+  size_t cand, cur, ptr, slen, fill, pairs, taken, total;
   __host__ __device__ SelLayout(int n, int C)
   {
     nl = (n + C - 1) / C;
-    const int ld = list_ld(n);
-    const int fit = (int)(kSelListBytes / ((size_t)nl * 2)) & ~7;
-    lp = (ld < fit) ? ld : fit;
-    const size_t lists = (size_t)nl * lp * 2, sort = (size_t)pow2ceil(n / 2 > 0 ? n / 2 : 1) * 16;
-    best = (lists > sort) ? lists : sort;  // the final ranking reuses the lists' space
-    pairs = best + (((size_t)nl * 4 + 15) & ~(size_t)15);
-    ms = pairs + (size_t)(n / 2 + 1) * 8;
-    total = ms + (size_t)n + 16;
+    R = pow2ceil(list_ld(n));
+    while (R > 64 && (size_t)nl * (R * 2 + 16) > kSelListBytes) R >>= 1;
+    stride = (size_t)R * 2 + 16;
+    const size_t lists = (size_t)nl * stride, sort = (size_t)pow2ceil(n / 2 > 0 ? n / 2 : 1) * 16;
+    cand = (lists > sort) ? lists : sort;  // the final ranking reuses the rings' space
+    n4 = (n + 3) & ~3;
+    cur = cand + (size_t)n4 * 8;
+    ptr = cur + (size_t)nl * 2;
+    slen = ptr + (size_t)nl * 2;
+    fill = slen + (size_t)nl * 2;
+    pairs = (fill + (size_t)nl * 2 + 15) & ~(size_t)15;
+    taken = pairs + (size_t)(n / 2 + 1) * 8;
+    total = taken + (size_t)((n + 31) / 32) * 4;
   }
 };
 
@@ -1327,12 +1350,15 @@ k_select(State *st, const double *__restrict__ Wm, const int *__restrict__ J, in
   const int C = (int)cluster.num_blocks(), c = (int)cluster.block_rank();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const SelLayout L(n, C);
-  unsigned short *lists = (unsigned short *)smem_raw;          // [nl][lp]
-  unsigned *best = (unsigned *)(smem_raw + L.best);            // [nl]: candidate | round << 16
+  unsigned *cand = (unsigned *)(smem_raw + L.cand);            // [2][n4]: candidate | (round + 1) << 16
+  unsigned short *cur = (unsigned short *)(smem_raw + L.cur);  // [nl]: the current candidate
+  unsigned short *ptr = (unsigned short *)(smem_raw + L.ptr);  // [nl]: its position
+  unsigned short *slen = (unsigned short *)(smem_raw + L.slen);
+  unsigned short *fill = (unsigned short *)(smem_raw + L.fill);  // [nl]: list entries fetched
   int2 *pairs = (int2 *)(smem_raw + L.pairs);                  // [n/2 + 1]  (block 0)
-  unsigned char *ms = (unsigned char *)(smem_raw + L.ms);      // [n]
-  __shared__ int s_cnt, s_nunp, s_got[3];
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = kSelThreads / 32, ld = list_ld(n);
+  unsigned *taken = (unsigned *)(smem_raw + L.taken);          // [(n + 31) / 32]: a bit per vertex
+  __shared__ int s_cnt, s_off, s_np, s_nunp, s_got[2];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, ld = list_ld(n);
   const bool solo = (C == 1);
   auto sync = [&]() { if (solo) __syncthreads(); else cluster.sync(); };
 
@@ -1347,142 +1373,210 @@ k_select(State *st, const double *__restrict__ Wm, const int *__restrict__ J, in
     if (c == 0 && tid == 0) st->stop = st->halt;
     return;
   }
-  if (tid == 0) { s_cnt = 0; s_nunp = 0; s_got[0] = 0; s_got[1] = 0; s_got[2] = 0; }
-  // the lists' prefixes, 16 bytes at a time
+  if (tid == 0) { s_cnt = 0; s_nunp = 0; s_got[0] = 0; s_got[1] = 0; }
+  // the lists' first R entries, 16 bytes at a time
+  const int first_fill = min(L.R, ld);
   {
-    const int pieces = L.lp / 8;
+    const int pieces = first_fill / 8;
     for (int k = tid; k < L.nl * pieces; k += kSelThreads) {
       const int lv = k / pieces, e = k % pieces, v = lv * C + c;
-      if (v < n) cp_async16((uint4 *)(lists + (size_t)lv * L.lp) + e, (const uint4 *)(list + (long long)v * ld) + e);
+      if (v < n) cp_async16(smem_raw + lv * L.stride + 16 * e, (const uint4 *)(list + (long long)v * ld) + e);
     }
     cp_async_commit();
   }
-  for (int v = tid; v < n; v += kSelThreads) ms[v] = 0;
-  // lane j of a warp owns vertex lv0 + j
-  const int K = (L.nl + nw - 1) / nw, lv0 = warp * K, mylv = lv0 + lane, myv = mylv * C + c;
-  bool active = (lane < K) && (mylv < L.nl) && (myv < n);
-  const int mylen = active ? len[myv] : 0;
-  int ptr = 0, cand = -1;
+  for (int k = tid; k < (n + 31) / 32; k += kSelThreads) taken[k] = 0u;
+  for (int lv = tid; lv < L.nl; lv += kSelThreads) {
+    cur[lv] = (unsigned short)kSelNone;
+    ptr[lv] = 0;
+    fill[lv] = (unsigned short)first_fill;
+    slen[lv] = (lv * C + c < n) ? (unsigned short)len[lv * C + c] : 0;
+  }
+  for (int v = tid; v < 2 * L.n4; v += kSelThreads) cand[v] = 0u;
   cp_async_wait<0>();
   sync();
   if (c == 0 && tid == 0) { st->nl = 0; st->err = 0; }
 
+  constexpr int kGroups = kSelThreads / kSelLanes, kProbe = kSelEntries * kSelLanes;
+  const int gl = lane % kSelLanes, gs = lane - gl;  // the lane within its group, the group's first lane
+  auto gone = [&](unsigned u) { return (taken[u >> 5] >> (u & 31)) & 1u; };
   int rounds = 0;
   for (int round = 0; round <= n / 2 + 1; ++round) {
-    // (A)
-    // (a slow thread may still read the last round's flag)
-    if (tid == 0) s_got[(round + 1) % 3] = 0;
-    bool moved = false;
-    if (active && ms[myv]) active = false;
-    unsigned need = __ballot_sync(0xFFFFFFFFu, active && (cand < 0 || ms[cand]));
-    while (need) {
-      const int sl = __ffs(need) - 1;
-      need &= need - 1;
-      const int p = __shfl_sync(0xFFFFFFFFu, ptr, sl), Lv = __shfl_sync(0xFFFFFFFFu, mylen, sl);
-      const unsigned short *row = lists + (size_t)(lv0 + sl) * L.lp;
-      const unsigned short *grow = list + (long long)((lv0 + sl) * C + c) * ld;
-      int found = -1, at = Lv;
-      for (int base = p & ~1; base < Lv; base += 64) {
-        const int idx = base + 2 * lane;
-        unsigned e = 0u;
-        if (idx < Lv) e = *(const unsigned *)((idx < L.lp ? row : grow) + idx);
-        const int u0 = (int)(e & 0xFFFFu), u1 = (int)(e >> 16);
-        const unsigned m0 = __ballot_sync(0xFFFFFFFFu, idx >= p && idx < Lv && !ms[u0]);
-        const unsigned m1 = __ballot_sync(0xFFFFFFFFu, idx + 1 < Lv && !ms[u1]);
-        if (m0 | m1) {
-          const int i0 = m0 ? 2 * (__ffs(m0) - 1) : 64, i1 = m1 ? 2 * (__ffs(m1) - 1) + 1 : 64;
-          const int i = (i0 < i1) ? i0 : i1;
-          found = __shfl_sync(0xFFFFFFFFu, (i & 1) ? u1 : u0, i >> 1);
-          at = base + i;
-          break;
+    unsigned *cnow = cand + (size_t)(round & 1) * L.n4, *cold = cand + (size_t)(~round & 1) * L.n4;
+    const unsigned stamp = (unsigned)(round + 1);
+    if (tid == 0) s_got[round & 1] = 0;
+    // the rings' refills of the last round
+    cp_async_wait<0>();
+    __syncwarp();
+    // (A) group g takes the own vertices g, g + kGroups, ...
+    for (int lv0 = warp * (32 / kSelLanes); lv0 < L.nl; lv0 += kGroups) {
+      const int lv = lv0 + lane / kSelLanes, v = lv * C + c;
+      const bool own = (lv < L.nl) && (v < n);
+      const unsigned old = own ? cur[lv] : kSelRetired;
+      // walking: free, not retired, and without a candidate that is still free
+      bool walking = old != kSelRetired && !gone(v) && (old == kSelNone || gone(old));
+      if (!__any_sync(0xFFFFFFFFu, walking)) continue;
+      const int Lv = own ? slen[lv] : 0, p = own ? ptr[lv] : 0, F = own ? fill[lv] : 0;
+      const unsigned char *ring = smem_raw + lv * L.stride;
+      unsigned found = kSelRetired;
+      int at = Lv, base = p & ~7;
+      bool moved = walking;
+      while (__any_sync(0xFFFFFFFFu, walking)) {
+        const int idx = base + kSelEntries * gl;
+        unsigned free = 0u;
+        if (walking && idx < Lv) {
+          unsigned t = 0u;
+#pragma unroll
+          for (int h = 0; h < kSelEntries / 8; ++h) {
+            const int ix = idx + 8 * h;
+            uint4 q4 = make_uint4(0u, 0u, 0u, 0u);
+            if (ix >= Lv) {}
+            else if (ix < F) q4 = *(const uint4 *)(ring + 2 * (ix & (L.R - 1)));
+            else q4 = *(const uint4 *)(list + (long long)v * ld + ix);
+            const unsigned w4[4] = { q4.x, q4.y, q4.z, q4.w };
+#pragma unroll
+            for (int e = 0; e < 8; ++e) {
+              const unsigned x = (w4[e >> 1] >> ((e & 1) * 16)) & 0xFFFFu;
+              t |= ((taken[x >> 5] >> (x & 31)) & 1u) << (8 * h + e);
+            }
+          }
+          // entries from the pointer on and before the list's end
+          constexpr unsigned all = (1u << kSelEntries) - 1u;
+          free = ~t & (all << max(p - idx, 0)) & (all >> max(idx + kSelEntries - Lv, 0));
+        }
+        const unsigned hit = (__ballot_sync(0xFFFFFFFFu, free != 0u) >> gs) & ((1u << kSelLanes) - 1u);
+        const int fi = __shfl_sync(0xFFFFFFFFu, idx + __ffs(free) - 1, gs + (hit ? __ffs(hit) - 1 : 0));
+        if (walking) {
+          if (hit) {
+            walking = false;
+            at = fi;
+            found = (fi < F) ? *(const unsigned short *)(ring + 2 * (fi & (L.R - 1))) : list[(long long)v * ld + fi];
+          }
+          else {
+            base += kProbe;
+            if (base >= Lv) walking = false;  // no free partner is left
+          }
         }
       }
-      if (lane == sl) {
-        ptr = at;
-        cand = found;
-        moved = (found >= 0);
-        if (found < 0) active = false;  // no free partner is left: retired
-        best[mylv] = (found < 0) ? 0xFFFFFFFFu : ((unsigned)found | ((unsigned)round << 16));
+      if (moved) {
+        const unsigned e = found | (stamp << 16);
+        if (solo) { if (gl == 0) cnow[v] = e; }
+        else
+          for (int r = gl; r < C; r += kSelLanes) *cluster.map_shared_rank(&cnow[v], r) = e;
+        int f = max(F, at & ~63);  // what a long walk has left behind is not fetched
+        const int room = min((at & ~63) + L.R, ld);
+        while (f < room) {
+#pragma unroll
+          for (int h = 0; h < kSelEntries / 8; ++h) {
+            const int ix = f + kSelEntries * gl + 8 * h;
+            if (ix < room) cp_async16(smem_raw + lv * L.stride + 2 * (ix & (L.R - 1)), list + (long long)v * ld + ix);
+          }
+          f += kProbe;
+        }
+        if (gl == 0) { cur[lv] = (unsigned short)found; ptr[lv] = (unsigned short)at; fill[lv] = (unsigned short)room; }
       }
     }
+    cp_async_commit();
     sync();
     // (B)
-    if (moved) {
-      const unsigned b = solo ? best[cand] : *cluster.map_shared_rank(&best[cand / C], cand % C);
-      if ((int)(b & 0xFFFFu) == myv && ((int)(b >> 16) != round || myv < cand)) {
-        if (solo) {
-          ms[myv] = 1;
-          ms[cand] = 1;
-          s_got[round % 3] = 1;
-          pairs[atomicAdd(&s_cnt, 1)] = make_int2(min(myv, cand), max(myv, cand));
-        }
-        else {
-          for (int b2 = 0; b2 < C; ++b2) {
-            *cluster.map_shared_rank(&ms[myv], b2) = 1;
-            *cluster.map_shared_rank(&ms[cand], b2) = 1;
-            *cluster.map_shared_rank(&s_got[round % 3], b2) = 1;
-          }
-          cluster.map_shared_rank(pairs, 0)[atomicAdd(cluster.map_shared_rank(&s_cnt, 0), 1)] =
-              make_int2(min(myv, cand), max(myv, cand));
-        }
-      }
+    auto settle = [&](unsigned v, unsigned u, unsigned e0, unsigned e1) {
+      const unsigned s0 = e0 >> 16, s1 = e1 >> 16;
+      const unsigned eu = (s0 <= stamp && (s1 > stamp || s0 > s1)) ? e0 : e1, su = eu >> 16;
+      // (stamp 0: not a vertex that moved, or nothing written there yet)
+      if ((eu & 0xFFFFu) != v || su == 0u || su > stamp || (su == stamp && v > u)) return;
+      atomicOr(&taken[v >> 5], 1u << (v & 31));
+      atomicOr(&taken[u >> 5], 1u << (u & 31));
+      s_got[round & 1] = 1;
+      if (solo || (v & (unsigned)(C - 1)) == (unsigned)c) pairs[atomicAdd(&s_cnt, 1)] = make_int2((int)min(v, u), (int)max(v, u));
+    };
+    auto now = [&](unsigned e) { return (e >> 16) == stamp && (e & 0xFFFFu) != kSelRetired; };
+    if (n <= kSelThreads) {
+      const unsigned e = (tid < n) ? cnow[tid] : 0u, u = e & 0xFFFFu;
+      if (now(e)) settle((unsigned)tid, u, cnow[u], cold[u]);
     }
-    sync();
+    else
+      for (int v0 = 4 * tid; v0 < n; v0 += 4 * kSelThreads) {
+        const uint4 e4 = *(const uint4 *)(cnow + v0);
+        const unsigned e[4] = { e4.x, e4.y, e4.z, e4.w };
+        unsigned e0[4], e1[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const unsigned u = e[j] & 0xFFFFu;
+          const bool in = now(e[j]);
+          e0[j] = in ? cnow[u] : 0u;
+          e1[j] = in ? cold[u] : 0u;
+        }
+#pragma unroll
+        for (int j = 0; j < 4; ++j) settle((unsigned)(v0 + j), e[j] & 0xFFFFu, e0[j], e1[j]);
+      }
+    __syncthreads();
     rounds = round + 1;
-    if (!s_got[round % 3]) break;
+    if (!s_got[round & 1]) break;
   }
 
-  // the pairs are complete
-  const int np = solo ? s_cnt : *cluster.map_shared_rank(&s_cnt, 0);
+  cp_async_wait<0>();
+  sync();  // every block's count stands
+  // the pairs are complete: their number and, per block, the place of its own among them
+  if (tid == 0) {
+    int np = 0;
+    for (int b = 0; b < C; ++b) {
+      if (b == c) s_off = np;
+      np += (b == c) ? s_cnt : *cluster.map_shared_rank(&s_cnt, b);
+    }
+    s_np = np;
+  }
+  __syncthreads();
+  const int np = s_np, off = s_off, cnt = s_cnt;
   const int sl = (np < n_2) ? np : n_2;
   const bool ranked = (np > n_2) || st->trace_on || !A;
   if (ranked) {
-    if (c == 0) {
-      const int s2 = pow2ceil(n / 2 > 0 ? n / 2 : 1);
-      unsigned long long *skey = (unsigned long long *)smem_raw;  // [s2]
-      unsigned *stie = (unsigned *)(skey + s2);                   // [s2]
-      int *sidx = (int *)(stie + s2);                             // [s2]
-      for (int i = tid; i < s2; i += kSelThreads) {
-        if (i < np) {
-          const int2 pr = pairs[i];
-          skey[i] = wkey(Wm[(long long)pr.x * n + pr.y]);
-          stie[i] = tkey(pr.x, pr.y);
-          sidx[i] = i;
-        }
-        else { skey[i] = 0ULL; stie[i] = 0u; sidx[i] = -1; }
+    // the pairs in rank order (AW_SRT), by block 0; piv is their first place of call
+    for (int i = tid; i < cnt; i += kSelThreads) { piv[off + i].p = pairs[i].x; piv[off + i].q = pairs[i].y; }
+    __threadfence();
+    sync();
+    if (c != 0) return;
+    const int s2 = pow2ceil(n / 2 > 0 ? n / 2 : 1);
+    unsigned long long *skey = (unsigned long long *)smem_raw;  // [s2]
+    unsigned *stie = (unsigned *)(skey + s2);                   // [s2]
+    int *sidx = (int *)(stie + s2);                             // [s2]
+    for (int i = tid; i < s2; i += kSelThreads) {
+      skey[i] = 0ULL; stie[i] = 0u; sidx[i] = -1;
+      if (i < np) {
+        const int p = __ldcg(&piv[i].p), q = __ldcg(&piv[i].q);
+        pairs[i] = make_int2(p, q);
+        skey[i] = wkey(Wm[(long long)p * n + q]);
+        stie[i] = tkey(p, q);
+        sidx[i] = i;
       }
-      __syncthreads();
-      bitonic_desc(skey, stie, sidx, s2);
-      for (int v = tid; v < n; v += kSelThreads) ms[v] = 0;
-      __syncthreads();
-      for (int r = tid; r < sl; r += kSelThreads) {
-        const int2 pr = pairs[sidx[r]];
-        ms[pr.x] = 1;
-        ms[pr.y] = 1;
-        piv[r].p = pr.x;
-        piv[r].q = pr.y;
-        piv[r].w = Wm[(long long)pr.x * n + pr.y];
-        if (A) pivot_hsvd<T>(st, A, J, n, pr.x, pr.y, piv[r], rr[r], quirk);
-      }
-      __syncthreads();
     }
-  }
-  else {
-    const int2 *pairs0 = solo ? pairs : cluster.map_shared_rank(pairs, 0);
-    // warps of different blocks first, so that few pivots share an SM
-    for (int r = (warp * C + c) * 32 + lane; r < np; r += kSelThreads * C) {
-      const int2 pr = pairs0[r];
+    __syncthreads();
+    bitonic_desc(skey, stie, sidx, s2);
+    for (int k = tid; k < (n + 31) / 32; k += kSelThreads) taken[k] = 0u;
+    __syncthreads();
+    for (int r = tid; r < sl; r += kSelThreads) {
+      const int2 pr = pairs[sidx[r]];
+      atomicOr(&taken[pr.x >> 5], 1u << (pr.x & 31));
+      atomicOr(&taken[pr.y >> 5], 1u << (pr.y & 31));
       piv[r].p = pr.x;
       piv[r].q = pr.y;
-      pivot_hsvd<T>(st, A, J, n, pr.x, pr.y, piv[r], rr[r], quirk);
+      piv[r].w = Wm[(long long)pr.x * n + pr.y];
+      if (A) pivot_hsvd<T>(st, A, J, n, pr.x, pr.y, piv[r], rr[r], quirk);
+    }
+    __syncthreads();
+  }
+  else {
+    for (int i = tid; i < cnt; i += kSelThreads) {
+      const int r = off + i;
+      piv[r].p = pairs[i].x;
+      piv[r].q = pairs[i].y;
+      pivot_hsvd<T>(st, A, J, n, pairs[i].x, pairs[i].y, piv[r], rr[r], quirk);
     }
     __threadfence();
-    sync();  // every pivot is counted, and every block is done with block 0's list
+    sync();  // every pivot is counted
   }
   if (c != 0) return;
   // the columns outside the pivots
   for (int v = tid; v < n; v += kSelThreads)
-    if (!ms[v]) unp[atomicAdd(&s_nunp, 1)] = v;
+    if (!((taken[v >> 5] >> (v & 31)) & 1u)) unp[atomicAdd(&s_nunp, 1)] = v;
   __syncthreads();
   if (tid == 0) {
     st->sl = sl;
