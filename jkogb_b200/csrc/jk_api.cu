@@ -10,6 +10,7 @@
 
 #include "../../include/jkogb.h"
 #include "jk_internal.h"
+#include "jk_device.cuh"
 
 using namespace jk;
 
@@ -80,7 +81,8 @@ int jstep_len(int n, int n_2)
 }
 
 // device workspace of one solve
-int make_workspace(Guard &g, Workspace &w, int n, int cplx, const int *J, int trace_on, int cap_steps, long long cap_piv)
+int make_workspace(Guard &g, Workspace &w, int n, int cplx, const int *J, int trace_on, int cap_steps, long long cap_piv,
+                   int small = 0)
 {
   memset(&w, 0, sizeof(w));
   w.n = n;
@@ -95,7 +97,22 @@ int make_workspace(Guard &g, Workspace &w, int n, int cplx, const int *J, int tr
   const size_t pivsz = cplx ? sizeof(Piv<double2>) : sizeof(Piv<double>);
   const size_t rrsz = cplx ? sizeof(RowRot<double2>) : sizeof(RowRot<double>);
   const int half = n / 2 + 1;
+  w.small = small && small_fits(cplx, n, w.n_plus);
   CK(g.alloc(&w.J, n * sizeof(int)));
+  CK(g.alloc(&w.st, sizeof(State)));
+  CK(cudaMallocHost((void **)&g.pinned, sizeof(State)));
+  w.st_host = (State *)g.pinned;
+  CK(cudaMemcpy(w.J, j32.data(), n * sizeof(int), cudaMemcpyHostToDevice));
+  State s0;
+  memset(&s0, 0, sizeof(s0));
+  s0.trace_on = trace_on;
+  s0.trace_cap_steps = trace_on ? cap_steps : 0;
+  s0.trace_cap_piv = trace_on ? cap_piv : 0;
+  CK(cudaMemcpy(w.st, &s0, sizeof(State), cudaMemcpyHostToDevice));
+  if (w.small) {
+    CK(prepare_small(cplx, n, w.n_plus));
+    return 0;
+  }
   CK(g.alloc(&w.plus, (plus.size() + 1) * sizeof(int)));
   CK(g.alloc(&w.minus, (minus.size() + 1) * sizeof(int)));
   CK(g.alloc(&w.Wm, (size_t)n * n * sizeof(double)));
@@ -105,7 +122,6 @@ int make_workspace(Guard &g, Workspace &w, int n, int cplx, const int *J, int tr
   CK(g.alloc(&w.list, (size_t)n * ((n + 7) & ~7) * sizeof(unsigned short)));
   CK(g.alloc(&w.len, n * sizeof(int)));
   CK(g.alloc(&w.unp, (n + 1) * sizeof(int)));
-  CK(g.alloc(&w.st, sizeof(State)));
   if (trace_on) {
     const int cs = cap_steps > 0 ? cap_steps : 1;
     const long long cp = cap_piv > 0 ? cap_piv : 1;
@@ -117,17 +133,8 @@ int make_workspace(Guard &g, Workspace &w, int n, int cplx, const int *J, int tr
     CK(g.alloc(&w.tr.rounds, cs * sizeof(int)));
     CK(g.alloc(&w.tr.piv, cp * sizeof(int2)));
   }
-  CK(cudaMallocHost((void **)&g.pinned, sizeof(State)));
-  w.st_host = (State *)g.pinned;
-  CK(cudaMemcpy(w.J, j32.data(), n * sizeof(int), cudaMemcpyHostToDevice));
   if (!plus.empty()) CK(cudaMemcpy(w.plus, plus.data(), plus.size() * sizeof(int), cudaMemcpyHostToDevice));
   if (!minus.empty()) CK(cudaMemcpy(w.minus, minus.data(), minus.size() * sizeof(int), cudaMemcpyHostToDevice));
-  State s0;
-  memset(&s0, 0, sizeof(s0));
-  s0.trace_on = trace_on;
-  s0.trace_cap_steps = trace_on ? cap_steps : 0;
-  s0.trace_cap_piv = trace_on ? cap_piv : 0;
-  CK(cudaMemcpy(w.st, &s0, sizeof(State), cudaMemcpyHostToDevice));
   CK(prepare_kernels(n));
   return 0;
 }
@@ -181,7 +188,10 @@ int solver_make(jk_solver *v, int cplx, int n, const int *J, int n_2, int id_ncp
   v->chunk = (v->o.graph_steps == 0) ? 32 : v->o.graph_steps;
   Workspace &w = v->w;
   Guard &g = v->g;
-  int rc = make_workspace(g, w, n, cplx, J, trace != nullptr, trace ? trace->max_steps : 0, trace ? trace->max_piv : 0);
+  // a small matrix's loop runs in one persistent launch, unless each step is to be recorded, scored
+  // or selected by AW_NCP3
+  int rc = make_workspace(g, w, n, cplx, J, trace != nullptr, trace ? trace->max_steps : 0, trace ? trace->max_piv : 0,
+                          !trace && !sc && id_ncp != 3);
   if (rc) return rc;
   w.zba_quirk = (v->o.zba_quirk == 0) ? 1 : 0;
   w.id_ncp = id_ncp;
@@ -274,14 +284,16 @@ int solver_advance(jk_solver *v, long long k)
   if (v->o.max_steps > 0 && (target == 0 || target > v->o.max_steps)) target = v->o.max_steps;
   CK(launch_limit(v->w, target, v->s));
   ++g_launches;
-  solver_graph(v);
-  const int per_sync = (v->chunk > 0) ? v->chunk : 32;
-  const long long per_step = step_launches(v->w);
+  const bool small = v->w.small;
+  if (!small) solver_graph(v);
+  const int per_sync = small ? 1 : (v->chunk > 0) ? v->chunk : 32;
+  const long long per_step = small ? 1 : step_launches(v->w);
   long long last = v->steps;
   int idle = 0;
   for (;;) {
     cudaError_t e = cudaSuccess;
-    if (v->exec) e = cudaGraphLaunch(v->exec, v->s);
+    if (small) e = launch_small(v->w, v->dA, v->dU, v->dZ, v->n_2, v->s);
+    else if (v->exec) e = cudaGraphLaunch(v->exec, v->s);
     else
       for (int j = 0; j < per_sync && e == cudaSuccess; ++j) e = launch_step(v->w, v->dA, v->dU, v->dZ, v->n_2, v->s);
     if (e == cudaSuccess) e = cudaMemcpyAsync(v->w.st_host, v->w.st, sizeof(State), cudaMemcpyDeviceToHost, v->s);

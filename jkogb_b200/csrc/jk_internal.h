@@ -45,14 +45,15 @@ struct Trace {
   int2 *piv;  // 0-based (p, q)
 };
 
-// One selected pivot (rank order) and its 2x2 transformation.
+// One selected pivot and its 2x2 transformation; R: the rotation coefficients (Rot, ZRot).
+template <typename T> struct Tr;
 template <typename T>
 struct Piv {
   int p, q, info, pad;
-  double w;       // its weight (for the statistics)
-  T V[4];         // left 2x2 of DHSVD2 (before UT2/UH2)
-  T W[4];         // right 2x2 (Z of DHSVD2), W(:,1:2,I) of DSTEP_TRANSF
-  double d[2];    // W(1,3,I), W(2,3,I): the new diagonal
+  double w;              // its weight (for the statistics)
+  typename Tr<T>::R tu;  // the columns of U, valid when info & 2
+  typename Tr<T>::R tz;  // the columns of A and Z, valid when info & 4
+  double d[2];           // W(1,3,I), W(2,3,I): the new diagonal
 };
 
 // Row-rotation record of one pivot: the BA coefficients of V (read by every block).
@@ -94,6 +95,7 @@ struct Workspace {
   State *st_host;    // pinned host mirror
   Trace tr;
   int zba_quirk;
+  int small;         // the loop runs in the persistent kernel, which needs none of the step's buffers
   double *offpart;   // per-block partial off-norms (learned solves)
   int *offcount;     // blocks done (the last one finishes the off-norm)
   int learned;       // rank the scanned hyperbolic pairs by `sc`
@@ -119,6 +121,11 @@ cudaError_t launch_weights(Workspace &w, const void *A, cudaStream_t s);
 cudaError_t launch_match(Workspace &w, int n_2, cudaStream_t s);
 cudaError_t launch_hsvd2_batch(int cplx, int count, void *A, const int *J, void *U, void *Z, int *info, double th1, cudaStream_t s);
 cudaError_t prepare_kernels(int n);
+// the whole loop of a small matrix in one persistent launch (jk_small.cu)
+constexpr int kSmallSteps = 16384;  // steps per launch
+bool small_fits(int cplx, int n, int n_plus);
+cudaError_t prepare_small(int cplx, int n, int n_plus);
+cudaError_t launch_small(Workspace &w, void *A, void *U, void *Z, int n_2, cudaStream_t s);
 // the batched solver (jk_batch.cu): one matrix of the packed batch
 struct BatchItem {
   long long off;  // offset of its n x n blocks in A, U, Z (doubles)

@@ -25,6 +25,7 @@
 
 #include "jk_internal.h"
 #include "jk_device.cuh"
+#include "jk_scan.cuh"
 
 namespace cg = cooperative_groups;
 
@@ -174,35 +175,6 @@ __global__ void k_weights_trig(const State *st, const T *__restrict__ A, const i
 // ---------------------------------------------------------------------------
 #define HR 64
 
-__device__ __forceinline__ void scan_rows_real(const double *xs, const double *ys, int rows, int i0, int p, int q, const Rot &t, double &d)
-{
-  if (t.c1 && t.c2) {
-#pragma unroll 4
-    for (int r = 0; r < rows; ++r) {
-      const double x = xs[r], y = ys[r];
-      const double xx = __dmul_rn(fma(y, t.r1, x), t.m1);
-      const double yy = __dmul_rn(fma(x, t.r2, y), t.m2);
-      const int i = i0 + r;
-      if (i != p && i != q) {
-        d = fma(__dsub_rn(x, xx), __dadd_rn(x, xx), d);
-        d = fma(__dsub_rn(y, yy), __dadd_rn(y, yy), d);
-      }
-    }
-  }
-  else {
-    for (int r = 0; r < rows; ++r) {
-      double x = xs[r], y = ys[r];
-      const double x0 = x, y0 = y;
-      rot_apply(t, x, y);
-      const int i = i0 + r;
-      if (i != p && i != q) {
-        d = fma(__dsub_rn(x0, x), __dadd_rn(x0, x), d);
-        d = fma(__dsub_rn(y0, y), __dadd_rn(y0, y), d);
-      }
-    }
-  }
-}
-
 // ---------------------------------------------------------------------------
 // the real hyperbolic weights, pipelined: a block owns 16 "+" columns x 32 "-"
 // columns; each thread owns two pairs sharing its "+" column (two independent fma
@@ -349,6 +321,53 @@ __device__ __forceinline__ void scan_chunk_kw(int kw, const double *const *xs, c
 #define SCAN_THREADS 256
 #define SCAN_STAGES 3
 
+// the 2x2 HSVDs of a sign-class tile's pairs: the scan parameters of its valid pairs, compacted in
+// slot order, into tpar; the weights that need no scan to W.  Returns the number of slots.  Out of
+// line: the scan that follows has no registers to share with it.
+static __device__ __noinline__ int tile_setup(const double *__restrict__ A, int n, const int *s_col, int *s_warp, HypPar *tpar,
+                                              double *__restrict__ Wm)
+{
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  int total = 0;
+  for (int base = 0; base < TW * TW; base += SCAN_THREADS) {
+    const int l = base + tid;
+    const int ci = l / TW, cj = TW + l % TW;  // tile columns of the "+" and the "-" vertex
+    const int a = s_col[ci], b = s_col[cj];
+    const bool valid = (a >= 0) && (b >= 0);
+    const unsigned m = __ballot_sync(0xFFFFFFFFu, valid);
+    if (!lane) s_warp[warp] = __popc(m);
+    __syncthreads();
+    int slot = total + __popc(m & ((1u << lane) - 1u));
+    for (int w2 = 0; w2 < SCAN_THREADS / 32; ++w2) {
+      const int cw = s_warp[w2];
+      slot += (w2 < warp) ? cw : 0;
+      total += cw;
+    }
+    __syncthreads();
+    if (valid) {
+      int pp, qq;
+      bool ap;
+      double w, d0 = 0.0;
+      Rot t;
+      const bool sc = hyp_pair_setup(A, n, a, b, pp, qq, ap, w, d0, t);
+      HypPar h;
+      h.p = pp; h.q = qq;
+      h.pad = ap ? (ci | (cj << 8)) : (cj | (ci << 8));  // the tile columns of p and of q
+      h.flags = sc ? (1 | (t.c1 ? 2 : 0) | (t.c2 ? 4 : 0)) : 0;
+      h.r1 = sc ? t.r1 : 0.0; h.r2 = sc ? t.r2 : 0.0; h.m1 = sc ? t.m1 : 0.0; h.m2 = sc ? t.m2 : 0.0;
+      h.d = d0;
+      tpar[slot] = h;
+      if (!sc) {
+        if (w < -JK_HUGE) w = nan_w();
+        Wm[(long long)qq * n + pp] = w;
+        Wm[(long long)pp * n + qq] = w;
+      }
+    }
+  }
+  __syncthreads();
+  return total;
+}
+
 // one sign-class tile: tile (ti, tj) holds the pairs of the "+" vertices
 // plus[32 ti .. 32 ti + 31] with the "-" vertices minus[32 tj .. 32 tj + 31], all of
 // them hyperbolic (up to 1024, 4 per thread).  First the 2x2 HSVDs of DMAGF2H (the scan
@@ -369,48 +388,13 @@ k_hyp_pm(const State *st, const double *__restrict__ A, const int *__restrict__ 
   const int P0 = (blockIdx.x / TM) * TW, Q0 = (blockIdx.x % TM) * TW;
   HypPar *tpar = (HypPar *)smem_raw;  // [TW * TW], before the row buffer takes the space
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  __shared__ int s_cnt, s_warp[SCAN_THREADS / 32], s_col[2 * TW];
+  __shared__ int s_warp[SCAN_THREADS / 32], s_col[2 * TW];
   if (tid < 2 * TW) {
     const int c = tid;
     s_col[c] = (c < TW) ? ((P0 + c < n_plus) ? plus[P0 + c] : -1) : ((Q0 + c - TW < n_minus) ? minus[Q0 + c - TW] : -1);
   }
-  if (tid == 0) s_cnt = 0;
   __syncthreads();
-  for (int base = 0; base < TW * TW; base += SCAN_THREADS) {
-    const int l = base + tid;
-    const int ci = l / TW, cj = TW + l % TW;  // tile columns of the "+" and the "-" vertex
-    const int a = s_col[ci], b = s_col[cj];
-    const bool valid = (a >= 0) && (b >= 0);
-    const unsigned m = __ballot_sync(0xFFFFFFFFu, valid);
-    if (!lane) s_warp[warp] = __popc(m);
-    __syncthreads();
-    int off = s_cnt;
-    for (int w2 = 0; w2 < warp; ++w2) off += s_warp[w2];
-    const int slot = off + __popc(m & ((1u << lane) - 1u));
-    __syncthreads();
-    if (tid == 0) { int t = 0; for (int w2 = 0; w2 < SCAN_THREADS / 32; ++w2) t += s_warp[w2]; s_cnt += t; }
-    if (valid) {
-      int pp, qq;
-      bool ap;
-      double w, d0 = 0.0;
-      Rot t;
-      const bool sc = hyp_pair_setup(A, n, a, b, pp, qq, ap, w, d0, t);
-      HypPar h;
-      h.p = pp; h.q = qq;
-      h.pad = ap ? (ci | (cj << 8)) : (cj | (ci << 8));  // the tile columns of p and of q
-      h.flags = sc ? (1 | (t.c1 ? 2 : 0) | (t.c2 ? 4 : 0)) : 0;
-      h.r1 = sc ? t.r1 : 0.0; h.r2 = sc ? t.r2 : 0.0; h.m1 = sc ? t.m1 : 0.0; h.m2 = sc ? t.m2 : 0.0;
-      h.d = d0;
-      tpar[slot] = h;
-      if (!sc) {
-        if (w < -JK_HUGE) w = nan_w();
-        Wm[(long long)qq * n + pp] = w;
-        Wm[(long long)pp * n + qq] = w;
-      }
-    }
-    __syncthreads();
-  }
-  const int cnt = s_cnt;
+  const int cnt = tile_setup(A, n, s_col, s_warp, tpar, Wm);
   if (!cnt) return;
 
   double *buf = (double *)smem_raw;  // [SCAN_STAGES][2 * TW][SCAN_RS]: the "+" columns, then the "-" columns
@@ -513,7 +497,7 @@ k_hyp_pm(const State *st, const double *__restrict__ A, const int *__restrict__ 
           Rot t;
           t.c1 = (fl[k] >> 1) & 1; t.c2 = (fl[k] >> 2) & 1;
           t.r1 = r1[k]; t.r2 = r2[k]; t.m1 = m1[k]; t.m2 = m2[k];
-          scan_rows_real(xs[k], ys[k], rows, i0, pv[k], qv[k], t, d[k]);
+          scan_rows_any(xs[k], ys[k], rows, i0, pv[k], qv[k], t, d[k]);
         }
     }
   }
@@ -537,37 +521,6 @@ __global__ void k_absmat(const State *st, const double2 *__restrict__ A, long lo
   if (st->stop || st->halt || st->learned_step) return;
   for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < nn; k += (long long)gridDim.x * blockDim.x)
     mag[k] = zabs(A[k]);
-}
-
-// hypot2 out of line: the rare operands hypot2_near does not take
-__device__ __noinline__ double hypot2_call(double x, double y) { return hypot2(x, y); }
-
-// whether hypot2_near takes a row's entry: the larger part within 2^(+-998) (a NaN in the
-// other part passes through), or both parts zero
-__device__ __forceinline__ bool scan_near(double2 a)
-{
-  const double u = fmax(fabs(a.x), fabs(a.y));
-  return (u >= 3.7e-301 && u <= 2.6e300) || u == 0.0;
-}
-
-// ABODNZF2's row scan (src/Z/ztransf.F90:452-637) with the magnitudes of the unrotated
-// entries taken from xa, ya: the same operations in the same order
-__device__ __forceinline__ void scan_rows_cplx_mag(const double2 *xs, const double2 *ys, const double *xa, const double *ya,
-                                                   int rows, int i0, int p, int q, const ZRot &t, double &d)
-{
-  for (int r = 0; r < rows; ++r) {
-    double2 x = xs[r], y = ys[r];
-    zrot_apply_ab(t, x, y);
-    double axx, ayy;
-    if (scan_near(x) && scan_near(y)) { axx = zabs_near(x); ayy = zabs_near(y); }
-    else { axx = hypot2_call(x.x, x.y); ayy = hypot2_call(y.x, y.y); }
-    const int i = i0 + r;
-    if (i != p && i != q) {
-      const double axi = xa[r], ayi = ya[r];
-      d = fma(__dsub_rn(axi, axx), __dadd_rn(axi, axx), d);
-      d = fma(__dsub_rn(ayi, ayy), __dadd_rn(ayi, ayy), d);
-    }
-  }
 }
 
 // The complex hyperbolic weights (ZMAGF2H, src/Z/zstep.F90:43-74): the tile of
@@ -598,27 +551,7 @@ k_weights_hyp_z(const State *st, const double2 *__restrict__ A, const double *__
     q = a_is_p ? b : a;
     const double2 app = A[(long long)p * n + p], aqp = A[(long long)p * n + q], apq = A[(long long)q * n + p],
                   aqq = A[(long long)q * n + q];
-    if (may_transform(app, aqp, apq, aqq)) {
-      double2 A2[4] = { app, aqp, apq, aqq }, U2[4], Z2[4];
-      int info = 0;
-      const int jp = a_is_p ? 1 : -1;  // "+" column a, "-" column b
-      zhsvd2(A2, jp, -jp, U2, Z2, JK_TH1FIX, info);
-      if (info < 0) w = nan_w();
-      else if (!(info & 1)) w = 0.0;
-      else if (!(info & 4)) w = dasum4(aqp.x, aqp.y, apq.x, apq.y);
-      else {
-        // the two off-diagonal terms that start ABODNZF2
-        const double2 a1 = (info & 8) ? A2[M21] : make_double2(0.0, 0.0);
-        const double2 a2 = (info & 8) ? A2[M12] : make_double2(0.0, 0.0);
-        d = 0.0;
-        d = fma(__dsub_rn(aqp.x, a1.x), __dadd_rn(aqp.x, a1.x), d);
-        d = fma(__dsub_rn(aqp.y, a1.y), __dadd_rn(aqp.y, a1.y), d);
-        d = fma(__dsub_rn(apq.x, a2.x), __dadd_rn(apq.x, a2.x), d);
-        d = fma(__dsub_rn(apq.y, a2.y), __dadd_rn(apq.y, a2.y), d);
-        t = zrot_ab(Z2);
-        scan = true;
-      }
-    }
+    scan = zhyp_setup(app, aqp, apq, aqq, a_is_p ? 1 : -1, w, d, t);
   }
   if (!__syncthreads_or(scan)) {
     if (valid) {
@@ -788,29 +721,12 @@ k_hyp_z_pm(const State *st, const double2 *__restrict__ A, const double *__restr
       h.flags = 0;
       h.d = 0.0;
       h.r1 = h.r2 = h.m1 = h.m2 = make_double2(0.0, 0.0);
-      double w = nan_w();
-      if (may_transform(app, aqp, apq, aqq)) {
-        double2 A2[4] = { app, aqp, apq, aqq }, U2[4], Z2[4];
-        int info = 0;
-        const int jp = ap ? 1 : -1;  // "+" column a, "-" column b
-        zhsvd2(A2, jp, -jp, U2, Z2, JK_TH1FIX, info);
-        if (info < 0) w = nan_w();
-        else if (!(info & 1)) w = 0.0;
-        else if (!(info & 4)) w = dasum4(aqp.x, aqp.y, apq.x, apq.y);
-        else {
-          // the four off-diagonal terms that start ABODNZF2
-          const double2 a1 = (info & 8) ? A2[M21] : make_double2(0.0, 0.0);
-          const double2 a2 = (info & 8) ? A2[M12] : make_double2(0.0, 0.0);
-          double d = 0.0;
-          d = fma(__dsub_rn(aqp.x, a1.x), __dadd_rn(aqp.x, a1.x), d);
-          d = fma(__dsub_rn(aqp.y, a1.y), __dadd_rn(aqp.y, a1.y), d);
-          d = fma(__dsub_rn(apq.x, a2.x), __dadd_rn(apq.x, a2.x), d);
-          d = fma(__dsub_rn(apq.y, a2.y), __dadd_rn(apq.y, a2.y), d);
-          const ZRot t = zrot_ab(Z2);
-          h.r1 = t.r1; h.r2 = t.r2; h.m1 = t.m1; h.m2 = t.m2;
-          h.flags = 1 | (t.c1 ? 2 : 0) | (t.c2 ? 4 : 0);
-          h.d = d;
-        }
+      double w, d = 0.0;
+      ZRot t;
+      if (zhyp_setup(app, aqp, apq, aqq, ap ? 1 : -1, w, d, t)) {
+        h.r1 = t.r1; h.r2 = t.r2; h.m1 = t.m1; h.m2 = t.m2;
+        h.flags = 1 | (t.c1 ? 2 : 0) | (t.c2 ? 4 : 0);
+        h.d = d;
       }
       tpar[slot] = h;
       if (!(h.flags & 1)) {
@@ -1243,15 +1159,16 @@ __device__ __forceinline__ void pivot_hsvd(State *st, const T *__restrict__ A, c
   RowRot<T> x;
   x.p = p; x.q = q; x.flags = 0;
   if (info >= 0) {
-#pragma unroll
-    for (int k = 0; k < 4; ++k) { pv.V[k] = V[k]; pv.W[k] = W[k]; }
     pv.d[0] = Tr<T>::re(B[M11]);
     pv.d[1] = Tr<T>::re(B[M22]);
     if (info & 2) {
       const typename Tr<T>::R t = Tr<T>::ba(V, quirk);
       x.flags = (t.c1 ? 1 : 0) | (t.c2 ? 2 : 0) | 4;
       x.r1 = t.r1; x.r2 = t.r2; x.m1 = t.m1; x.m2 = t.m2;
+      Tr<T>::ut2(V);
+      pv.tu = Tr<T>::ab(V);
     }
+    if (info & 4) pv.tz = Tr<T>::ab(W);
     if ((info & 1) && (info & 6)) atomicAdd(&st->nl, 1);
   }
   else
@@ -1846,8 +1763,7 @@ k_rotate(const State *st, T *__restrict__ A, T *__restrict__ U, T *__restrict__ 
     const Piv<T> &pv = piv[k];
     const int info = pv.info;
     if (info & 4) {
-      T W[4] = { pv.W[0], pv.W[1], pv.W[2], pv.W[3] };
-      const typename Tr<T>::R t = Tr<T>::ab(W);
+      const typename Tr<T>::R t = pv.tz;
       for (int i = threadIdx.x; i < n; i += blockDim.x) Tr<T>::apply_ab(t, col[i], col[n + i]);
     }
     __syncthreads();
@@ -1871,9 +1787,7 @@ k_rotate(const State *st, T *__restrict__ A, T *__restrict__ U, T *__restrict__ 
   const int info = pv.info;
   if (info < 0) return;
   if (info & 2) {
-    T V[4] = { pv.V[0], pv.V[1], pv.V[2], pv.V[3] };
-    Tr<T>::ut2(V);
-    const typename Tr<T>::R t = Tr<T>::ab(V);
+    const typename Tr<T>::R t = pv.tu;
     T *u0 = U + (long long)c0 * n, *u1 = U + (long long)c1 * n;
     for (int i = threadIdx.x; i < n; i += blockDim.x) {
       T x = u0[i], y = u1[i];
@@ -1882,8 +1796,7 @@ k_rotate(const State *st, T *__restrict__ A, T *__restrict__ U, T *__restrict__ 
     }
   }
   if (info & 4) {
-    T W[4] = { pv.W[0], pv.W[1], pv.W[2], pv.W[3] };
-    const typename Tr<T>::R t = Tr<T>::ab(W);
+    const typename Tr<T>::R t = pv.tz;
     T *z0 = Z + (long long)c0 * n, *z1 = Z + (long long)c1 * n;
     for (int i = threadIdx.x; i < n; i += blockDim.x) {
       T x = z0[i], y = z1[i];

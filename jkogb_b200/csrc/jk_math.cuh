@@ -501,149 +501,188 @@ __device__ __forceinline__ double hypot2_near(double x, double y)
   return (ea - eb > 54) ? a : __dmul_rn(h, pow2(ea));
 }
 
-// whether the exponents of a 2x2 block's nonzero entries allow the straight-line forms: all
-// within 2^-200 of the largest, which lies in 2^(+-300), and no zero column
-__device__ __forceinline__ bool near_block(const double A[4])
+// 2^-600, 2^600: a block scaled to its largest binade (2^1021) times the first is in quot's range
+__device__ __forceinline__ double down600(double x) { return __dmul_rn(x, 2.409919865102884e-181); }
+__device__ __forceinline__ double up600(double x) { return __dmul_rn(x, 4.149515568880993e+180); }
+
+__device__ __forceinline__ int bexp(double x) { return (__double2hiint(x) >> 20) & 0x7FF; }
+
+// a numerator that quot takes over a denominator in [2^-1, 2^1]: zero or at least 2^-960, so that
+// its remainder is a multiple of 2^-1074
+__device__ __forceinline__ bool quot_num(double a) { return bexp(a) >= 63 || a == 0.0; }
+
+// a/b for scaled entries a, b; ok is cleared when quot does not take them
+__device__ __forceinline__ double quot_scaled(double a, double b, double yb, bool &ok)
 {
-  int hi = 0, lo = 0x7FF;
-#pragma unroll
-  for (int k = 0; k < 4; ++k) {
-    const int e = (__double2hiint(A[k]) >> 20) & 0x7FF;
-    hi = max(hi, e);
-    lo = min(lo, (A[k] == 0.0) ? 0x7FF : e);
-  }
-  return hi >= 723 && hi <= 1323 && lo >= hi - 200 && (A[M11] != 0.0 || A[M21] != 0.0) && (A[M12] != 0.0 || A[M22] != 0.0);
+  const double x = down600(a), y = down600(b);
+  const int ex = bexp(x), ey = bexp(y);
+  ok = ok && ey >= 123 && (a == 0.0 || (ex >= 123 && ex - ey >= -1000));
+  return quot(x, y, yb);
 }
 
-// zero or at least 2^-300
-__device__ __forceinline__ bool near_ratio(double x) { return x == 0.0 || x >= 4.909093465297727e-91; }
+// hypot2 of scaled entries, not both zero (2^-600 times the smaller one is exact or too small to count)
+__device__ __forceinline__ double hypot2_scaled(double x, double y) { return up600(hypot2_near(down600(x), down600(y))); }
 
 // the factors of a triangle: the left rotation [cu, tu; -tu, cu] and the right one [cz, c12; tz, cz]
-// (each still to be divided by its cosine's inverse cu, cz), the reciprocals of cu, cz, the new
-// diagonal
+// (each still to be divided by cu, cz), the reciprocals of cu, cz, the new diagonal
 struct NearK {
   double tu, tz, c12, cu, cz, yu, yz, g0, g1;
 };
 
-// KHSVD2, src/shared/ktransf.F90:15-217, on an unscaled nonnegative triangle.  An upper one
-// [a, b; 0, c] takes T (equal signs) or U, a lower one [c, 0; b, a] (unequal signs) L.  Returns
-// false for KHSVD2's argument errors, for INFO -10 and -11 and for operands that the
-// straight-line forms do not take.
-__device__ __forceinline__ bool khsvd2_near(const double A[4], const int J0, const int J1, double th1, int &info, NearK &k)
+// KHSVD2, src/shared/ktransf.F90:15-217, on a nonnegative triangle scaled by 2^s.  An upper one
+// [a, b; 0, c] takes T (equal signs) or U, a lower one [c, 0; b, a] (unequal signs) L.  One straight line:
+// ok is cleared for KHSVD2's argument errors, for INFO -10 and -11 and for operands that the
+// straight-line forms do not take (a vanishing denominator, a new diagonal below 2^-1000).
+__device__ __forceinline__ void khsvd2_near(const double A[4], const bool tg, int s, double th1, int &info, NearK &k, bool &ok)
 {
   const bool upper = (A[M21] == 0.0);
-  if (!upper && (A[M12] != 0.0 || J0 == J1)) return false;  // the argument errors of KHSVD2
   const double a = upper ? A[M11] : A[M22], b = upper ? A[M12] : A[M21], c = upper ? A[M22] : A[M11];
-  const double ya = recip(a);
-  const double x = fmax(quot(b, a, ya), 0.0), y = fmax(quot(c, a, ya), 0.0);
-  if (!(a > 0.0) || !(b >= 0.0) || !(c >= 0.0) || !near_ratio(x) || !near_ratio(y)) return false;
-  const bool tg = (J0 == J1);
+  ok = ok && (upper || (A[M12] == 0.0 && !tg)) && a > 0.0 && b >= 0.0 && c >= 0.0;
+  const double as = down600(a), cs = down600(c), ya = recip(as);
+  const double x = fmax(quot_scaled(b, a, ya, ok), 0.0), y = fmax(quot_scaled(c, a, ya, ok), 0.0);
   const double nu = __dmul_rn(__dmul_rn(fmin(x, y), 2.0), fmax(x, y));
   const double de = fma(tg ? __dsub_rn(x, y) : __dsub_rn(y, x), __dadd_rn(x, y), 1.0);
-  if (!(de >= 8.881784197001252e-16)) return false;  // (unequal signs: also a vanishing or negative denominator)
-  double t2 = fmin(quot(nu, de, recip(de)), twof());
-  if (t2 > 1e100) return false;
+  // (the quotient times 2^200, so that a tiny numerator's remainder is exact)
+  const double up = 1.6069380442589903e60, dn = 6.223015277861142e-61;
+  const double t2 = fmin(__dmul_rn(quot(__dmul_rn(nu, up), de, recip(de)), dn), twof());
+  ok = ok && (nu == 0.0 || bexp(nu) >= 23) && de >= 8.881784197001252e-16 && t2 <= 1e100;
   const double q2 = __dadd_rn(1.0, root(fma(t2, t2, 1.0)));
   double tu = quot(t2, q2, recip(q2));  // |tan| of the left rotation
-  double tz, cz;
   const double cu = root(fma(tu, tu, 1.0));
-  if (tg) {
-    tz = fma(y, tu, x);
-    cz = root(fma(tz, tz, 1.0));
-  }
-  else {
-    if (upper) tu = -tu;
-    tz = fma(y, tu, upper ? x : -x);
-    if (upper) tz = -tz;
-    const double at = fabs(tz);
-    if (at >= 1.0) return false;  // INFO -10, -11
-    if (at >= th1) { tz = copysign(JK_TH1FIX, tz); info += 8; }
-    cz = root(fma(-tz, tz, 1.0));
-  }
+  tu = (!tg && upper) ? -tu : tu;
+  const double f = fma(y, tu, (tg || upper) ? x : -x);  // T: tz; U: -tz; L: tz
+  double tz = (!tg && upper) ? -f : f;
+  const double at = fabs(tz);
+  const bool cut = !tg && at >= th1;
+  ok = ok && (tg || at < 1.0);
+  tz = cut ? copysign(JK_TH1FIX, tz) : tz;
+  info += cut ? 8 : 0;
+  const double cz = root(fma(tg ? tz : -tz, tz, 1.0));
   const double yu = recip(cu), yz = recip(cz);
-  double g0 = 0.0, g1 = 0.0;
-  if (!(info & 8)) {
-    const double w = tg ? quot(cz, cu, yu) : quot(cu, cz, yz);
-    const double m = __dmul_rn(tg ? a : c, w), dv = quot(tg ? c : a, w, recip(w));
-    // T: G = (a w, c / w); U: (a / w, c w); L (a = A22, c = A11): (c w, a / w)
-    g0 = tg ? m : (upper ? dv : m);
-    g1 = tg ? dv : (upper ? m : dv);
-  }
-  k.tu = tu; k.tz = tz; k.c12 = tg ? -tz : tz; k.cu = cu; k.cz = cz; k.yu = yu; k.yz = yz; k.g0 = g0; k.g1 = g1;
-  return true;
+  const double w = quot(tg ? cz : cu, tg ? cu : cz, tg ? yu : yz);
+  const double m = __dmul_rn(tg ? as : cs, w), dv = quot(tg ? cs : as, w, recip(w));
+  // the original multiplies or divides and scales with one rounding; so does this while the results
+  // are normal
+  const int em = bexp(m), ed = bexp(dv);
+  ok = ok && (cut || ((m == 0.0 || (em >= 123 && em + 600 - s >= 23)) && (dv == 0.0 || (ed >= 123 && ed + 600 - s >= 23))));
+  const double f1 = pow2(600 - s), m1 = __dmul_rn(m, f1), dv1 = __dmul_rn(dv, f1);
+  // T: G = (a w, c / w); U: (a / w, c w); L (a = A22, c = A11): (c w, a / w)
+  const bool mf = tg || !upper;
+  k.g0 = mf ? m1 : dv1;
+  k.g1 = mf ? dv1 : m1;
+  k.tu = tu; k.tz = tz; k.c12 = tg ? -tz : tz; k.cu = cu; k.cz = cz; k.yu = yu; k.yz = yz;
 }
 
-// DHSVD2 for the blocks that near_block takes: the operations of dhsvd2_any in the same order on
-// the unscaled block.  Scaling by a power of two changes no bit of any result while every
-// result stays normal, which near_block and the test of the two ratios x, y ensure (products
-// of three entries, U and Z stay above 2^-900).  Returns false, with nothing written, when the
-// block or its ratios do not allow it.
+// quotients by the same number b in [2^-1, 2^1], y = recip(b); by 1 they are exact for every numerator
+template <int N>
+__device__ __forceinline__ void quots(double *a, double b, double y, bool &ok)
+{
+  bool num = true;
+#pragma unroll
+  for (int k = 0; k < N; ++k) {
+    num = num && quot_num(a[k]);
+    a[k] = quot(a[k], b, y);
+  }
+  ok = ok && (num || b == 1.0);
+}
+
+// A := B A with B = [c, t; -t, c] / c^2 (C2A, src/D/dtransf.F90:87-100)
+__device__ __forceinline__ void c2a_near(double t, double c, double y, double A[4], bool &ok)
+{
+  double v[4] = { fma(t, A[M21], A[M11]), fma(-t, A[M11], A[M21]), fma(t, A[M22], A[M12]), fma(-t, A[M12], A[M22]) };
+  quots<4>(v, c, y, ok);
+#pragma unroll
+  for (int k = 0; k < 4; ++k) A[k] = v[k];
+}
+
+// A := A B with B = [c, t12; t21, c] / c^2 (A2C, src/D/dtransf.F90:104-117)
+__device__ __forceinline__ void a2c_near(double A[4], double t21, double t12, double c, double y, bool &ok)
+{
+  double v[4] = { fma(A[M12], t21, A[M11]), fma(A[M22], t21, A[M21]), fma(A[M11], t12, A[M12]), fma(A[M21], t12, A[M22]) };
+  quots<4>(v, c, y, ok);
+#pragma unroll
+  for (int k = 0; k < 4; ++k) A[k] = v[k];
+}
+
+__device__ __forceinline__ void cswap(bool c, double &a, double &b) { const double t = a; a = c ? b : a; b = c ? t : b; }
+__device__ __forceinline__ double cneg(bool c, double a) { return c ? -a : a; }
+
+// DHSVD2 for a block without a zero column whose largest entry lies in 2^(+-300): the operations
+// of dhsvd2_any in the same order on the block scaled as there, with the straight-line division,
+// square root and magnitude and with selects for the swaps and sign changes.  Off-diagonal entries
+// shrink to zero through the whole exponent range before a loop ends (in a quarter of all blocks of a
+// solve they are below 2^-200 of the diagonal); the forms hold down to about 2^-1000 of it.
+// Returns false, with nothing written, when the block does not allow it.
 __device__ __forceinline__ bool dhsvd2_near(double Ain[4], const int J0, const int J1, double Uo[4], double Zo[4], double th1, int &info_o)
 {
-  if (!near_block(Ain) || abs(J0) != 1 || abs(J1) != 1) return false;
-  double A[4] = { Ain[0], Ain[1], Ain[2], Ain[3] }, U[4] = { 1.0, 0.0, 0.0, 1.0 }, Z[4] = { 1.0, 0.0, 0.0, 1.0 };
-  int info;
+  const int hi = max(max(bexp(Ain[0]), bexp(Ain[1])), max(bexp(Ain[2]), bexp(Ain[3])));
+  if (hi < 723 || hi > 1323 || (Ain[M11] == 0.0 && Ain[M21] == 0.0) || (Ain[M12] == 0.0 && Ain[M22] == 0.0) ||
+      abs(J0) != 1 || abs(J1) != 1) return false;
+  bool ok = true;
+  const bool tg = (J0 == J1);
+  const int s = 2044 - hi;  // DSCALEA's
+  const double fs = pow2(s - 600);
+  double A[4], U[4] = { 1.0, 0.0, 0.0, 1.0 }, Z[4] = { 1.0, 0.0, 0.0, 1.0 };
+#pragma unroll
+  for (int k = 0; k < 4; ++k) A[k] = up600(__dmul_rn(Ain[k], fs));
   // DHSVD2T, src/D/dtransf.F90:352-532
+  const bool d = (A[M21] == 0.0) && (A[M12] == 0.0);
+  const double c = hypot2_scaled(A[M11], A[M21]), t0 = hypot2_scaled(A[M12], A[M22]);
+  const bool p = (c < t0);
+  const double r = p ? t0 : c;
+  cswap(p, A[M11], A[M12]); cswap(p, A[M21], A[M22]);
+  cswap(p && tg, Z[M11], Z[M12]); cswap(p && tg, Z[M21], Z[M22]);
+  const bool n1 = neg(A[M11]), n2 = neg(A[M21]);
+  U[M11] = cneg(n1, U[M11]); U[M12] = cneg(n1, U[M12]); A[M12] = cneg(n1, A[M12]); A[M11] = cneg(n1, A[M11]);
+  U[M21] = cneg(n2, U[M21]); U[M22] = cneg(n2, U[M22]); A[M22] = cneg(n2, A[M22]); A[M21] = cneg(n2, A[M21]);
+  const bool sw = (A[M11] < A[M21]);
+  cswap(sw, U[M11], U[M21]); cswap(sw, U[M12], U[M22]);
+  cswap(sw, A[M11], A[M21]); cswap(sw, A[M12], A[M22]);
   {
-    const bool d = (A[M21] == 0.0) && (A[M12] == 0.0);
-    const double c = hypot2_near(A[M11], A[M21]), s = hypot2_near(A[M12], A[M22]);
-    const bool p = (c < s);
-    const double r = p ? s : c;
-    if (p) {
-      dswap(A[M11], A[M12]); dswap(A[M21], A[M22]);
-      if (J0 == J1) { dswap(Z[M11], Z[M12]); dswap(Z[M21], Z[M22]); }
-    }
-    if (neg(A[M11])) { U[M11] = -U[M11]; U[M12] = -U[M12]; A[M12] = -A[M12]; A[M11] = -A[M11]; }
-    if (neg(A[M21])) { U[M21] = -U[M21]; U[M22] = -U[M22]; A[M22] = -A[M22]; A[M21] = -A[M21]; }
-    if (A[M11] < A[M21]) {
-      dswap(U[M11], U[M21]); dswap(U[M12], U[M22]);
-      dswap(A[M11], A[M21]); dswap(A[M12], A[M22]);
-    }
-    if (!d) {
-      const double t = quot(A[M21], A[M11], recip(A[M11]));
-      const double q = root(fma(t, t, 1.0)), y = recip(q);
-      const double u11 = fma(t, U[M21], U[M11]), u21 = fma(-t, U[M11], U[M21]);
-      const double u12 = fma(t, U[M22], U[M12]), u22 = fma(-t, U[M12], U[M22]);
-      const double a1 = fma(t, A[M22], A[M12]), a2 = fma(-t, A[M12], A[M22]);
-      U[M11] = quot(u11, q, y); U[M21] = quot(u21, q, y); U[M12] = quot(u12, q, y); U[M22] = quot(u22, q, y);
-      A[M12] = quot(a1, q, y); A[M22] = quot(a2, q, y);
-    }
-    A[M11] = r;
-    A[M21] = 0.0;
-    if ((J0 != J1) && p) {
-      dswap(A[M11], A[M12]); dswap(A[M21], A[M22]);
-      dswap(U[M11], U[M21]); dswap(U[M12], U[M22]);
-      dswap(A[M11], A[M21]); dswap(A[M12], A[M22]);
-      if (neg(A[M21])) { Z[M11] = -Z[M11]; Z[M21] = -Z[M21]; A[M11] = -A[M11]; A[M21] = -A[M21]; }
-      if (neg(A[M11])) { U[M11] = -U[M11]; U[M12] = -U[M12]; A[M11] = -A[M11]; }
-    }
-    else {
-      if (neg(A[M12])) { Z[M12] = -Z[M12]; Z[M22] = -Z[M22]; A[M22] = -A[M22]; A[M12] = -A[M12]; }
-      if (neg(A[M22])) { U[M21] = -U[M21]; U[M22] = -U[M22]; A[M22] = -A[M22]; }
-    }
-    info = d ? 0 : 1;
+    const double t = quot_scaled(A[M21], A[M11], recip(down600(A[M11])), ok);
+    const double q = root(fma(t, t, 1.0)), y = recip(q);
+    double V[4] = { U[0], U[1], U[2], U[3] };
+    c2a_near(t, q, y, V, ok);
+    double v[2] = { fma(t, A[M22], A[M12]), fma(-t, A[M12], A[M22]) };  // C1A
+    quots<2>(v, q, y, ok);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) U[k] = d ? U[k] : V[k];
+    A[M12] = d ? A[M12] : v[0];
+    A[M22] = d ? A[M22] : v[1];
   }
-  if (info) {
+  A[M11] = r;
+  A[M21] = 0.0;
+  // unequal signs and swapped columns: rows and columns swapped back, a lower triangle
+  const bool lo = !tg && p;
+  cswap(lo, A[M11], A[M12]); cswap(lo, A[M21], A[M22]);
+  cswap(lo, U[M11], U[M21]); cswap(lo, U[M12], U[M22]);
+  cswap(lo, A[M11], A[M21]); cswap(lo, A[M12], A[M22]);
+  {
+    const bool m1 = neg(lo ? A[M21] : A[M12]);
+    Z[M11] = cneg(m1 && lo, Z[M11]); Z[M21] = cneg(m1 && lo, Z[M21]);
+    Z[M12] = cneg(m1 && !lo, Z[M12]); Z[M22] = cneg(m1 && !lo, Z[M22]);
+    A[M11] = cneg(m1 && lo, A[M11]); A[M21] = cneg(m1 && lo, A[M21]);
+    A[M22] = cneg(m1 && !lo, A[M22]); A[M12] = cneg(m1 && !lo, A[M12]);
+    const bool m2 = neg(lo ? A[M11] : A[M22]);
+    U[M11] = cneg(m2 && lo, U[M11]); U[M12] = cneg(m2 && lo, U[M12]); A[M11] = cneg(m2 && lo, A[M11]);
+    U[M21] = cneg(m2 && !lo, U[M21]); U[M22] = cneg(m2 && !lo, U[M22]); A[M22] = cneg(m2 && !lo, A[M22]);
+  }
+  int info = d ? 0 : 1;
+  if (d) { A[M11] = scale(A[M11], -s); A[M22] = scale(A[M22], -s); }
+  else {
     NearK k;
-    if (!khsvd2_near(A, J0, J1, th1, info, k)) return false;
-    const double tu = k.tu, tz = k.tz, c12 = k.c12, cu = k.cu, cz = k.cz, yu = k.yu, yz = k.yz;
-    // C2A(B, U) with B = [cu, tu; -tu, cu], A2C(Z, C) with C = [cz, C12; tz, cz]
-    const double u11 = fma(tu, U[M21], U[M11]), u21 = fma(-tu, U[M11], U[M21]);
-    const double u12 = fma(tu, U[M22], U[M12]), u22 = fma(-tu, U[M12], U[M22]);
-    U[M11] = quot(u11, cu, yu); U[M21] = quot(u21, cu, yu); U[M12] = quot(u12, cu, yu); U[M22] = quot(u22, cu, yu);
-    const double z11 = fma(Z[M12], tz, Z[M11]), z12 = fma(Z[M11], c12, Z[M12]);
-    const double z21 = fma(Z[M22], tz, Z[M21]), z22 = fma(Z[M21], c12, Z[M22]);
-    Z[M11] = quot(z11, cz, yz); Z[M12] = quot(z12, cz, yz); Z[M21] = quot(z21, cz, yz); Z[M22] = quot(z22, cz, yz);
+    khsvd2_near(A, tg, s, th1, info, k, ok);
+    c2a_near(k.tu, k.cu, k.yu, U, ok);
+    a2c_near(Z, k.tz, k.c12, k.cz, k.yz, ok);
     if (!(info & 8)) { A[M11] = k.g0; A[M22] = k.g1; }
     else {
-      const double a11 = fma(tu, A[M21], A[M11]), a21 = fma(-tu, A[M11], A[M21]);
-      const double a12 = fma(tu, A[M22], A[M12]), a22 = fma(-tu, A[M12], A[M22]);
-      A[M11] = quot(a11, cu, yu); A[M21] = quot(a21, cu, yu); A[M12] = quot(a12, cu, yu); A[M22] = quot(a22, cu, yu);
-      const double b11 = fma(A[M12], tz, A[M11]), b12 = fma(A[M11], c12, A[M12]);
-      const double b21 = fma(A[M22], tz, A[M21]), b22 = fma(A[M21], c12, A[M22]);
-      A[M11] = quot(b11, cz, yz); A[M12] = quot(b12, cz, yz); A[M21] = quot(b21, cz, yz); A[M22] = quot(b22, cz, yz);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) A[i] = scale(A[i], -s);
+      c2a_near(k.tu, k.cu, k.yu, A, ok);
+      a2c_near(A, k.tz, k.c12, k.cz, k.yz, ok);
     }
   }
+  if (!ok) return false;
   dhsvd2s(A, J0, J1, U, Z, info);
 #pragma unroll
   for (int k = 0; k < 4; ++k) { Ain[k] = A[k]; Uo[k] = U[k]; Zo[k] = Z[k]; }
@@ -676,13 +715,12 @@ struct Rot {
   int c1, c2;
 };
 
-// n1/d1 and n2/d2, as straight-line code when the operands allow it
+// n1/d1 and n2/d2, |n| <= |d|, as straight-line code when the operands allow it
 __device__ __forceinline__ void div2(double n1, double d1, double n2, double d2, double &r1, double &r2)
 {
-  const int e1 = (__double2hiint(d1) >> 20) & 0x7FF, e2 = (__double2hiint(d2) >> 20) & 0x7FF;
-  const double lim = 1.9010857885610293e-211;  // 2^-700
-  const bool ok = (n1 == 0.0 || fabs(n1) >= lim) && (n2 == 0.0 || fabs(n2) >= lim) && imin(e1, e2) >= 723 &&
-                  max(e1, e2) <= 1323 && fabs(n1) <= fabs(d1) && fabs(n2) <= fabs(d2);
+  const int e1 = bexp(d1), e2 = bexp(d2);
+  const bool ok = (quot_num(n1) || fabs(d1) == 1.0) && (quot_num(n2) || fabs(d2) == 1.0) && imin(e1, e2) >= 1013 &&
+                  max(e1, e2) <= 1033 && fabs(n1) <= fabs(d1) && fabs(n2) <= fabs(d2);
   if (ok) {
     r1 = quot(n1, d1, recip(d1));
     r2 = quot(n2, d2, recip(d2));

@@ -1,0 +1,139 @@
+// jk_scan.cuh -- the sequential column scans of the hyperbolic pair weights (ABODNDF2, ABODNZF2) as
+// one thread runs them for one pair, and the 2x2 part of the complex weight.
+#pragma once
+
+#include "jk_device.cuh"
+
+namespace jk {
+
+// ABODNDF2's sum as scan_rows_real, for any branches of the rotation
+__device__ __forceinline__ void scan_rows_any(const double *xs, const double *ys, int rows, int i0, int p, int q, const Rot &t, double &d)
+{
+  for (int r = 0; r < rows; ++r) {
+    double x = xs[r], y = ys[r];
+    const double x0 = x, y0 = y;
+    rot_apply(t, x, y);
+    const int i = i0 + r;
+    if (i != p && i != q) {
+      d = fma(__dsub_rn(x0, x), __dadd_rn(x0, x), d);
+      d = fma(__dsub_rn(y0, y), __dadd_rn(y0, y), d);
+    }
+  }
+}
+
+// ABODNDF2's sum (src/D/dtransf.F90:246-348) over the rows i0 .. i0 + rows - 1 without p, q of
+// the columns xs (p), ys (q).  Its two fused multiply-adds per row are one dependent chain (46 cycles a
+// row); the four differences and sums they take are formed four rows ahead of it.
+__device__ __forceinline__ void scan_rows_real(const double *xs, const double *ys, int rows, int i0, int p, int q, const Rot &t, double &d)
+{
+  if (t.c1 && t.c2) {
+    struct Terms { double s1, a1, s2, a2; };
+    auto terms = [&](int r) {
+      const double x = xs[r], y = ys[r];
+      const double xx = __dmul_rn(fma(y, t.r1, x), t.m1);
+      const double yy = __dmul_rn(fma(x, t.r2, y), t.m2);
+      return Terms{ __dsub_rn(x, xx), __dadd_rn(x, xx), __dsub_rn(y, yy), __dadd_rn(y, yy) };
+    };
+    auto add = [&](const Terms &v, int r) {
+      const int i = i0 + r;
+      if (i != p && i != q) {
+        d = fma(v.s1, v.a1, d);
+        d = fma(v.s2, v.a2, d);
+      }
+    };
+    constexpr int G = 4;
+    const int full = rows - rows % G;
+    Terms v[G];
+    if (full > 0) {
+#pragma unroll
+      for (int k = 0; k < G; ++k) v[k] = terms(k);
+    }
+#pragma unroll 2
+    for (int r = 0; r < full; r += G) {
+      Terms u[G];
+      const int nx = (r + G < full) ? r + G : r;  // (the last group is formed once more)
+#pragma unroll
+      for (int k = 0; k < G; ++k) u[k] = terms(nx + k);
+#pragma unroll
+      for (int k = 0; k < G; ++k) add(v[k], r + k);
+#pragma unroll
+      for (int k = 0; k < G; ++k) v[k] = u[k];
+    }
+    for (int r = full; r < rows; ++r) add(terms(r), r);
+  }
+  else scan_rows_any(xs, ys, rows, i0, p, q, t, d);
+}
+
+// hypot2 out of line: the rare operands hypot2_near does not take
+static __device__ __noinline__ double hypot2_call(double x, double y) { return hypot2(x, y); }
+
+// whether zabs_near takes an entry: the larger part within 2^(+-998) (a NaN in the other part
+// passes through), or both parts zero
+__device__ __forceinline__ bool scan_near(double2 a)
+{
+  const double u = fmax(fabs(a.x), fabs(a.y));
+  return (u >= 3.7e-301 && u <= 2.6e300) || u == 0.0;
+}
+
+// ABODNZF2's sum (src/Z/ztransf.F90:452-637) with the magnitudes of the unrotated entries taken from
+// xa, ya.  Two rows at a time, so that the square roots and divisions of four magnitudes overlap.
+__device__ __forceinline__ void scan_rows_cplx_mag(const double2 *xs, const double2 *ys, const double *xa, const double *ya,
+                                                   int rows, int i0, int p, int q, const ZRot &t, double &d)
+{
+  constexpr int G = 2;
+  for (int r = 0; r < rows; r += G) {
+    double2 x[G], y[G];
+    double mx[G], my[G];
+    bool near = true;
+#pragma unroll
+    for (int k = 0; k < G; ++k) {
+      const int e = min(r + k, rows - 1);
+      x[k] = xs[e];
+      y[k] = ys[e];
+      zrot_apply_ab(t, x[k], y[k]);
+      near = near && scan_near(x[k]) && scan_near(y[k]);
+    }
+    if (near) {
+#pragma unroll
+      for (int k = 0; k < G; ++k) { mx[k] = zabs_near(x[k]); my[k] = zabs_near(y[k]); }
+    }
+    else {
+#pragma unroll
+      for (int k = 0; k < G; ++k) { mx[k] = hypot2_call(x[k].x, x[k].y); my[k] = hypot2_call(y[k].x, y[k].y); }
+    }
+#pragma unroll
+    for (int k = 0; k < G; ++k) {
+      const int i = i0 + r + k;
+      if (r + k < rows && i != p && i != q) {
+        const double axi = xa[r + k], ayi = ya[r + k];
+        d = fma(__dsub_rn(axi, mx[k]), __dadd_rn(axi, mx[k]), d);
+        d = fma(__dsub_rn(ayi, my[k]), __dadd_rn(ayi, my[k]), d);
+      }
+    }
+  }
+}
+
+// hyp_setup for a complex pair (ZMAGF2H, src/Z/zstep.F90:43-74)
+__device__ __forceinline__ bool zhyp_setup(double2 app, double2 aqp, double2 apq, double2 aqq, int jp, double &w, double &d, ZRot &t)
+{
+  w = nan_w();
+  if (!may_transform(app, aqp, apq, aqq)) return false;
+  double2 A2[4] = { app, aqp, apq, aqq }, U2[4], Z2[4];
+  int info = 0;
+  zhsvd2(A2, jp, -jp, U2, Z2, JK_TH1FIX, info);
+  if (info < 0) return false;
+  if (!(info & 1)) { w = 0.0; return false; }
+  if (!(info & 4)) { w = dasum4(aqp.x, aqp.y, apq.x, apq.y); return false; }
+  // the four off-diagonal terms that start ABODNZF2
+  const double2 a1 = (info & 8) ? A2[M21] : make_double2(0.0, 0.0);
+  const double2 a2 = (info & 8) ? A2[M12] : make_double2(0.0, 0.0);
+  d = 0.0;
+  d = fma(__dsub_rn(aqp.x, a1.x), __dadd_rn(aqp.x, a1.x), d);
+  d = fma(__dsub_rn(aqp.y, a1.y), __dadd_rn(aqp.y, a1.y), d);
+  d = fma(__dsub_rn(apq.x, a2.x), __dadd_rn(apq.x, a2.x), d);
+  d = fma(__dsub_rn(apq.y, a2.y), __dadd_rn(apq.y, a2.y), d);
+  t = zrot_ab(Z2);
+  return true;
+}
+
+}  // namespace jk

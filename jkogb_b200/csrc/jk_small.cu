@@ -1,0 +1,512 @@
+// jk_small.cu -- the step loop of one small matrix (real and complex) in one persistent
+// launch: a cluster of blocks runs the whole loop of DSTEP_LOOP / ZSTEP_LOOP
+// (src/D/dstep.F90:564-583, src/Z/zstep.F90:575-594) from shared memory.
+//
+// A step of a small matrix is a chain of short dependent phases.  As five launches it took 50 us at
+// N = 16 and 71 us at N = 97, nearly all of it launch gaps, loads through L2 and instruction
+// fetches of code that runs once per launch (a 2x2 HSVD: 10000 cycles in a fresh launch, 2200 in
+// a loop).
+//
+// Every block keeps a replica of A and of the step's weight keys and does the selection, the pivots
+// and the rotations of A for itself; only the hyperbolic weights, the one phase whose work grows with
+// N^3, are divided among the blocks, a pair per thread, and their keys written to every
+// replica through distributed shared memory: one exchange per step.  The rows of U and Z are divided
+// among the blocks.  All blocks compute the same values, so that they take the same decisions.
+//   weights    DMAGF2H / ZMAGF2H of the block's share of the pairs (ABODNDF2 / ABODNZF2's sequential
+//              sums); DMAGF2T / ZMAGF2T of all pairs by the threads without a share
+//   selection  the greedy matching in rounds of mutual best proposals: a warp finds a vertex's best
+//              free partner among all keys (no sorted lists)
+//   pivots     the 2x2 HSVDs, a thread each
+//   rotations  BA, then AB and the diagonal write-back on A; the columns of U and Z
+//   loop test  SL := MIN(SL, NL), S, INFO
+#include <cooperative_groups.h>
+
+#include "jk_internal.h"
+#include "jk_device.cuh"
+#include "jk_scan.cuh"
+
+namespace cg = cooperative_groups;
+
+namespace jk {
+
+namespace {
+
+template <typename T>
+struct SPiv {
+  typename Tr<T>::R ba, tu, tz;  // rows of A; columns of U; columns of A and Z
+  double d0, d1;                 // the new diagonal
+  int p, q, info, pad;
+};
+
+__host__ __device__ __forceinline__ size_t al16(size_t x) { return (x + 15) & ~(size_t)15; }
+__host__ __device__ __forceinline__ int tri2(int i, int j) { return (j * (j - 1)) / 2 + i; }  // i < j
+
+// shared memory of one block
+struct SLayout {
+  int lda, m;  // stride of A's columns and of the keys' rows (odd: a warp's lanes in distinct banks); rows of U, Z
+  size_t a, mag, k, u, z, piv, pairs, rk, pos, vl, jv, cand, total;
+  template <typename T>
+  __host__ __device__ static SLayout make(int n, int C)
+  {
+    SLayout L;
+    L.lda = n | 1;
+    L.m = (n + C - 1) / C;
+    L.a = 0;
+    L.mag = al16(L.a + (size_t)n * L.lda * sizeof(T));
+    L.k = al16(L.mag + (sizeof(T) == 16 ? (size_t)n * L.lda * 8 : 0));
+    L.u = al16(L.k + ((size_t)n * L.lda + 32) * 8);  // (a row is read in whole warps)
+    L.z = L.u + (size_t)n * L.m * sizeof(T);
+    L.piv = al16(L.z + (size_t)n * L.m * sizeof(T));
+    L.pairs = al16(L.piv + (size_t)(n / 2 + 1) * sizeof(SPiv<T>));
+    L.rk = L.pairs + (size_t)(n / 2 + 1) * 8;
+    L.pos = L.rk + (size_t)(n / 2 + 1) * 4;
+    L.vl = L.pos + (size_t)n * 4;
+    L.jv = L.vl + (size_t)n * 4;
+    L.cand = L.jv + (size_t)n * 4;
+    L.total = L.cand + (size_t)n * 4;
+    return L;
+  }
+};
+
+constexpr int kSmallMaxN = 128;  // bound of the free-bit words (the shared memory ends before it)
+constexpr size_t kSmallSmem = 227 * 1024 - 512;
+
+// a thread's share of a hyperbolic pair: p < q with columns x (p) and y (q)
+__device__ __forceinline__ double hyp_weight(const double *x, const double *y, const double *, const double *, int n, int p,
+                                             int q, int jp)
+{
+  double w, d = 0.0;
+  Rot t;
+  if (hyp_setup(x[p], x[q], y[p], y[q], jp, w, d, t)) {
+    scan_rows_real(x, y, n, 0, p, q, t, d);
+    w = d;
+  }
+  return (w < -JK_HUGE) ? nan_w() : w;
+}
+
+__device__ __forceinline__ double hyp_weight(const double2 *x, const double2 *y, const double *xa, const double *ya, int n,
+                                             int p, int q, int jp)
+{
+  double w, d = 0.0;
+  ZRot t;
+  if (zhyp_setup(x[p], x[q], y[p], y[q], jp, w, d, t)) {
+    scan_rows_cplx_mag(x, y, xa, ya, n, 0, p, q, t, d);
+    w = d;
+  }
+  return (w < -JK_HUGE) ? nan_w() : w;
+}
+
+template <typename T, int THREADS>
+__global__ void __launch_bounds__(THREADS, 1)
+k_small(State *st, T *__restrict__ gA, T *__restrict__ gU, T *__restrict__ gZ, const int *__restrict__ gJ, int n, int np,
+        int n_2, int quirk, int budget)
+{
+  cg::cluster_group cluster = cg::this_cluster();
+  const int C = (int)cluster.num_blocks(), c = (int)cluster.block_rank();
+  const bool solo = (C == 1);
+  extern __shared__ __align__(16) unsigned char smem[];
+  const SLayout L = SLayout::make<T>(n, C);
+  T *As = (T *)(smem + L.a), *Us = (T *)(smem + L.u), *Zs = (T *)(smem + L.z);
+  double *mag = (double *)(smem + L.mag);
+  unsigned long long *Ks = (unsigned long long *)(smem + L.k);  // keys by position, symmetric, 0 on the diagonal
+  SPiv<T> *pv = (SPiv<T> *)(smem + L.piv);
+  int2 *pairs = (int2 *)(smem + L.pairs);  // positions (i, j)
+  int *rk = (int *)(smem + L.rk), *pos = (int *)(smem + L.pos), *vl = (int *)(smem + L.vl), *Jv = (int *)(smem + L.jv),
+      *cand = (int *)(smem + L.cand);
+  __shared__ unsigned s_free[kSmallMaxN / 32], s_first[kSmallMaxN / 32];
+  __shared__ int s_nl, s_err;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, NW = THREADS / 32;
+  const int nm = n - np, lda = L.lda, m = L.m, r0 = c * m, mr = max(0, min(m, n - r0));
+  constexpr bool kCplx = (sizeof(T) == 16);
+
+  if (*(volatile int *)&st->stop) return;
+  const long long limit = st->limit;
+  int steps = st->steps;
+
+  // the positions of the vertices (+ columns first), A, this block's rows of U and Z
+  if (warp == 0) {
+    int k = 0;
+    for (int s = 1; s >= -1; s -= 2)
+      for (int b = 0; b < n; b += 32) {
+        const int v = b + lane;
+        const bool in = (v < n) && gJ[v] == s;
+        const unsigned bal = __ballot_sync(0xFFFFFFFFu, in);
+        if (in) {
+          const int i = k + __popc(bal & ((1u << lane) - 1u));
+          pos[v] = i;
+          vl[i] = v;
+          Jv[v] = s;
+        }
+        k += __popc(bal);
+      }
+  }
+  __syncthreads();
+  for (int k = tid; k < n * n; k += THREADS) {
+    const int i = k % n, j = k / n;
+    As[pos[j] * lda + i] = gA[k];
+  }
+  for (int k = tid; k < n * mr; k += THREADS) {
+    const int i = k % mr, j = k / mr;
+    Us[j * m + i] = gU[(long long)j * n + r0 + i];
+    Zs[j * m + i] = gZ[(long long)j * n + r0 + i];
+  }
+  // this block's share of the hyperbolic pairs (+ column, - column), and the threads without one,
+  // who take the trigonometric pairs (all threads, where no quarter of them is idle)
+  const int nh = np * nm, per = (nh + C - 1) / C, h0 = c * per, h1 = min(nh, h0 + per);
+  const int busy = min((max(h1 - h0, 0) + 31) & ~31, THREADS);
+  const int t0 = (THREADS - busy >= THREADS / 4) ? busy : 0, tn = THREADS - t0;
+  const int ntp = np * (np - 1) / 2, nt = ntp + nm * (nm - 1) / 2;
+  if (!solo) cluster.barrier_arrive();  // the replicas' keys may be written (every block is running)
+  else __syncthreads();
+  for (int i = tid; i < n; i += THREADS) Ks[i * lda + i] = 0ULL;
+  int stop = 0, info = 0;
+
+  for (int it = 0; it < budget && !stop; ++it) {
+    // ---- the magnitudes of the unrotated entries (complex)
+    __syncthreads();
+    if constexpr (kCplx) {
+#pragma unroll 4
+      for (int k = tid; k < n * lda; k += THREADS) {
+        const double2 a = As[k];
+        mag[k] = scan_near(a) ? zabs_near(a) : hypot2_call(a.x, a.y);
+      }
+      __syncthreads();
+    }
+    // ---- weights
+    if (tid >= t0)
+      for (int k = tid - t0; k < nt; k += tn) {
+        const bool plus = k < ntp;
+        const int kk = plus ? k : k - ntp;
+        int j = (int)((1.0f + sqrtf(8.0f * kk + 1.0f)) * 0.5f);
+        while (tri2(0, j) > kk) --j;
+        while (tri2(0, j + 1) <= kk) ++j;
+        const int i = kk - tri2(0, j), o = plus ? 0 : np;
+        const int p = vl[i + o], q = vl[j + o];  // ascending within a class
+        const T *ca = As + (i + o) * lda, *cb = As + (j + o) * lda;
+        const T app = ca[p], aqp = ca[q], apq = cb[p], aqq = cb[q];
+        const bool nz = may_transform(app, aqp, apq, aqq);
+        const double w = (nz || (plus ? Tr<T>::re(app) < Tr<T>::re(aqq) : Tr<T>::re(aqq) < Tr<T>::re(app)))
+                             ? Tr<T>::magt(aqp, apq) : nan_w();
+        Ks[(i + o) * lda + j + o] = Ks[(j + o) * lda + i + o] = wkey(w);
+      }
+    bool waited = solo;
+    for (int k = h0 + tid; k - tid < h1; k += THREADS) {
+      unsigned long long key = 0;
+      int ci = 0, cj = 0;
+      if (k < h1) {
+        ci = k / nm;
+        cj = k - ci * nm;
+        const int a = vl[ci], b = vl[np + cj];
+        const bool ap = a < b;
+        const int x = ap ? ci : np + cj, y = ap ? np + cj : ci;
+        key = wkey(hyp_weight(As + x * lda, As + y * lda, mag + x * lda, mag + y * lda, n, ap ? a : b, ap ? b : a, ap ? 1 : -1));
+      }
+      __syncwarp();
+      if (!waited) { cluster.barrier_wait(); waited = true; }  // every block is done with the last step's keys
+      if (k < h1) {
+        // (consecutive threads write consecutive entries; the transposed half is filled in place)
+        unsigned long long *e = Ks + ci * lda + np + cj;
+        if (solo) *e = key;
+        else
+          for (int r = 0; r < C; ++r) *cluster.map_shared_rank(e, r) = key;
+      }
+    }
+    if (!waited) cluster.barrier_wait();
+    // the matching starts with all vertices free
+    if (tid < (n + 31) / 32) s_free[tid] = (n - 32 * tid >= 32) ? 0xFFFFFFFFu : ((1u << (n - 32 * tid)) - 1u);
+    for (int i = tid; i < n; i += THREADS) cand[i] = -1;
+    if (tid == 0) { s_nl = 0; s_err = 0; }
+    if (solo) __syncthreads();
+    else cluster.sync();
+
+    for (int ci = warp; ci < np; ci += NW)
+      for (int cj = lane; cj < nm; cj += 32) Ks[(np + cj) * lda + ci] = Ks[ci * lda + np + cj];
+    __syncthreads();
+
+    // ---- selection: rounds of mutual best proposals (positions, not vertices).  The instructions
+    // issued count here: a row is four loads and the comparison of the high halves of its keys, their low
+    // halves and the tie rule among what is left.
+    for (int round = 0; round <= n / 2; ++round) {
+      constexpr int W = kSmallMaxN / 32;
+      unsigned fw[W];  // all ones where this lane's k-th position is free
+#pragma unroll
+      for (int k = 0; k < W; ++k) fw[k] = (32 * k < n) ? 0u - ((s_free[k] >> lane) & 1u) : 0u;
+      // the warp's vertices (warp + NW k) that are free and whose candidate is gone, one per lane; two rows
+      // at a time, so that their latencies overlap
+      bool need = false;
+      {
+        const int i = warp + NW * lane;
+        if (i < n && ((s_free[i >> 5] >> (i & 31)) & 1u)) {
+          const int u0 = cand[i];
+          need = u0 == -1 || (u0 >= 0 && !((s_free[u0 >> 5] >> (u0 & 31)) & 1u));
+        }
+      }
+      for (unsigned todo = __ballot_sync(0xFFFFFFFFu, need); todo;) {
+        int iv[2];
+        iv[0] = warp + NW * (__ffs(todo) - 1);
+        todo &= todo - 1u;
+        iv[1] = todo ? warp + NW * (__ffs(todo) - 1) : iv[0];
+        todo &= todo - 1u;
+        unsigned hi[2][W], lo[2][W], mh[2] = { 0u, 0u }, ml[2] = { 0u, 0u };
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const unsigned long long *row = Ks + iv[h] * lda + lane;
+#pragma unroll
+          for (int k = 0; k < W; ++k) {
+            // (a lane beyond the row's end reads another entry and drops it)
+            const unsigned long long x = (32 * k < n) ? row[32 * k] : 0ULL;
+            hi[h][k] = (unsigned)(x >> 32) & fw[k];
+            lo[h][k] = (unsigned)x & fw[k];
+            mh[h] = max(mh[h], hi[h][k]);
+          }
+        }
+#pragma unroll
+        for (int h = 0; h < 2; ++h) mh[h] = __reduce_max_sync(0xFFFFFFFFu, mh[h]);
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+#pragma unroll
+          for (int k = 0; k < W; ++k) ml[h] = max(ml[h], (hi[h][k] == mh[h]) ? lo[h][k] : 0u);
+        }
+#pragma unroll
+        for (int h = 0; h < 2; ++h) ml[h] = __reduce_max_sync(0xFFFFFFFFu, ml[h]);
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const int i = iv[h];
+          const bool none = (mh[h] | ml[h]) == 0u;  // (a key is never 0: no partner is left then)
+          int j = -2, eq = 0;
+#pragma unroll
+          for (int k = 0; k < W; ++k)
+            if (hi[h][k] == mh[h] && lo[h][k] == ml[h]) { j = 32 * k + lane; ++eq; }
+          const unsigned b = __ballot_sync(0xFFFFFFFFu, eq > 0), b2 = __ballot_sync(0xFFFFFFFFu, eq > 1);
+          if (!none && (b2 | (b & (b - 1u)))) {
+            // equal keys: the larger band, then the larger p
+            const int v = vl[i];
+            unsigned bt = 0u;
+#pragma unroll
+            for (int k = 0; k < W; ++k)
+              if (hi[h][k] == mh[h] && lo[h][k] == ml[h]) bt = max(bt, tkey(v, vl[32 * k + lane]));
+            bt = __reduce_max_sync(0xFFFFFFFFu, bt);
+            const int p = (int)(bt & 0xFFFFu), q = p + (int)(bt >> 16);
+            if (lane == 0) cand[i] = pos[p == v ? q : p];
+          }
+          else if (none ? lane == 0 : eq > 0) cand[i] = none ? -2 : j;
+        }
+      }
+      __syncthreads();
+      // both ends of a mutual proposal see it
+      bool got = false;
+      if (32 * warp < n) {
+        const unsigned f = s_free[warp];
+        const int u = (tid < n) ? cand[tid] : -2;
+        got = ((f >> lane) & 1u) && u >= 0 && cand[u] == tid;
+        const unsigned m = __ballot_sync(0xFFFFFFFFu, got);
+        if (lane == 0) s_free[warp] = f & ~m;
+      }
+      if (!__syncthreads_or(got)) break;
+    }
+    // the matched pairs, in the order of their first position
+    int cnt = 0;
+    {
+      const bool first = tid < n && !((s_free[tid >> 5] >> (tid & 31)) & 1u) && cand[tid] > tid;
+      const unsigned m = __ballot_sync(0xFFFFFFFFu, first);
+      if (lane == 0 && warp < kSmallMaxN / 32) s_first[warp] = m;
+      __syncthreads();
+      int before = 0;
+#pragma unroll
+      for (int k = 0; k < kSmallMaxN / 32; ++k) {
+        const int x = __popc(s_first[k]);
+        before += (k < warp) ? x : 0;
+        cnt += x;
+      }
+      if (first) pairs[before + __popc(m & ((1u << lane) - 1u))] = make_int2(tid, cand[tid]);
+      __syncthreads();
+    }
+    const int sl = min(cnt, n_2);
+    // the first N_2 pairs in the record order, where there are more
+    if (cnt > n_2) {
+      for (int r = tid; r < cnt; r += THREADS) {
+        const int2 a = pairs[r];
+        const unsigned long long ka = Ks[a.x * lda + a.y];
+        const unsigned ta = tkey(vl[a.x], vl[a.y]);
+        int k = 0;
+        for (int o = 0; o < cnt; ++o) {
+          const int2 b = pairs[o];
+          k += kbetter(Ks[b.x * lda + b.y], tkey(vl[b.x], vl[b.y]), ka, ta) ? 1 : 0;
+        }
+        rk[k] = r;
+      }
+      __syncthreads();
+    }
+    __syncwarp();
+    if (!solo) cluster.barrier_arrive();  // done with this step's keys
+    if (sl <= 0) { stop = 1; info = steps; break; }  // DSTEP_EXEC with SL = 0 (src/D/dstep.F90:421, 575-582)
+
+    // ---- the 2x2 HSVDs of the pivots (src/D/dstep.F90:301-326)
+    for (int r = tid; r < sl; r += THREADS) {
+      const int2 pr = pairs[cnt > n_2 ? rk[r] : r];
+      const int va = vl[pr.x], vb = vl[pr.y];
+      SPiv<T> x;
+      x.p = min(va, vb);
+      x.q = max(va, vb);
+      const T *cp = As + pos[x.p] * lda, *cq = As + pos[x.q] * lda;
+      T B[4] = { cp[x.p], cp[x.q], cq[x.p], cq[x.q] }, V[4], W[4];
+      int inf = 0;
+      Tr<T>::hsvd2(B, Jv[x.p], Jv[x.q], V, W, JK_TH1FIX, inf);
+      x.info = inf;
+      x.pad = 0;
+      x.d0 = Tr<T>::re(B[M11]);
+      x.d1 = Tr<T>::re(B[M22]);
+      if (inf >= 0) {
+        if (inf & 2) {
+          x.ba = Tr<T>::ba(V, quirk);
+          Tr<T>::ut2(V);
+          x.tu = Tr<T>::ab(V);
+        }
+        if (inf & 4) x.tz = Tr<T>::ab(W);
+        if ((inf & 1) && (inf & 6)) atomicAdd(&s_nl, 1);
+      }
+      else
+        atomicMin(&s_err, inf);
+      pv[r] = x;
+    }
+    __syncthreads();
+    const int err = s_err, nl = s_nl;
+
+    // ---- rows p, q of A (BA); columns p, q of the own rows of U (by V^T) and Z (by W)
+    for (int r = warp; r < sl; r += NW) {
+      const SPiv<T> &x = pv[r];
+      const int inf = x.info, p = x.p, q = x.q;
+      if (inf < 0) continue;
+      if (inf & 2) {
+        typename Tr<T>::R ba = x.ba, tu = x.tu;
+        if (ba.c1 && ba.c2) {
+          ba.c1 = ba.c2 = 1;
+#pragma unroll 4
+          for (int j = lane; j < n; j += 32) Tr<T>::apply_ba(ba, As[j * lda + p], As[j * lda + q]);
+        }
+        else
+          for (int j = lane; j < n; j += 32) Tr<T>::apply_ba(ba, As[j * lda + p], As[j * lda + q]);
+        for (int i = lane; i < mr; i += 32) Tr<T>::apply_ab(tu, Us[p * m + i], Us[q * m + i]);
+      }
+      if (inf & 4) {
+        const typename Tr<T>::R tz = x.tz;
+        for (int i = lane; i < mr; i += 32) Tr<T>::apply_ab(tz, Zs[p * m + i], Zs[q * m + i]);
+      }
+    }
+    __syncthreads();
+    if (err == 0) {
+      // ---- columns p, q of A (AB), with the diagonal write-back
+      for (int r = warp; r < sl; r += NW) {
+        const SPiv<T> &x = pv[r];
+        const int inf = x.info, p = x.p, q = x.q;
+        T *ca = As + pos[p] * lda, *cb = As + pos[q] * lda;
+        if (inf & 4) {
+          typename Tr<T>::R tz = x.tz;
+          if (tz.c1 && tz.c2) {
+            tz.c1 = tz.c2 = 1;
+#pragma unroll 4
+            for (int i = lane; i < n; i += 32) Tr<T>::apply_ab(tz, ca[i], cb[i]);
+          }
+          else
+            for (int i = lane; i < n; i += 32) Tr<T>::apply_ab(tz, ca[i], cb[i]);
+        }
+        __syncwarp();
+        if (!(inf & 8) && lane == 0) {
+          T d0 = Tr<T>::zero(), d1 = Tr<T>::zero();
+          *(double *)&d0 = x.d0;
+          *(double *)&d1 = x.d1;
+          ca[p] = d0;
+          ca[q] = Tr<T>::zero();
+          cb[p] = Tr<T>::zero();
+          cb[q] = d1;
+        }
+      }
+    }
+    // ---- the loop test (src/D/dstep.F90:442, 564-583)
+    if (err < 0) { stop = 1; info = err; }
+    else if (min(sl, nl) <= 0) { stop = 1; info = steps; }
+    else {
+      ++steps;
+      if (limit > 0 && steps >= limit) stop = 2;
+    }
+  }
+  if (!solo) cluster.barrier_wait();
+  __syncthreads();
+
+  for (int k = tid; k < n * n; k += THREADS) {
+    const int i = k % n, j = k / n;
+    if (j % C == c) gA[k] = As[pos[j] * lda + i];
+  }
+  for (int k = tid; k < n * mr; k += THREADS) {
+    const int i = k % mr, j = k / mr;
+    gU[(long long)j * n + r0 + i] = Us[j * m + i];
+    gZ[(long long)j * n + r0 + i] = Zs[j * m + i];
+  }
+  if (c == 0 && tid == 0) {
+    st->steps = steps;
+    st->info = info;
+    st->stop = stop;
+  }
+}
+
+// blocks per cluster: a warp's worth of pairs per scheduler and block where 16 blocks allow it
+// (256 real pairs, whose scans are bound by the latency of their fma chains; 64 complex ones, whose
+// magnitudes fill the pipe)
+int small_cluster(int cplx, long long nh)
+{
+  const long long per = cplx ? 64 : 256;
+  int C = 1;
+  while (C < 16 && C * per < nh) C *= 2;
+  return C;
+}
+
+template <typename T> struct SThreads { static constexpr int v = sizeof(T) == 8 ? 512 : 256; };
+
+template <typename T>
+size_t small_bytes(int n, int np) { return SLayout::make<T>(n, small_cluster(sizeof(T) == 16, (long long)np * (n - np))).total; }
+
+template <typename T>
+cudaError_t launch_t(Workspace &w, T *A, T *U, T *Z, int n_2, cudaStream_t s)
+{
+  constexpr int kThreads = SThreads<T>::v;
+  const int C = small_cluster(w.cplx, (long long)w.n_plus * w.n_minus);
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = (unsigned)C;
+  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  cfg.gridDim = dim3((unsigned)C);
+  cfg.blockDim = dim3(kThreads);
+  cfg.dynamicSmemBytes = small_bytes<T>(w.n, w.n_plus);
+  cfg.stream = s;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, k_small<T, kThreads>, w.st, A, U, Z, (const int *)w.J, w.n, w.n_plus, n_2, w.zba_quirk,
+                            kSmallSteps);
+}
+
+}  // namespace
+
+// whether the loop of this matrix fits the persistent kernel
+bool small_fits(int cplx, int n, int n_plus)
+{
+  return n <= kSmallMaxN && (cplx ? small_bytes<double2>(n, n_plus) : small_bytes<double>(n, n_plus)) <= kSmallSmem;
+}
+
+cudaError_t prepare_small(int cplx, int n, int n_plus)
+{
+  const void *f = cplx ? (const void *)k_small<double2, SThreads<double2>::v> : (const void *)k_small<double, SThreads<double>::v>;
+  cudaError_t e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       (int)(cplx ? small_bytes<double2>(n, n_plus) : small_bytes<double>(n, n_plus)));
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(f, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+  return e;
+}
+
+// up to kSmallSteps steps of the loop, or to its end or limit
+cudaError_t launch_small(Workspace &w, void *A, void *U, void *Z, int n_2, cudaStream_t s)
+{
+  return w.cplx ? launch_t(w, (double2 *)A, (double2 *)U, (double2 *)Z, n_2, s)
+                : launch_t(w, (double *)A, (double *)U, (double *)Z, n_2, s);
+}
+
+}  // namespace jk

@@ -219,11 +219,9 @@ static __device__ __noinline__ void zhsvd2_any(double2 A[4], const int J0, const
 // quot, root in jk_math.cuh)
 // ------------------------------------------------------------------------
 
-// both parts zero or at least 2^-300 in magnitude
-__device__ __forceinline__ bool near_parts(double2 z)
-{
-  return near_ratio(fabs(z.x)) && near_ratio(fabs(z.y));
-}
+// zero, or at least 2^-300 in magnitude
+__device__ __forceinline__ bool near_ratio(double x) { return x == 0.0 || fabs(x) >= 4.909093465297727e-91; }
+__device__ __forceinline__ bool near_parts(double2 z) { return near_ratio(z.x) && near_ratio(z.y); }
 
 // hypot2 for two operands below 2^300 of which the larger is zero or at least 2^-1000
 __device__ __forceinline__ double hypot2_near0(double x, double y)
@@ -231,148 +229,153 @@ __device__ __forceinline__ double hypot2_near0(double x, double y)
   return (x == 0.0 && y == 0.0) ? 0.0 : hypot2_near(x, y);
 }
 __device__ __forceinline__ double zabs_near(double2 a) { return hypot2_near0(a.x, a.y); }
+__device__ __forceinline__ double2 zdown600(double2 a) { return zc(down600(a.x), down600(a.y)); }
 
 // a division of both parts by the same number, y = recip(b)
 __device__ __forceinline__ double2 zquot(double2 a, double b, double y) { return zc(quot(a.x, b, y), quot(a.y, b, y)); }
+__device__ __forceinline__ bool zquot_num(double2 a) { return quot_num(a.x) && quot_num(a.y); }
 
-// ZPOLAR (see zpolar) for parts that are zero or near
-__device__ __forceinline__ void zpolar_near(double2 z, double2 &e)
+// e of ZPOLAR (see zpolar) for a scaled entry
+__device__ __forceinline__ void zpolar_scaled(double2 z, double2 &e, bool &ok)
 {
-  const double a = zabs_near(z), y = recip(a);
-  const bool zero = (a == 0.0);
-  const double c = copysign(zero ? 1.0 : fmin(quot(fabs(z.x), a, y), 1.0), z.x);
-  e = zc(c, zero ? z.y : quot(z.y, a, y));
+  const double2 x = zdown600(z);
+  const double a = zabs_near(x), y = recip(a);
+  const int ea = bexp(a), ex = bexp(x.x), ey = bexp(x.y);
+  const bool zero = zeq0(z);
+  ok = ok && (zero || (ea >= 123 && (z.x == 0.0 || (ex >= 123 && ex - ea >= -1000)) && (z.y == 0.0 || (ey >= 123 && ey - ea >= -1000))));
+  const double c = zero ? 1.0 : fmin(quot(fabs(x.x), a, y), 1.0);
+  e = zc(copysign(c, z.x), zero ? z.y : quot(x.y, a, y));
 }
 
-// the exponents of a block's nonzero parts all within 2^-150 of the largest, which lies in
-// 2^(+-100), and no zero column
-__device__ __forceinline__ bool znear_block(const double2 A[4])
+template <int N>
+__device__ __forceinline__ void zquots(double2 *a, double b, double y, bool &ok)
 {
-  int hi = 0, lo = 0x7FF;
+  bool num = true;
 #pragma unroll
-  for (int k = 0; k < 4; ++k) {
-    const int e = (__double2hiint(A[k].x) >> 20) & 0x7FF, f = (__double2hiint(A[k].y) >> 20) & 0x7FF;
-    hi = max(hi, max(e, f));
-    lo = imin(lo, imin((A[k].x == 0.0) ? 0x7FF : e, (A[k].y == 0.0) ? 0x7FF : f));
+  for (int k = 0; k < N; ++k) {
+    num = num && zquot_num(a[k]);
+    a[k] = zquot(a[k], b, y);
   }
-  return hi >= 923 && hi <= 1123 && lo >= hi - 150 && !(zeq0(A[M11]) && zeq0(A[M21])) && !(zeq0(A[M12]) && zeq0(A[M22]));
+  ok = ok && (num || b == 1.0);
 }
 
-// ZHSVD2 for the blocks that znear_block takes: the operations of zhsvd2_any in the same order on
-// the unscaled block, as dhsvd2_near.  Every quantity that is divided is tested (near_parts,
-// near_ratio), so that no product of two of them leaves the normal numbers.  Returns false, with
-// nothing written, when the block does not allow it.
+// C2A and A2C (src/Z/ztransf.F90:245-275) with the rotations of c2a_near, a2c_near
+__device__ __forceinline__ void zc2a_near(double t, double c, double y, double2 A[4], bool &ok)
+{
+  double2 v[4] = { zdfma(t, A[M21], A[M11]), zdfma(-t, A[M11], A[M21]), zdfma(t, A[M22], A[M12]), zdfma(-t, A[M12], A[M22]) };
+  zquots<4>(v, c, y, ok);
+#pragma unroll
+  for (int k = 0; k < 4; ++k) A[k] = v[k];
+}
+__device__ __forceinline__ void za2c_near(double2 A[4], double t21, double t12, double c, double y, bool &ok)
+{
+  double2 v[4] = { zdfma(t21, A[M12], A[M11]), zdfma(t21, A[M22], A[M21]), zdfma(t12, A[M11], A[M12]), zdfma(t12, A[M21], A[M22]) };
+  zquots<4>(v, c, y, ok);
+#pragma unroll
+  for (int k = 0; k < 4; ++k) A[k] = v[k];
+}
+
+__device__ __forceinline__ double2 zsel(bool c, double2 a, double2 b) { return zc(c ? a.x : b.x, c ? a.y : b.y); }
+__device__ __forceinline__ void zcswap(bool c, double2 &a, double2 &b) { cswap(c, a.x, b.x); cswap(c, a.y, b.y); }
+// a v where c, else a
+__device__ __forceinline__ double2 zcmul(bool c, double2 a, double2 v) { return zsel(c, zzmul(a, v), a); }
+
+// ZHSVD2 for a block without a zero column whose largest part lies in 2^(+-300): the operations
+// of zhsvd2_any in the same order, as dhsvd2_near.  Returns false, with nothing written, when the
+// block does not allow it.
 __device__ __forceinline__ bool zhsvd2_near(double2 Ain[4], const int J0, const int J1, double2 Uo[4], double2 Zo[4], double th1, int &info_o)
 {
-  if (!znear_block(Ain) || abs(J0) != 1 || abs(J1) != 1) return false;
+  int hi = 0;
+#pragma unroll
+  for (int k = 0; k < 4; ++k) hi = max(hi, max(bexp(Ain[k].x), bexp(Ain[k].y)));
+  if (hi < 723 || hi > 1323 || (zeq0(Ain[M11]) && zeq0(Ain[M21])) || (zeq0(Ain[M12]) && zeq0(Ain[M22])) || abs(J0) != 1 ||
+      abs(J1) != 1) return false;
+  bool ok = true;
+  const bool tg = (J0 == J1);
+  const int sc = 2044 - hi;  // ZSCALEA's
+  const double fs = pow2(sc - 600);
   const double2 one = zc(1.0, 0.0), zero = zc(0.0, 0.0);
-  double2 A[4] = { Ain[0], Ain[1], Ain[2], Ain[3] }, U[4] = { one, zero, zero, one }, Z[4] = { one, zero, zero, one };
+  double2 A[4], U[4] = { one, zero, zero, one }, Z[4] = { one, zero, zero, one };
+#pragma unroll
+  for (int k = 0; k < 4; ++k) A[k] = zc(up600(__dmul_rn(Ain[k].x, fs)), up600(__dmul_rn(Ain[k].y, fs)));
   // ZHSVD2T, src/Z/ztransf.F90:641-835
   const bool d = zeq0(A[M21]) && zeq0(A[M12]);
-  const double c = hypot2_near(zabs_near(A[M11]), zabs_near(A[M21]));
-  const double t0 = hypot2_near(zabs_near(A[M12]), zabs_near(A[M22]));
+  const double c = up600(hypot2_near(zabs_near(zdown600(A[M11])), zabs_near(zdown600(A[M21]))));
+  const double t0 = up600(hypot2_near(zabs_near(zdown600(A[M12])), zabs_near(zdown600(A[M22]))));
   const bool p = (c < t0);
   const double w = p ? t0 : c;
-  if (p) {
-    zswap(A[M11], A[M12]); zswap(A[M21], A[M22]);
-    if (J0 == J1) { zswap(Z[M11], Z[M12]); zswap(Z[M21], Z[M22]); }
-  }
+  zcswap(p, A[M11], A[M12]); zcswap(p, A[M21], A[M22]);
+  zcswap(p && tg, Z[M11], Z[M12]); zcswap(p && tg, Z[M21], Z[M22]);
   double2 r, s;
-  zpolar_near(A[M11], r);
-  zpolar_near(A[M21], s);
-  if (zne1(r)) {
-    const double2 v = conj(r);
-    U[M11] = zzmul(U[M11], v); U[M12] = zzmul(U[M12], v);
-    A[M11] = zzmul(A[M11], v); A[M12] = zzmul(A[M12], v);
+  zpolar_scaled(A[M11], r, ok);
+  zpolar_scaled(A[M21], s, ok);
+  {
+    const bool nr = zne1(r), ns = zne1(s);
+    const double2 vr = conj(r), vs = conj(s);
+    U[M11] = zcmul(nr, U[M11], vr); U[M12] = zcmul(nr, U[M12], vr);
+    A[M11] = zcmul(nr, A[M11], vr); A[M12] = zcmul(nr, A[M12], vr);
+    U[M21] = zcmul(ns, U[M21], vs); U[M22] = zcmul(ns, U[M22], vs);
+    A[M21] = zcmul(ns, A[M21], vs); A[M22] = zcmul(ns, A[M22], vs);
   }
-  if (zne1(s)) {
-    const double2 v = conj(s);
-    U[M21] = zzmul(U[M21], v); U[M22] = zzmul(U[M22], v);
-    A[M21] = zzmul(A[M21], v); A[M22] = zzmul(A[M22], v);
-  }
-  if (A[M11].x < A[M21].x) {
-    zswap(U[M11], U[M21]); zswap(U[M12], U[M22]);
-    zswap(A[M11], A[M21]); zswap(A[M12], A[M22]);
-  }
-  if (!d) {
-    if (!(A[M11].x > 0.0)) return false;
-    const double t = quot(A[M21].x, A[M11].x, recip(A[M11].x));
+  const bool sw = (A[M11].x < A[M21].x);
+  zcswap(sw, U[M11], U[M21]); zcswap(sw, U[M12], U[M22]);
+  zcswap(sw, A[M11], A[M21]); zcswap(sw, A[M12], A[M22]);
+  {
+    ok = ok && (d || A[M11].x > 0.0);
+    const double t = quot_scaled(A[M21].x, A[M11].x, recip(down600(A[M11].x)), ok);
     const double q = root(fma(t, t, 1.0)), y = recip(q);
-    const double2 u11 = zdfma(t, U[M21], U[M11]), u21 = zdfma(-t, U[M11], U[M21]);
-    const double2 u12 = zdfma(t, U[M22], U[M12]), u22 = zdfma(-t, U[M12], U[M22]);
-    const double2 a1 = zdfma(t, A[M22], A[M12]), a2 = zdfma(-t, A[M12], A[M22]);
-    U[M11] = zquot(u11, q, y); U[M21] = zquot(u21, q, y); U[M12] = zquot(u12, q, y); U[M22] = zquot(u22, q, y);
-    A[M12] = zquot(a1, q, y); A[M22] = zquot(a2, q, y);
+    double2 V[4] = { U[0], U[1], U[2], U[3] };
+    zc2a_near(t, q, y, V, ok);
+    double2 v[2] = { zdfma(t, A[M22], A[M12]), zdfma(-t, A[M12], A[M22]) };  // C1A
+    zquots<2>(v, q, y, ok);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) U[k] = zsel(d, U[k], V[k]);
+    A[M12] = zsel(d, A[M12], v[0]);
+    A[M22] = zsel(d, A[M22], v[1]);
   }
   A[M11] = zc(w, 0.0);
   A[M21] = zero;
-  if (!near_parts(A[M12]) || !near_parts(A[M22])) return false;
-  if ((J0 != J1) && p) {
-    zswap(A[M11], A[M12]); zswap(A[M21], A[M22]);
-    zswap(U[M11], U[M21]); zswap(U[M12], U[M22]);
-    zswap(A[M11], A[M21]); zswap(A[M12], A[M22]);
-    zpolar_near(A[M21], s);
-    if (zne1(s)) {
-      const double2 v = conj(s);
-      Z[M11] = zzmul(Z[M11], v); Z[M21] = zzmul(Z[M21], v);
-      A[M11] = zzmul(A[M11], v); A[M21] = zzmul(A[M21], v);
-    }
-    if (!near_parts(A[M11])) return false;
-    zpolar_near(A[M11], r);
-    if (zne1(r)) {
-      const double2 v = conj(r);
-      U[M11] = zzmul(U[M11], v); U[M12] = zzmul(U[M12], v);
-      A[M11] = zzmul(A[M11], v);
-    }
-  }
-  else {
-    zpolar_near(A[M12], r);
-    if (zne1(r)) {
-      const double2 v = conj(r);
-      Z[M12] = zzmul(Z[M12], v); Z[M22] = zzmul(Z[M22], v);
-      A[M12] = zzmul(A[M12], v); A[M22] = zzmul(A[M22], v);
-    }
-    if (!near_parts(A[M22])) return false;
-    zpolar_near(A[M22], s);
-    if (zne1(s)) {
-      const double2 v = conj(s);
-      U[M21] = zzmul(U[M21], v); U[M22] = zzmul(U[M22], v);
-      A[M22] = zzmul(A[M22], v);
-    }
+  // unequal signs and swapped columns: rows and columns swapped back, a lower triangle
+  const bool lo = !tg && p;
+  zcswap(lo, A[M11], A[M12]); zcswap(lo, A[M21], A[M22]);
+  zcswap(lo, U[M11], U[M21]); zcswap(lo, U[M12], U[M22]);
+  zcswap(lo, A[M11], A[M21]); zcswap(lo, A[M12], A[M22]);
+  {
+    zpolar_scaled(zsel(lo, A[M21], A[M12]), s, ok);
+    const bool ns = zne1(s);
+    const double2 vs = conj(s);
+    Z[M11] = zcmul(ns && lo, Z[M11], vs); Z[M21] = zcmul(ns && lo, Z[M21], vs);
+    Z[M12] = zcmul(ns && !lo, Z[M12], vs); Z[M22] = zcmul(ns && !lo, Z[M22], vs);
+    A[M11] = zcmul(ns && lo, A[M11], vs); A[M21] = zcmul(ns && lo, A[M21], vs);
+    A[M12] = zcmul(ns && !lo, A[M12], vs); A[M22] = zcmul(ns && !lo, A[M22], vs);
+    zpolar_scaled(zsel(lo, A[M11], A[M22]), r, ok);
+    const bool nr = zne1(r);
+    const double2 vr = conj(r);
+    U[M11] = zcmul(nr && lo, U[M11], vr); U[M12] = zcmul(nr && lo, U[M12], vr); A[M11] = zcmul(nr && lo, A[M11], vr);
+    U[M21] = zcmul(nr && !lo, U[M21], vr); U[M22] = zcmul(nr && !lo, U[M22], vr); A[M22] = zcmul(nr && !lo, A[M22], vr);
   }
   int info = d ? 0 : 1;
-  double w11 = A[M11].x, w22 = A[M22].x;
-  if (info) {
-    double W[4] = { A[M11].x, A[M21].x, A[M12].x, A[M22].x };
+  double w11, w22;
+  if (d) {
+    w11 = scale(A[M11].x, -sc);
+    w22 = scale(A[M22].x, -sc);
+  }
+  else {
+    const double W[4] = { A[M11].x, A[M21].x, A[M12].x, A[M22].x };
     NearK k;
-    if (!khsvd2_near(W, J0, J1, th1, info, k)) return false;
-    if (!near_ratio(fabs(k.tu)) || !near_ratio(fabs(k.tz))) return false;
+    khsvd2_near(W, tg, sc, th1, info, k, ok);
+    zc2a_near(k.tu, k.cu, k.yu, U, ok);
+    za2c_near(Z, k.tz, k.c12, k.cz, k.yz, ok);
+    w11 = k.g0;
+    w22 = k.g1;
+    if (info & 8) {
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
-      if (!near_parts(U[i]) || !near_parts(Z[i])) return false;
-    const double2 u11 = zdfma(k.tu, U[M21], U[M11]), u21 = zdfma(-k.tu, U[M11], U[M21]);
-    const double2 u12 = zdfma(k.tu, U[M22], U[M12]), u22 = zdfma(-k.tu, U[M12], U[M22]);
-    U[M11] = zquot(u11, k.cu, k.yu); U[M21] = zquot(u21, k.cu, k.yu);
-    U[M12] = zquot(u12, k.cu, k.yu); U[M22] = zquot(u22, k.cu, k.yu);
-    const double2 z11 = zdfma(k.tz, Z[M12], Z[M11]), z12 = zdfma(k.c12, Z[M11], Z[M12]);
-    const double2 z21 = zdfma(k.tz, Z[M22], Z[M21]), z22 = zdfma(k.c12, Z[M21], Z[M22]);
-    Z[M11] = zquot(z11, k.cz, k.yz); Z[M12] = zquot(z12, k.cz, k.yz);
-    Z[M21] = zquot(z21, k.cz, k.yz); Z[M22] = zquot(z22, k.cz, k.yz);
-    if (!(info & 8)) { w11 = k.g0; w22 = k.g1; }
-    else {
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-        if (!near_parts(A[i])) return false;
-      const double2 a11 = zdfma(k.tu, A[M21], A[M11]), a21 = zdfma(-k.tu, A[M11], A[M21]);
-      const double2 a12 = zdfma(k.tu, A[M22], A[M12]), a22 = zdfma(-k.tu, A[M12], A[M22]);
-      A[M11] = zquot(a11, k.cu, k.yu); A[M21] = zquot(a21, k.cu, k.yu);
-      A[M12] = zquot(a12, k.cu, k.yu); A[M22] = zquot(a22, k.cu, k.yu);
-      const double2 b11 = zdfma(k.tz, A[M12], A[M11]), b12 = zdfma(k.c12, A[M11], A[M12]);
-      const double2 b21 = zdfma(k.tz, A[M22], A[M21]), b22 = zdfma(k.c12, A[M21], A[M22]);
-      A[M11] = zquot(b11, k.cz, k.yz); A[M12] = zquot(b12, k.cz, k.yz);
-      A[M21] = zquot(b21, k.cz, k.yz); A[M22] = zquot(b22, k.cz, k.yz);
+      for (int i = 0; i < 4; ++i) A[i] = zc(scale(A[i].x, -sc), scale(A[i].y, -sc));
+      zc2a_near(k.tu, k.cu, k.yu, A, ok);
+      za2c_near(A, k.tz, k.c12, k.cz, k.yz, ok);
     }
   }
+  if (!ok) return false;
   if (!(info & 8)) { A[M11] = zc(w11, 0.0); A[M22] = zc(w22, 0.0); }
   zhsvd2s(A, J0, J1, U, Z, info);
 #pragma unroll
