@@ -1274,7 +1274,7 @@ k_select(State *st, const double *__restrict__ Wm, const int *__restrict__ J, in
   unsigned short *fill = (unsigned short *)(smem_raw + L.fill);  // [nl]: list entries fetched
   int2 *pairs = (int2 *)(smem_raw + L.pairs);                  // [n/2 + 1]  (block 0)
   unsigned *taken = (unsigned *)(smem_raw + L.taken);          // [(n + 31) / 32]: a bit per vertex
-  __shared__ int s_cnt, s_off, s_np, s_nunp, s_got[2];
+  __shared__ int s_cnt, s_nunp, s_got[2], s_all[16];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, ld = list_ld(n);
   const bool solo = (C == 1);
   auto sync = [&]() { if (solo) __syncthreads(); else cluster.sync(); };
@@ -1432,22 +1432,27 @@ k_select(State *st, const double *__restrict__ Wm, const int *__restrict__ J, in
 
   cp_async_wait<0>();
   sync();  // every block's count stands
-  // the pairs are complete: their number and, per block, the place of its own among them
-  if (tid == 0) {
-    int np = 0;
-    for (int b = 0; b < C; ++b) {
-      if (b == c) s_off = np;
-      np += (b == c) ? s_cnt : *cluster.map_shared_rank(&s_cnt, b);
-    }
-    s_np = np;
-  }
+  // the pairs are complete.  The blocks' lists are interleaved: a block's vertices are congruent
+  // modulo C, and k_rotate's lanes take consecutive pivots, whose rows would share a bank.
+  if (tid < C) s_all[tid] = (tid == c) ? s_cnt : *cluster.map_shared_rank(&s_cnt, tid);
   __syncthreads();
-  const int np = s_np, off = s_off, cnt = s_cnt;
+  const int cnt = s_all[c];
+  int np = 0;
+  for (int b = 0; b < C; ++b) np += s_all[b];
+  auto place = [&](int i) {
+    int r = 0;
+    for (int b = 0; b < C; ++b) r += min(s_all[b], i + (b < c ? 1 : 0));
+    return r;
+  };
   const int sl = (np < n_2) ? np : n_2;
   const bool ranked = (np > n_2) || st->trace_on || !A;
   if (ranked) {
     // the pairs in rank order (AW_SRT), by block 0; piv is their first place of call
-    for (int i = tid; i < cnt; i += kSelThreads) { piv[off + i].p = pairs[i].x; piv[off + i].q = pairs[i].y; }
+    for (int i = tid; i < cnt; i += kSelThreads) {
+      const int r = place(i);
+      piv[r].p = pairs[i].x;
+      piv[r].q = pairs[i].y;
+    }
     __threadfence();
     sync();
     if (c != 0) return;
@@ -1482,7 +1487,7 @@ k_select(State *st, const double *__restrict__ Wm, const int *__restrict__ J, in
   }
   else {
     for (int i = tid; i < cnt; i += kSelThreads) {
-      const int r = off + i;
+      const int r = place(i);
       piv[r].p = pairs[i].x;
       piv[r].q = pairs[i].y;
       pivot_hsvd<T>(st, A, J, n, pairs[i].x, pairs[i].y, piv[r], rr[r], quirk);
