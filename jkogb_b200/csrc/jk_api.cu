@@ -6,6 +6,7 @@
 #include <cstdlib>
 #include <cstring>
 #include <algorithm>
+#include <mutex>
 #include <vector>
 
 #include "../../include/jkogb.h"
@@ -34,6 +35,81 @@ struct Guard {
     return e;
   }
 };
+
+// What every solve needs however small it is: the loop state on the device with its pinned host
+// mirror, and room for the index arrays.  Making and freeing the pinned page and the device pages took
+// 3 ms a call, twice the whole solve at N = 16, so finished solves hand them on to later ones: at most
+// kKept blocks per process stay (0.8 MB), the rest is freed.  A block is handed on only when nothing
+// that uses it is pending.
+struct StateBlock {
+  int dev = -1;
+  unsigned char *d = nullptr;  // kBytes on device `dev`
+  State *host = nullptr;
+  size_t used = 0;
+  static constexpr size_t kBytes = 100 * 1024;
+  template <typename X> bool take(X **p, size_t bytes)
+  {
+    if (used + bytes > kBytes) return false;
+    *p = (X *)(d + used);
+    used += (bytes + 255) & ~(size_t)255;
+    return true;
+  }
+};
+
+class StateBlocks {
+  static constexpr size_t kKept = 8;
+  std::mutex mu;
+  std::vector<StateBlock> kept;
+  static void release(StateBlock &b)
+  {
+    if (b.d) cudaFree(b.d);
+    if (b.host) cudaFreeHost(b.host);
+    b = StateBlock();
+  }
+
+public:
+  cudaError_t get(StateBlock &b)
+  {
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    {
+      std::lock_guard<std::mutex> lk(mu);
+      for (size_t i = 0; i < kept.size(); ++i)
+        if (kept[i].dev == dev) {
+          b = kept[i];
+          b.used = 0;
+          kept.erase(kept.begin() + i);
+          return cudaSuccess;
+        }
+    }
+    b = StateBlock();
+    b.dev = dev;
+    e = cudaMalloc((void **)&b.d, StateBlock::kBytes);
+    if (e == cudaSuccess) e = cudaMallocHost((void **)&b.host, sizeof(State));
+    if (e != cudaSuccess) release(b);
+    return e;
+  }
+  void put(StateBlock &b, bool keep)
+  {
+    if (!b.d) return;
+    if (keep) {
+      std::lock_guard<std::mutex> lk(mu);
+      if (kept.size() < kKept) {
+        kept.push_back(b);
+        b = StateBlock();
+        return;
+      }
+    }
+    release(b);
+  }
+};
+
+StateBlocks &state_blocks()
+{
+  static StateBlocks *p = new StateBlocks;  // (never destroyed: the driver may be gone before it)
+  return *p;
+}
 
 inline int cuda_fail(cudaError_t e)
 {
@@ -82,7 +158,7 @@ int jstep_len(int n, int n_2)
 
 // device workspace of one solve
 int make_workspace(Guard &g, Workspace &w, int n, int cplx, const int *J, int trace_on, int cap_steps, long long cap_piv,
-                   int small = 0)
+                   int small = 0, StateBlock *blk = nullptr)
 {
   memset(&w, 0, sizeof(w));
   w.n = n;
@@ -98,10 +174,17 @@ int make_workspace(Guard &g, Workspace &w, int n, int cplx, const int *J, int tr
   const size_t rrsz = cplx ? sizeof(RowRot<double2>) : sizeof(RowRot<double>);
   const int half = n / 2 + 1;
   w.small = small && small_fits(cplx, n, w.n_plus);
-  CK(g.alloc(&w.J, n * sizeof(int)));
-  CK(g.alloc(&w.st, sizeof(State)));
-  CK(cudaMallocHost((void **)&g.pinned, sizeof(State)));
-  w.st_host = (State *)g.pinned;
+  auto take = [&](auto **p, size_t bytes) { return (blk && blk->take(p, bytes)) ? cudaSuccess : g.alloc(p, bytes); };
+  if (blk) {
+    CK(state_blocks().get(*blk));
+    w.st_host = blk->host;
+  }
+  else {
+    CK(cudaMallocHost((void **)&g.pinned, sizeof(State)));
+    w.st_host = (State *)g.pinned;
+  }
+  CK(take(&w.st, sizeof(State)));
+  CK(take(&w.J, n * sizeof(int)));
   CK(cudaMemcpy(w.J, j32.data(), n * sizeof(int), cudaMemcpyHostToDevice));
   State s0;
   memset(&s0, 0, sizeof(s0));
@@ -113,15 +196,15 @@ int make_workspace(Guard &g, Workspace &w, int n, int cplx, const int *J, int tr
     CK(prepare_small(cplx, n, w.n_plus));
     return 0;
   }
-  CK(g.alloc(&w.plus, (plus.size() + 1) * sizeof(int)));
-  CK(g.alloc(&w.minus, (minus.size() + 1) * sizeof(int)));
+  CK(take(&w.plus, (plus.size() + 1) * sizeof(int)));
+  CK(take(&w.minus, (minus.size() + 1) * sizeof(int)));
   CK(g.alloc(&w.Wm, (size_t)n * n * sizeof(double)));
   if (cplx) CK(g.alloc(&w.mag, (size_t)n * n * sizeof(double)));
   CK(g.alloc(&w.piv, half * pivsz));
   CK(g.alloc(&w.rowrot, half * rrsz));
   CK(g.alloc(&w.list, (size_t)n * ((n + 7) & ~7) * sizeof(unsigned short)));
-  CK(g.alloc(&w.len, n * sizeof(int)));
-  CK(g.alloc(&w.unp, (n + 1) * sizeof(int)));
+  CK(take(&w.len, n * sizeof(int)));
+  CK(take(&w.unp, (n + 1) * sizeof(int)));
   if (trace_on) {
     const int cs = cap_steps > 0 ? cap_steps : 1;
     const long long cp = cap_piv > 0 ? cap_piv : 1;
@@ -155,6 +238,7 @@ struct jk_scorer {
 // whole steps and the loop's position.
 struct jk_solver {
   Guard g;
+  StateBlock blk;
   Workspace w;
   jk_opts o;
   int n = 0, cplx = 0, n_2 = 0;
@@ -171,6 +255,9 @@ struct jk_solver {
   ~jk_solver()
   {
     if (exec) cudaGraphExecDestroy(exec);
+    // (a started loop has work in flight until it has ended or stopped: advance and finish synchronise)
+    const bool idle = (phase == 0 || phase == 2 || phase == 3 || cudaDeviceSynchronize() == cudaSuccess);
+    state_blocks().put(blk, idle && cudaPeekAtLastError() == cudaSuccess);
   }
 };
 
@@ -191,7 +278,7 @@ int solver_make(jk_solver *v, int cplx, int n, const int *J, int n_2, int id_ncp
   // a small matrix's loop runs in one persistent launch, unless each step is to be recorded, scored
   // or selected by AW_NCP3
   int rc = make_workspace(g, w, n, cplx, J, trace != nullptr, trace ? trace->max_steps : 0, trace ? trace->max_piv : 0,
-                          !trace && !sc && id_ncp != 3);
+                          !trace && !sc && id_ncp != 3, &v->blk);
   if (rc) return rc;
   w.zba_quirk = (v->o.zba_quirk == 0) ? 1 : 0;
   w.id_ncp = id_ncp;
@@ -259,14 +346,23 @@ void solver_graph(jk_solver *v)
   if (v->exec && !memcmp(key, v->key, sizeof(key))) return;
   if (v->exec) { cudaGraphExecDestroy(v->exec); v->exec = nullptr; }
   cudaGraph_t graph = nullptr;
-  cudaError_t e = cudaStreamBeginCapture(v->s, cudaStreamCaptureModeThreadLocal);
+  // the default stream cannot be captured, but a graph captured elsewhere is launched into it (plain
+  // launches, 6 to 11 a step, left the host the bottleneck up to N = 1024)
+  cudaStream_t cs = v->s, own = nullptr;
+  cudaError_t e = cudaSuccess;
+  if (cs == nullptr || cs == cudaStreamLegacy) {
+    e = cudaStreamCreateWithFlags(&own, cudaStreamNonBlocking);
+    cs = own;
+  }
+  if (e == cudaSuccess) e = cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal);
   if (e == cudaSuccess) {
-    for (int k = 0; k < v->chunk && e == cudaSuccess; ++k) e = launch_step(v->w, v->dA, v->dU, v->dZ, v->n_2, v->s);
-    const cudaError_t e2 = cudaStreamEndCapture(v->s, &graph);
+    for (int k = 0; k < v->chunk && e == cudaSuccess; ++k) e = launch_step(v->w, v->dA, v->dU, v->dZ, v->n_2, cs);
+    const cudaError_t e2 = cudaStreamEndCapture(cs, &graph);
     if (e == cudaSuccess) e = e2;
   }
   if (e == cudaSuccess) e = cudaGraphInstantiate(&v->exec, graph, 0);
   if (graph) cudaGraphDestroy(graph);
+  if (own) cudaStreamDestroy(own);
   if (e != cudaSuccess) {
     cudaGetLastError();
     if (v->exec) { cudaGraphExecDestroy(v->exec); v->exec = nullptr; }
