@@ -263,6 +263,17 @@ struct jk_solver {
 
 namespace {
 
+// Where the filter pays: it adds the Gram products, a bound per pair and five launches to a step (60 us
+// at the smallest orders) and takes the column scans away.  Measured over the first steps, filter
+// against scan: real N = 512 graded 176 to 173 us a step, 701 258 to 247, 800 (where the scan takes its
+// large tiles) 199 to 302, 2048 graded 0.80 to 2.11 ms, 4096 3.9 to 14.3 ms; complex N = 100 103 to 118 us,
+// 200 128 to 178, 1024 0.37 to 3.18 ms.
+bool filter_pays(int cplx, int n, int np, int nm)
+{
+  const long long nh = (long long)np * nm;
+  return cplx ? nh * n >= 250000 : nh >= kHypTileMin;
+}
+
 int solver_make(jk_solver *v, int cplx, int n, const int *J, int n_2, int id_ncp, const jk_opts *opts,
                 const jk_trace *trace, const jk_scorer *sc)
 {
@@ -292,6 +303,27 @@ int solver_make(jk_solver *v, int cplx, int n, const int *J, int n_2, int id_ncp
     CK(g.alloc(&w.n3it, sizeof(int)));
     CK(cudaMemset(w.n3it, 0, sizeof(int)));
   }
+  // the exact ranking by the filter, where the column scans outweigh what it adds and no step's
+  // weights or ranked pivots are asked for
+  if (!w.small && !trace && !sc && id_ncp != 3 && v->n_2 == n / 2 && filter_pays(cplx, n, w.n_plus, w.n_minus)) {
+    const size_t npm = (size_t)w.n_plus * w.n_minus;
+    FilterDev &f = w.fd;
+    f.cap = (int)(npm / 64);
+    CK(g.alloc(&f.code, npm * sizeof(short)));
+    CK(g.alloc(&f.claim, (npm / 32 + 1) * sizeof(unsigned)));
+    CK(g.alloc(&f.list, ((size_t)f.cap + 1) * sizeof(int)));
+    CK(g.alloc(&f.dirty, n * sizeof(int)));
+    CK(g.alloc(&f.cls, n * sizeof(int)));
+    CK(g.alloc(&w.gram, ((size_t)(cplx ? 2 : 1) * npm + 1) * sizeof(double)));
+    CK(g.alloc(&w.cn, (size_t)n * sizeof(double)));
+    std::vector<int> cls(n);
+    int np = 0, nm = 0;
+    for (int i = 0; i < n; ++i) cls[i] = (J[i] == 1) ? np++ : ~nm++;
+    CK(cudaMemcpy(f.cls, cls.data(), n * sizeof(int), cudaMemcpyHostToDevice));
+    CK(cudaMemset(f.dirty, 0, n * sizeof(int)));
+    CK(prepare_gram());
+    w.filter = 1;
+  }
   if (sc) {
     // a learned solve: the scorer's device parameters, the off-norm buffers
     w.learned = 1;
@@ -313,7 +345,8 @@ int solver_make(jk_solver *v, int cplx, int n, const int *J, int n_2, int id_ncp
 long long step_launches(const Workspace &w)
 {
   const bool hyp = (w.n_plus > 0 && w.n_minus > 0);
-  const int learned = !w.learned ? 0 : (hyp ? 4 : 1);  // norms, Gram, weights; the off-norm
+  // norms, Gram, weights; the off-norm (learned) or the exact weights and a second ranking (filtered)
+  const int learned = w.learned ? (hyp ? 4 : 1) : w.filter ? 5 : 0;
   return kStepLaunches - (hyp ? 0 : 1) + ((w.cplx && hyp) ? 1 : 0) + learned;
 }
 
@@ -326,6 +359,8 @@ int solver_start(jk_solver *v, void *dU, void *dA, void *dZ, const double *dsigm
   v->dU = dU;
   v->dZ = dZ;
   v->s = s;
+  // (the Gram products copy 16 bytes at a time; an 8-byte aligned real matrix takes the column scans)
+  v->w.filter = v->w.fd.code && !((uintptr_t)dA & 15);
   v->phase = 1;
   v->info = 0;
   v->steps = steps0;

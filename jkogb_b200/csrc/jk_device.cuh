@@ -145,4 +145,39 @@ __device__ __forceinline__ double gram_weight(double d, const double Z2[4], doub
   return d + (nx * c1 + ny * c2 - 2.0 * c3 * g);
 }
 
+// zhyp_setup's 2x2 part (ZMAGF2H, src/Z/zstep.F90:43-74) with the right transformation itself
+__device__ __forceinline__ bool zhyp_setup_z(double2 app, double2 aqp, double2 apq, double2 aqq, int jp, double &w, double &d,
+                                             double2 Z2[4])
+{
+  w = nan_w();
+  if (!may_transform(app, aqp, apq, aqq)) return false;
+  double2 A2[4] = { app, aqp, apq, aqq }, U2[4];
+  int info = 0;
+  zhsvd2(A2, jp, -jp, U2, Z2, JK_TH1FIX, info);
+  if (info < 0) return false;
+  if (!(info & 1)) { w = 0.0; return false; }
+  if (!(info & 4)) { w = dasum4(aqp.x, aqp.y, apq.x, apq.y); return false; }
+  // the four off-diagonal terms that start ABODNZF2
+  const double2 a1 = (info & 8) ? A2[M21] : make_double2(0.0, 0.0);
+  const double2 a2 = (info & 8) ? A2[M12] : make_double2(0.0, 0.0);
+  d = 0.0;
+  d = fma(__dsub_rn(aqp.x, a1.x), __dadd_rn(aqp.x, a1.x), d);
+  d = fma(__dsub_rn(aqp.y, a1.y), __dadd_rn(aqp.y, a1.y), d);
+  d = fma(__dsub_rn(apq.x, a2.x), __dadd_rn(apq.x, a2.x), d);
+  d = fma(__dsub_rn(apq.y, a2.y), __dadd_rn(apq.y, a2.y), d);
+  return true;
+}
+
+// the Gram form of a complex pair's scanned weight: gr + i gi = x^H y of its columns p, q
+__device__ __forceinline__ double zgram_weight(double d, const double2 Z2[4], double nx, double ny, double gr, double gi)
+{
+  const double2 z11 = Z2[M11], z21 = Z2[M21], z12 = Z2[M12], z22 = Z2[M22];
+  const double c1 = (1.0 - z11.x) * (1.0 + z11.x) - z11.y * z11.y - (z12.x * z12.x + z12.y * z12.y);
+  const double c2 = (1.0 - z22.x) * (1.0 + z22.x) - z22.y * z22.y - (z21.x * z21.x + z21.y * z21.y);
+  // conj(z11) z21 + conj(z12) z22
+  const double c3r = (z11.x * z21.x + z11.y * z21.y) + (z12.x * z22.x + z12.y * z22.y);
+  const double c3i = (z11.x * z21.y - z11.y * z21.x) + (z12.x * z22.y - z12.y * z22.x);
+  return d + (nx * c1 + ny * c2 - 2.0 * (c3r * gr - c3i * gi));
+}
+
 }  // namespace jk

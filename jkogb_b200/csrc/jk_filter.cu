@@ -1,0 +1,230 @@
+// jk_filter.cu -- the exact ranking of the hyperbolic pairs without the O(N) column scan of every pair.
+//
+// DMAGF2H's weight of a scanned pair is ABODNDF2's sequential sum over the rows of two columns
+// (src/D/dtransf.F90:246-348; ZMAGF2H, ABODNZF2 src/Z/ztransf.F90:452-637): 14 flop a row on the FP64
+// pipe (a step at N = 2048: 1.67 of 2.1 ms), a chain that no matrix product gives bit for bit.  But a
+// step uses the weights only to rank every vertex's partners.  So they are filtered, as
+// geometric predicates are: every scanned pair gets its weight from the Gram products of the columns
+// (k_gram, FP64 tensor pipe; the formula of the scored ranking) with a bound on how far the sequential
+// sum can lie from it, every vertex's partners are ranked by it, and only the pairs whose interval
+// meets a neighbour's in some list are summed exactly and their lists ranked again.  The lists, and
+// with them the pivots, are those of the exact weights.  Where too many pairs are ambiguous (weights
+// at the level of their own rounding) the full scan runs, and for the next kDirectSteps steps at once.
+//
+// The bound.  Let u = 2^-53, x, y the columns without rows p, q, (z11, z21), (z12, z22) the right
+// transformation's columns, S = |x|^2 + |y|^2 <= cn[p] + cn[q], zm = max(z11^2 + z12^2, z21^2 + z22^2),
+// and k = |1 - z11^2| + |1 - z22^2| + z12^2 + z21^2 + 2 |z11 z21| + 2 |z12 z22|.
+//  E1, the terms.  A rotated entry is off by at most 3.01 u P, P = |z11 x_i| + |z21 y_i| (ratio, fma,
+//     product), so a term (x - x')(x + x') by 6.1 u P^2 + 2.1 u (x_i^2 + P^2), and P^2 <= 2 (z11^2 x_i^2 +
+//     z21^2 y_i^2): both sums together by (17 zm + 2.2) u S.  Where |z11| = |z22| = 1 (a rotation below
+//     2^-26) the only rounding is that of x + z21 y, which moves it by no more than |z21 y|: then also by
+//     1.2 (|z12| + |z21|) S.
+//  E2, the additions.  The terms' magnitudes sum to at most V = k S + E1.  Each of the 2 (n - 2) additions
+//     rounds a partial sum of at most |d| + V (d the leading terms) and moves it by no more than the term
+//     added: min(2 n u (|d| + V), V).
+//  E3, the Gram form: products of n terms (n + 8) u S/2 each way, doubled for the tensor pipe's order,
+//     norms (n/32 + 8) u, coefficients and sums a few u: (1.04 n + 48) u k S, and the last addition
+//     min(2 u |d|, 1.01 k S) more.
+// Together, with a tenth added for what is of second order: 1.1 (E1 + min(2 n u (|d| + V), V) +
+// (1.04 n + 64) u k S + min(4 u |d|, 1.1 V)).  Where V is below 2^-56 |d|, or below every number, no
+// addition changes d: the weight is d, exactly.  Complex: a rotated entry's magnitude is off by at most 32
+// u P (zzfma, zzmul, the ratio, the project's hypot), the Gram products have 2 n terms, 1 - |z11|^2 is
+// formed from parts: 1.1 u ((150 zm + 60) S + k S (7 n + 64) + (2 n + 16) |d|).  Bounds are kept as
+// powers of two (two bytes a pair), at least 2^-1000 (complex) or 2^-1056 (real: 4 n roundings
+// below the normal numbers), which covers underflow; a pair whose numbers leave [0, 1e300] is summed
+// exactly.  On the graded inputs a bound is about 1e-12 of its weight, and no pair of a step's million is
+// ambiguous in the first fifth of a solve.
+#include "jk_internal.h"
+#include "jk_device.cuh"
+#include "jk_scan.cuh"
+
+namespace jk {
+
+namespace {
+
+// a bound e as the exponent of a power of two that is not below it
+__device__ __forceinline__ short bound_code(double e, int least) { return (short)max(exponent(e), least); }
+
+// the weight of a hyperbolic pair from the Gram products: exact (code kBoundExact), or with a
+// bound; kBoundNone when it has to be summed
+__device__ __forceinline__ double filter_pair(const double *__restrict__ A, int n, int a, int b, long long gidx, long long,
+                                              const double *__restrict__ G, const double *__restrict__ cn, short &code)
+{
+  const bool ap = a < b;
+  const int p = ap ? a : b, q = ap ? b : a;
+  const double app = A[(long long)p * n + p], aqp = A[(long long)p * n + q], apq = A[(long long)q * n + p], aqq = A[(long long)q * n + q];
+  double w, d, Z[4];
+  code = kBoundExact;
+  if (!hyp_setup_z(app, aqp, apq, aqq, ap ? 1 : -1, w, d, Z)) return w;
+  const double z11 = Z[M11], z21 = Z[M21], z12 = Z[M12], z22 = Z[M22];
+  const double cp = cn[p], cq = cn[q];
+  w = gram_weight(d, Z, cp - aqp * aqp, cq - apq * apq, G[gidx]);
+  const double S = cp + cq;
+  const double zm = fmax(z11 * z11 + z12 * z12, z21 * z21 + z22 * z22);
+  const double k = fabs((1.0 - z11) * (1.0 + z11)) + fabs((1.0 - z22) * (1.0 + z22)) + z12 * z12 + z21 * z21 +
+                   2.0 * fabs(z11 * z21) + 2.0 * fabs(z12 * z22);
+  const double u = 0x1p-53, kS = k * S, ad = fabs(d);
+  double e1 = (17.0 * zm + 2.2) * u * S;
+  if (fabs(z11) == 1.0 && fabs(z22) == 1.0) e1 = fmin(e1, 1.2 * (fabs(z12) + fabs(z21)) * S);
+  const double V = 1.01 * (kS + e1);
+  // (times 2^200, where a product below 2^-1080 is still a number)
+  const double V200 = 1.2 * ((k * 0x1p200) * S + e1 * 0x1p200);
+  if (ad <= 1e300 && ((ad >= 0x1p-960 && V <= 0x1p-56 * ad) || (V200 < 0x1p-880 && S <= 1e300))) return d;
+  const double e = 1.1 * (e1 + fmin(2.0 * n * u * (ad + V), V) + (1.04 * n + 64.0) * u * kS + fmin(4.0 * u * ad, 1.1 * V));
+  code = (fabs(w) <= 1e300 && S <= 1e300 && e <= 1e300) ? bound_code(e, -1056) : kBoundNone;
+  return w;
+}
+
+__device__ __forceinline__ double filter_pair(const double2 *__restrict__ A, int n, int a, int b, long long gidx, long long npm,
+                                              const double *__restrict__ G, const double *__restrict__ cn, short &code)
+{
+  const bool ap = a < b;
+  const int p = ap ? a : b, q = ap ? b : a;
+  const double2 app = A[(long long)p * n + p], aqp = A[(long long)p * n + q], apq = A[(long long)q * n + p], aqq = A[(long long)q * n + q];
+  double w, d;
+  double2 Z[4];
+  code = kBoundExact;
+  if (!zhyp_setup_z(app, aqp, apq, aqq, ap ? 1 : -1, w, d, Z)) return w;
+  const double cp = cn[p], cq = cn[q];
+  w = zgram_weight(d, Z, cp - (aqp.x * aqp.x + aqp.y * aqp.y), cq - (apq.x * apq.x + apq.y * apq.y), G[gidx],
+                   ap ? G[npm + gidx] : -G[npm + gidx]);
+  auto sq = [](double2 z) { return z.x * z.x + z.y * z.y; };
+  const double s11 = sq(Z[M11]), s21 = sq(Z[M21]), s12 = sq(Z[M12]), s22 = sq(Z[M22]);
+  const double S = cp + cq, zm = fmax(s11 + s12, s21 + s22);
+  const double k = fabs(1.0 - s11) + fabs(1.0 - s22) + s12 + s21 + 2.0 * sqrt(s11 * s21) + 2.0 * sqrt(s12 * s22);
+  const double e = 1.1 * 0x1p-53 * ((150.0 * zm + 60.0) * S + k * S * (7.0 * n + 64.0) + (2.0 * n + 16.0) * fabs(d));
+  code = (fabs(w) <= 1e300 && S <= 1e300 && e <= 1e300) ? bound_code(e, -1000) : kBoundNone;
+  return w;
+}
+
+// the weights and bounds of all hyperbolic pairs, one thread each ((+, -) order)
+template <typename T>
+__global__ void __launch_bounds__(256)
+k_hyp_filter(State *st, const T *__restrict__ A, const int *__restrict__ plus, const int *__restrict__ minus, int n_plus,
+             int n_minus, int n, const double *__restrict__ G, const double *__restrict__ cn, double *__restrict__ Wm,
+             FilterDev f)
+{
+  if (st->stop || st->halt || !st->filter) return;
+  const long long npm = (long long)n_plus * n_minus, k = blockIdx.x * 256LL + threadIdx.x;
+  bool none = false;
+  if (k < npm) {
+    const int ia = (int)(k / n_minus), ib = (int)(k % n_minus);
+    const int a = plus[ia], b = minus[ib];
+    short code;
+    double w = filter_pair(A, n, a, b, k, npm, G, cn, code);
+    if (code == kBoundExact && w < -JK_HUGE) w = nan_w();
+    f.code[k] = code;
+    Wm[(long long)b * n + a] = w;
+    Wm[(long long)a * n + b] = w;
+    none = (code == kBoundNone);
+    if (none) {
+      const int i = atomicAdd(&st->namb, 1);
+      if (i < f.cap) f.list[i] = (int)k;
+      f.dirty[a] = 1;
+      f.dirty[b] = 1;
+    }
+  }
+  // the bits of the pairs that are already in the list
+  const unsigned m = __ballot_sync(0xFFFFFFFFu, none);
+  if ((threadIdx.x & 31) == 0 && k < npm) f.claim[k >> 5] = m;
+}
+
+// one row's terms of the sequential sum: d = fma(s1, a1, d), d = fma(s2, a2, d)
+struct Terms { double s1, a1, s2, a2; };
+
+__device__ __forceinline__ bool pair_setup(double app, double aqp, double apq, double aqq, int jp, double &w, double &d, Rot &t)
+{
+  return hyp_setup(app, aqp, apq, aqq, jp, w, d, t);
+}
+__device__ __forceinline__ bool pair_setup(double2 app, double2 aqp, double2 apq, double2 aqq, int jp, double &w, double &d, ZRot &t)
+{
+  return zhyp_setup(app, aqp, apq, aqq, jp, w, d, t);
+}
+__device__ __forceinline__ Terms pair_terms(double x, double y, const Rot &t)
+{
+  double xx = x, yy = y;
+  rot_apply(t, xx, yy);
+  return Terms{ __dsub_rn(x, xx), __dadd_rn(x, xx), __dsub_rn(y, yy), __dadd_rn(y, yy) };
+}
+__device__ __forceinline__ Terms pair_terms(double2 x, double2 y, const ZRot &t)
+{
+  double2 xx = x, yy = y;
+  zrot_apply_ab(t, xx, yy);
+  const double ax = zabs(x), bx = zabs(xx), ay = zabs(y), by = zabs(yy);
+  return Terms{ __dsub_rn(ax, bx), __dadd_rn(ax, bx), __dsub_rn(ay, by), __dadd_rn(ay, by) };
+}
+
+// the exact weights of the listed pairs, a warp each: the lanes form the terms of 32 rows, every lane
+// runs the chain over them in row order.  Bound by the chain's latency, 46 cycles a row.
+template <typename T>
+__global__ void __launch_bounds__(256)
+k_exact_pairs(const State *st, const T *__restrict__ A, const int *__restrict__ plus, const int *__restrict__ minus,
+              int n_minus, int n, double *__restrict__ Wm, FilterDev f)
+{
+  if (st->stop || st->halt || !st->filter || st->namb > f.cap) return;
+  __shared__ Terms sh[8][2][32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, cnt = st->namb;
+  for (int i = blockIdx.x * 8 + warp; i < cnt; i += gridDim.x * 8) {
+    const int k = f.list[i], a = plus[k / n_minus], b = minus[k % n_minus];
+    const bool ap = a < b;
+    const int p = ap ? a : b, q = ap ? b : a;
+    const T *x = A + (long long)p * n, *y = A + (long long)q * n;
+    double w, d = 0.0;
+    typename Tr<T>::R t;
+    if (pair_setup(x[p], x[q], y[p], y[q], ap ? 1 : -1, w, d, t)) {
+      T nx = Tr<T>::zero(), ny = Tr<T>::zero();
+      if (lane < n) { nx = x[lane]; ny = y[lane]; }
+      for (int r0 = 0, buf = 0; r0 < n; r0 += 32, buf ^= 1) {
+        const T cx = nx, cy = ny;
+        if (r0 + 32 + lane < n) { nx = x[r0 + 32 + lane]; ny = y[r0 + 32 + lane]; }
+        sh[warp][buf][lane] = pair_terms(cx, cy, t);
+        __syncwarp();
+        const int rows = min(32, n - r0);
+#pragma unroll 4
+        for (int r = 0; r < rows; ++r) {
+          const Terms v = sh[warp][buf][r];
+          if (r0 + r != p && r0 + r != q) {
+            d = fma(v.s1, v.a1, d);
+            d = fma(v.s2, v.a2, d);
+          }
+        }
+      }
+      w = d;
+      __syncwarp();
+    }
+    if (lane == 0) {
+      if (w < -JK_HUGE) w = nan_w();
+      Wm[(long long)q * n + p] = w;
+      Wm[(long long)p * n + q] = w;
+    }
+  }
+}
+
+template <typename T>
+cudaError_t filter_t(Workspace &w, const T *A, cudaStream_t s)
+{
+  const cudaError_t e = launch_gram(w, A, s);
+  if (e != cudaSuccess) return e;
+  const long long npm = (long long)w.n_plus * w.n_minus;
+  k_hyp_filter<T><<<(unsigned)((npm + 255) / 256), 256, 0, s>>>(w.st, A, w.plus, w.minus, w.n_plus, w.n_minus, w.n, w.gram,
+                                                                w.cn, w.Wm, w.fd);
+  return cudaGetLastError();
+}
+
+}  // namespace
+
+cudaError_t launch_filter(Workspace &w, const void *A, cudaStream_t s)
+{
+  return w.cplx ? filter_t(w, (const double2 *)A, s) : filter_t(w, (const double *)A, s);
+}
+
+cudaError_t launch_exact(Workspace &w, const void *A, cudaStream_t s)
+{
+  if (w.cplx)
+    k_exact_pairs<double2><<<148 * 4, 256, 0, s>>>(w.st, (const double2 *)A, w.plus, w.minus, w.n_minus, w.n, w.Wm, w.fd);
+  else
+    k_exact_pairs<double><<<148 * 4, 256, 0, s>>>(w.st, (const double *)A, w.plus, w.minus, w.n_minus, w.n, w.Wm, w.fd);
+  return cudaGetLastError();
+}
+
+}  // namespace jk

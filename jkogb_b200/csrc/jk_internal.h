@@ -36,6 +36,10 @@ struct State {
   int retry;         // a learned step without an effective pivot: the loop goes on with an exact step
   double off, best_off;  // off-norm after the last step, its minimum so far
   long long limit;   // the loop waits (stop = 2) once `steps` reaches this (0: never)
+  // the filtered exact ranking (jk_filter.cu)
+  int filter;        // this step ranks by the filter (0: the full scan)
+  int namb;          // pairs of this step that have to be summed exactly
+  int direct;        // steps left that take the full scan at once
 };
 
 // Per-step trace on the device (optional).
@@ -78,6 +82,19 @@ struct ScorerDev {
   int nf;
 };
 
+// the filter's buffers; a pair's bound is 2^code
+constexpr short kBoundExact = -32768, kBoundNone = 32767;
+constexpr long long kHypTileMin = 512LL * 148 * 2;  // real hyperbolic pairs from which the scan takes its large tiles
+constexpr int kDirectSteps = 64;  // full scans after a step with too many ambiguous pairs
+struct FilterDev {
+  short *code;       // n_plus x n_minus bounds
+  unsigned *claim;   // a bit per pair that is in the list
+  int *list;         // the pairs to be summed exactly
+  int *dirty;        // per vertex: its list has to be ranked again
+  int *cls;          // per vertex: its index in its sign class (+), or the complement of it (-)
+  int cap;           // capacity of the list; with more pairs the step takes the full scan
+};
+
 struct Workspace {
   int n;
   int cplx;
@@ -102,6 +119,8 @@ struct Workspace {
   ScorerDev sc;      // sc.nf == 0: the Gram form alone (no network)
   double *gram;      // scored steps: n_plus x n_minus products of the columns without their diagonal
   double *cn;        // ... and the columns' off-diagonal squared norms
+  int filter;        // the exact ranking is filtered (jk_filter.cu)
+  FilterDev fd;
   // ID_NCP = 3 (AW_NCP3): per record key and tie, the sorted order, every start's walk
   int id_ncp;
   unsigned long long *n3key;
@@ -150,6 +169,10 @@ constexpr int kMlpHidden = 64;
 constexpr int kMlpFeat = 8;
 __host__ __device__ constexpr int mlp_params(int nf) { return kMlpHidden * nf + kMlpHidden + kMlpHidden * kMlpHidden + kMlpHidden + kMlpHidden + 1; }
 cudaError_t launch_learned_weights(Workspace &w, const void *A, cudaStream_t s);
+cudaError_t launch_gram(Workspace &w, const void *A, cudaStream_t s);  // column norms, Gram products
+// the filtered exact ranking (jk_filter.cu)
+cudaError_t launch_filter(Workspace &w, const void *A, cudaStream_t s);
+cudaError_t launch_exact(Workspace &w, const void *A, cudaStream_t s);
 cudaError_t prepare_gram();
 constexpr int kOffBlocks = 296;  // fixed grid of the off-norm reduction (a fixed summation order)
 cudaError_t launch_offnorm(Workspace &w, const void *A, cudaStream_t s);

@@ -48,7 +48,7 @@ __global__ void k_identity2(T *U, T *Z, int n)
 
 // the loop state at the start of a solve (S = steps0; 0 for a new solve); the trace
 // capacities are kept, the learned-ranking settings are the caller's
-__global__ void k_state_init(State *st, int learned, int stall_k, int steps0)
+__global__ void k_state_init(State *st, int learned, int stall_k, int steps0, int filter)
 {
   const int cap_s = st->trace_cap_steps, on = st->trace_on;
   const long long cap_p = st->trace_cap_piv;
@@ -61,6 +61,7 @@ __global__ void k_state_init(State *st, int learned, int stall_k, int steps0)
   z.learned = learned;
   z.learned_step = learned;
   z.stall_k = stall_k;
+  z.filter = filter;
   z.best_off = __longlong_as_double(0x7FF0000000000000LL);  // +inf
   *st = z;
 }
@@ -142,6 +143,13 @@ __global__ void k_jztj(T *Z, const int *J, int n)
       }
     }
   }
+}
+
+// Whether a step leaves out the column scans: at the loop's end, in a learned step (the scorer
+// ranks the pairs) and in a filtered one without more than cap ambiguous pairs.
+__device__ __forceinline__ bool scan_off(const State *st, int cap)
+{
+  return st->stop || st->halt || st->learned_step || (st->filter && st->namb <= cap);
 }
 
 // ---------------------------------------------------------------------------
@@ -380,9 +388,9 @@ static __device__ __noinline__ int tile_setup(const double *__restrict__ A, int 
 // thread's pairs share once per row pair.
 __global__ void __launch_bounds__(SCAN_THREADS, 2)
 k_hyp_pm(const State *st, const double *__restrict__ A, const int *__restrict__ plus, const int *__restrict__ minus,
-         int n_plus, int n_minus, int n, double *__restrict__ Wm)
+         int n_plus, int n_minus, int n, double *__restrict__ Wm, int cap)
 {
-  if (st->stop || st->halt || st->learned_step) return;  // a learned step ranks these pairs by the scorer
+  if (scan_off(st, cap)) return;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int TM = (n_minus + TW - 1) / TW;
   const int P0 = (blockIdx.x / TM) * TW, Q0 = (blockIdx.x % TM) * TW;
@@ -516,9 +524,9 @@ k_hyp_pm(const State *st, const double *__restrict__ A, const int *__restrict__ 
 // |A(i,j)| of every entry of a complex A (the project's hypot), once per step: the
 // column scan of ABODNZF2 needs the magnitude of every unrotated entry of its two
 // columns, and every pair of a column would otherwise compute it again
-__global__ void k_absmat(const State *st, const double2 *__restrict__ A, long long nn, double *__restrict__ mag)
+__global__ void k_absmat(const State *st, const double2 *__restrict__ A, long long nn, double *__restrict__ mag, int cap)
 {
-  if (st->stop || st->halt || st->learned_step) return;
+  if (scan_off(st, cap)) return;
   for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < nn; k += (long long)gridDim.x * blockDim.x)
     mag[k] = zabs(A[k]);
 }
@@ -530,9 +538,9 @@ __global__ void k_absmat(const State *st, const double2 *__restrict__ A, long lo
 template <int HP, int HM>
 __global__ void __launch_bounds__(HP * HM)
 k_weights_hyp_z(const State *st, const double2 *__restrict__ A, const double *__restrict__ mag, const int *__restrict__ plus,
-                const int *__restrict__ minus, int n_plus, int n_minus, double *__restrict__ Wm, int n)
+                const int *__restrict__ minus, int n_plus, int n_minus, double *__restrict__ Wm, int n, int cap)
 {
-  if (st->stop || st->halt || st->learned_step) return;  // a learned step ranks these pairs by the scorer
+  if (scan_off(st, cap)) return;
   __shared__ double2 sP[HP][ZHR + 1];
   __shared__ double2 sM[HM][ZHR + 1];
   __shared__ double aP[HP][ZHR + 1];
@@ -682,9 +690,9 @@ __device__ __forceinline__ void zscan_rows(const double2 *const *xs, const doubl
 // the tile's 48 columns and their magnitudes stream through two buffers in row chunks.
 __global__ void __launch_bounds__(ZTHREADS, 2)
 k_hyp_z_pm(const State *st, const double2 *__restrict__ A, const double *__restrict__ mag, const int *__restrict__ plus,
-           const int *__restrict__ minus, int n_plus, int n_minus, int n, double *__restrict__ Wm)
+           const int *__restrict__ minus, int n_plus, int n_minus, int n, double *__restrict__ Wm, int cap)
 {
-  if (st->stop || st->halt || st->learned_step) return;  // a learned step ranks these pairs by the scorer
+  if (scan_off(st, cap)) return;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int TM = (n_minus + ZTM - 1) / ZTM;
   const int P0 = (blockIdx.x / TM) * ZTP, Q0 = (blockIdx.x % TM) * ZTM;
@@ -832,9 +840,9 @@ k_hyp_z_pm(const State *st, const double2 *__restrict__ A, const double *__restr
 template <int HP, int HM>
 __global__ void __launch_bounds__(HP * HM)
 k_weights_hyp(const State *st, const double *__restrict__ A, const int *__restrict__ plus, const int *__restrict__ minus,
-              int n_plus, int n_minus, double *__restrict__ Wm, int n)
+              int n_plus, int n_minus, double *__restrict__ Wm, int n, int cap)
 {
-  if (st->stop || st->halt || st->learned_step) return;  // a learned step ranks these pairs by the scorer
+  if (scan_off(st, cap)) return;
   __shared__ double sP[HP][HR + 1];
   __shared__ double sM[HM][HR + 1];
   const int tx = threadIdx.x % HP, ty = threadIdx.x / HP;
@@ -1009,11 +1017,104 @@ __device__ __forceinline__ void block_sort_desc(unsigned long long (&k)[E], unsi
   }
 }
 
+// The pairs of a list (sk, sorted by the filtered weights) whose order is not certain.  Position i is
+// cut from i + 1 where every interval up to i lies above every one from i + 1 on; an
+// approximate weight without a cut on either side is ambiguous.  (Exact weights among
+// themselves are in order.)
 template <int E>
+__device__ __forceinline__ void mark_ambiguous(State *st, const double *col, int v, int cnt, unsigned long long *sk, unsigned short *slo,
+                                               const FilterDev &f, int n_minus)
+{
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  __shared__ double s_lo[SORT_THREADS / 32], s_hi[SORT_THREADS / 32];
+  const double inf = __longlong_as_double(0x7FF0000000000000LL);
+  const int cv = f.cls[v];
+  double lo[E], hi[E];
+  int pair[E];
+#pragma unroll
+  for (int e = 0; e < E; ++e) {
+    const int i = tid * E + e;
+    lo[e] = inf;
+    hi[e] = -inf;
+    pair[e] = -1;
+    if (i < cnt) {
+      const int u = ckey_u(sk[i], v), cu = f.cls[u];
+      const double w = col[u];
+      lo[e] = hi[e] = w;
+      if ((cv < 0) != (cu < 0)) {
+        const int k = ((cv < 0) ? cu : cv) * n_minus + ~((cv < 0) ? cv : cu);
+        const short c = f.code[k];
+        // (a pair without a bound is summed anyway, and its lists are ranked again)
+        if (c != kBoundExact && c != kBoundNone) {
+          const double r = (c >= -1022) ? pow2(c) : __longlong_as_double(1LL << (c + 1074));
+          pair[e] = k;
+          lo[e] = __dsub_rd(w, r);
+          hi[e] = __dadd_ru(w, r);
+        }
+      }
+    }
+  }
+  __syncthreads();
+  // the least lower end up to each position, the greatest upper end from each position on
+#pragma unroll
+  for (int e = 1; e < E; ++e) lo[e] = fmin(lo[e], lo[e - 1]);
+#pragma unroll
+  for (int e = E - 2; e >= 0; --e) hi[e] = fmax(hi[e], hi[e + 1]);
+  double a = lo[E - 1], b = hi[0];
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const double x = __shfl_up_sync(0xFFFFFFFFu, a, o), y = __shfl_down_sync(0xFFFFFFFFu, b, o);
+    if (lane >= o) a = fmin(a, x);
+    if (lane + o < 32) b = fmax(b, y);
+  }
+  if (lane == 31) s_lo[warp] = a;
+  if (lane == 0) s_hi[warp] = b;
+  const double al = __shfl_up_sync(0xFFFFFFFFu, a, 1), bl = __shfl_down_sync(0xFFFFFFFFu, b, 1);
+  __syncthreads();
+  double pl = lane > 0 ? al : inf, sh = lane < 31 ? bl : -inf;
+#pragma unroll
+  for (int k = 0; k < SORT_THREADS / 32; ++k) {
+    if (k < warp) pl = fmin(pl, s_lo[k]);
+    if (k > warp) sh = fmax(sh, s_hi[k]);
+  }
+  double *S = (double *)sk;
+#pragma unroll
+  for (int e = 0; e < E; ++e) S[tid * E + e] = fmax(hi[e], sh);
+  __syncthreads();
+#pragma unroll
+  for (int e = 0; e < E; ++e) {
+    const int i = tid * E + e;
+    slo[i] = (i >= cnt - 1 || fmin(lo[e], pl) > S[i + 1]) ? 1 : 0;  // cut after i
+  }
+  __syncthreads();
+#pragma unroll
+  for (int e = 0; e < E; ++e) {
+    const int i = tid * E + e;
+    if (pair[e] >= 0 && !(slo[i] && (i == 0 || slo[i - 1]))) {
+      f.dirty[v] = 1;
+      if (!((atomicOr(&f.claim[pair[e] >> 5], 1u << (pair[e] & 31)) >> (pair[e] & 31)) & 1u)) {
+        const int x = atomicAdd(&st->namb, 1);
+        if (x < f.cap) f.list[x] = pair[e];
+      }
+    }
+  }
+}
+
+// MODE 0: the lists of the exact weights.  MODE 1: the lists of the filtered weights; the pairs
+// whose interval meets that of a neighbour go to the list of pairs to be summed exactly, and the
+// vertex is marked to be ranked again.  MODE 2: those vertices again, or all after a full scan.
+template <int E, int MODE>
 __global__ void __launch_bounds__(SORT_THREADS)
-k_colsort(const State *st, const double *__restrict__ Wm, int n, unsigned short *list, int *len)
+k_colsort(State *st, const double *__restrict__ Wm, int n, unsigned short *list, int *len, FilterDev f, int n_minus)
 {
   if (st->stop || st->halt) return;
+  if (MODE == 1 && !st->filter) return;
+  if (MODE == 2) {
+    const int d = f.dirty[blockIdx.x];
+    if (st->filter && st->namb <= f.cap && !d) return;
+    __syncthreads();
+    if (threadIdx.x == 0 && d) f.dirty[blockIdx.x] = 0;
+  }
   __shared__ unsigned long long sk[SORT_THREADS * E];
   __shared__ unsigned short slo[SORT_THREADS * E];  // low 16 bits of the sorted keys' weight keys
   __shared__ int s_cnt, s_warp[SORT_THREADS / 32];
@@ -1097,6 +1198,7 @@ k_colsort(const State *st, const double *__restrict__ Wm, int n, unsigned short 
   for (int r = tid; r < cnt; r += blockDim.x) {
     lv[r] = (unsigned short)ckey_u(sk[r], v);
   }
+  if constexpr (MODE == 1) mark_ambiguous<E>(st, col, v, cnt, sk, slo, f, n_minus);
   // the last group of 8 is read whole
   if (tid < 8 && cnt + tid < ((cnt + 7) & ~7)) lv[cnt + tid] = 0;
   if (tid == 0) len[v] = cnt;
@@ -1261,7 +1363,7 @@ template <typename T>
 __global__ void __launch_bounds__(kSelThreads, 1)
 k_select(State *st, const double *__restrict__ Wm, const int *__restrict__ J, int n, int n_2,
          const unsigned short *__restrict__ list, const int *__restrict__ len, const T *__restrict__ A, Piv<T> *piv,
-         RowRot<T> *rr, int *unp, Trace tr, int quirk, int early)
+         RowRot<T> *rr, int *unp, Trace tr, int quirk, int early, int cap)
 {
   cg::cluster_group cluster = cg::this_cluster();
   const int C = (int)cluster.num_blocks(), c = (int)cluster.block_rank();
@@ -1504,6 +1606,12 @@ k_select(State *st, const double *__restrict__ Wm, const int *__restrict__ J, in
     st->sl = sl;
     st->nunp = s_nunp;
     st->rounds = rounds;
+    if (cap >= 0) {
+      // how the next step ranks
+      if (!st->filter) { if (--st->direct <= 0) st->filter = 1; }
+      else if (st->namb > cap) { st->filter = 0; st->direct = kDirectSteps; }
+      st->namb = 0;
+    }
     if (sl <= 0) {
       // DSTEP_EXEC returns with SL = 0: the loop ends with INFO = S (src/D/dstep.F90:421, 575-582)
       st->info = st->steps;
@@ -1861,7 +1969,7 @@ cudaError_t prepare_kernels(int n)
 template <typename T>
 static cudaError_t init_t(Workspace &w, T *U, T *Z, int learned, int stall_k, int steps0, int fresh, cudaStream_t s)
 {
-  k_state_init<<<1, 1, 0, s>>>(w.st, learned, stall_k, steps0);
+  k_state_init<<<1, 1, 0, s>>>(w.st, learned, stall_k, steps0, w.filter);
   if (fresh) k_identity2<T><<<grid1((long long)w.n * w.n, 256), 256, 0, s>>>(U, Z, w.n);
   return cudaGetLastError();
 }
@@ -1904,47 +2012,54 @@ static void hyp_d_launch(Workspace &w, const double *A, cudaStream_t s)
 {
   const int nt = ((w.n_plus + TW - 1) / TW) * ((w.n_minus + TW - 1) / TW);
   const size_t smem = SCAN_STAGES * (2 * TW) * SCAN_RS * sizeof(double);
-  k_hyp_pm<<<nt, SCAN_THREADS, smem, s>>>(w.st, A, w.plus, w.minus, w.n_plus, w.n_minus, w.n, w.Wm);
+  k_hyp_pm<<<nt, SCAN_THREADS, smem, s>>>(w.st, A, w.plus, w.minus, w.n_plus, w.n_minus, w.n, w.Wm, w.fd.cap);
 }
 
 static void hyp_small_launch(const State *st, const double *A, const int *plus, const int *minus, int n_plus, int n_minus,
-                             double *W, int n, cudaStream_t s)
+                             double *W, int n, int cap, cudaStream_t s)
 {
   if ((long long)n_plus * n_minus >= 256LL * 148 * 4) {
     dim3 gh((n_plus + 15) / 16, (n_minus + 15) / 16);
-    k_weights_hyp<16, 16><<<gh, 256, 0, s>>>(st, A, plus, minus, n_plus, n_minus, W, n);
+    k_weights_hyp<16, 16><<<gh, 256, 0, s>>>(st, A, plus, minus, n_plus, n_minus, W, n, cap);
   }
   else {
     dim3 gh((n_plus + 7) / 8, (n_minus + 7) / 8);
-    k_weights_hyp<8, 8><<<gh, 64, 0, s>>>(st, A, plus, minus, n_plus, n_minus, W, n);
+    k_weights_hyp<8, 8><<<gh, 64, 0, s>>>(st, A, plus, minus, n_plus, n_minus, W, n, cap);
   }
+}
+
+template <typename T>
+static cudaError_t trig_t(Workspace &w, const T *A, cudaStream_t s)
+{
+  const int n = w.n;
+  dim3 bt(32, 8), gt((n + 31) / 32, (n + 7) / 8);
+  k_weights_trig<T><<<gt, bt, 0, s>>>(w.st, A, w.J, w.Wm, n);
+  return cudaGetLastError();
 }
 
 template <typename T>
 static cudaError_t weights_t(Workspace &w, const T *A, cudaStream_t s)
 {
   const int n = w.n;
-  dim3 bt(32, 8), gt((n + 31) / 32, (n + 7) / 8);
-  k_weights_trig<T><<<gt, bt, 0, s>>>(w.st, A, w.J, w.Wm, n);
   if (w.n_plus > 0 && w.n_minus > 0) {
     const long long nh = (long long)w.n_plus * w.n_minus;
     if constexpr (sizeof(T) == sizeof(double)) {
       // the pipelined kernel once its tiles fill the GPU; 16 x 16 / 8 x 8 tiles otherwise
-      if (nh >= 512LL * 148 * 2) hyp_d_launch(w, A, s);
-      else hyp_small_launch(w.st, A, w.plus, w.minus, w.n_plus, w.n_minus, w.Wm, n, s);
+      if (nh >= kHypTileMin) hyp_d_launch(w, A, s);
+      else hyp_small_launch(w.st, A, w.plus, w.minus, w.n_plus, w.n_minus, w.Wm, n, w.fd.cap, s);
     }
     else {
       // the magnitudes of all entries once, then the tiles
       const long long nn = (long long)n * n;
-      k_absmat<<<(unsigned)((nn + 255) / 256 < 4096 ? (nn + 255) / 256 : 4096), 256, 0, s>>>(w.st, A, nn, w.mag);
+      k_absmat<<<(unsigned)((nn + 255) / 256 < 4096 ? (nn + 255) / 256 : 4096), 256, 0, s>>>(w.st, A, nn, w.mag, w.fd.cap);
       if (nh >= (long long)ZTP * ZTM * 148) {
         // the pipelined tiles once they fill the GPU
         const int nt = ((w.n_plus + ZTP - 1) / ZTP) * ((w.n_minus + ZTM - 1) / ZTM);
-        k_hyp_z_pm<<<nt, ZTHREADS, kZSmem, s>>>(w.st, A, w.mag, w.plus, w.minus, w.n_plus, w.n_minus, n, w.Wm);
+        k_hyp_z_pm<<<nt, ZTHREADS, kZSmem, s>>>(w.st, A, w.mag, w.plus, w.minus, w.n_plus, w.n_minus, n, w.Wm, w.fd.cap);
       }
       else {
         dim3 gh((w.n_plus + 7) / 8, (w.n_minus + 7) / 8);
-        k_weights_hyp_z<8, 8><<<gh, 64, 0, s>>>(w.st, A, w.mag, w.plus, w.minus, w.n_plus, w.n_minus, w.Wm, n);
+        k_weights_hyp_z<8, 8><<<gh, 64, 0, s>>>(w.st, A, w.mag, w.plus, w.minus, w.n_plus, w.n_minus, w.Wm, n, w.fd.cap);
       }
     }
   }
@@ -1953,18 +2068,21 @@ static cudaError_t weights_t(Workspace &w, const T *A, cudaStream_t s)
 
 cudaError_t launch_weights(Workspace &w, const void *A, cudaStream_t s)
 {
+  const cudaError_t e = w.cplx ? trig_t(w, (const double2 *)A, s) : trig_t(w, (const double *)A, s);
+  if (e != cudaSuccess) return e;
   return w.cplx ? weights_t(w, (const double2 *)A, s) : weights_t(w, (const double *)A, s);
 }
 
+template <int MODE>
 static cudaError_t colsort(Workspace &w, cudaStream_t s)
 {
   const int n = w.n;
   switch (colsort_e(n)) {
-  case 1: k_colsort<1><<<n, SORT_THREADS, 0, s>>>(w.st, w.Wm, n, w.list, w.len); break;
-  case 2: k_colsort<2><<<n, SORT_THREADS, 0, s>>>(w.st, w.Wm, n, w.list, w.len); break;
-  case 4: k_colsort<4><<<n, SORT_THREADS, 0, s>>>(w.st, w.Wm, n, w.list, w.len); break;
-  case 8: k_colsort<8><<<n, SORT_THREADS, 0, s>>>(w.st, w.Wm, n, w.list, w.len); break;
-  case 16: k_colsort<16><<<n, SORT_THREADS, 0, s>>>(w.st, w.Wm, n, w.list, w.len); break;
+  case 1: k_colsort<1, MODE><<<n, SORT_THREADS, 0, s>>>(w.st, w.Wm, n, w.list, w.len, w.fd, w.n_minus); break;
+  case 2: k_colsort<2, MODE><<<n, SORT_THREADS, 0, s>>>(w.st, w.Wm, n, w.list, w.len, w.fd, w.n_minus); break;
+  case 4: k_colsort<4, MODE><<<n, SORT_THREADS, 0, s>>>(w.st, w.Wm, n, w.list, w.len, w.fd, w.n_minus); break;
+  case 8: k_colsort<8, MODE><<<n, SORT_THREADS, 0, s>>>(w.st, w.Wm, n, w.list, w.len, w.fd, w.n_minus); break;
+  case 16: k_colsort<16, MODE><<<n, SORT_THREADS, 0, s>>>(w.st, w.Wm, n, w.list, w.len, w.fd, w.n_minus); break;
   default: return cudaErrorInvalidValue;
   }
   return cudaGetLastError();
@@ -1990,7 +2108,7 @@ static cudaError_t select_t(Workspace &w, const T *A, int n_2, cudaStream_t s)
     }
   }
   else {
-    e = colsort(w, s);
+    e = w.filter ? colsort<2>(w, s) : colsort<0>(w, s);
     if (e != cudaSuccess) return e;
     const int C = select_cluster(n);
     cudaLaunchConfig_t cfg = {};
@@ -2006,7 +2124,7 @@ static cudaError_t select_t(Workspace &w, const T *A, int n_2, cudaStream_t s)
     cfg.numAttrs = 1;
     e = cudaLaunchKernelEx(&cfg, k_select<T>, w.st, (const double *)w.Wm, (const int *)w.J, n, n_2,
                            (const unsigned short *)w.list, (const int *)w.len, A, (Piv<T> *)w.piv, (RowRot<T> *)w.rowrot,
-                           w.unp, w.tr, w.zba_quirk, w.learned ? 0 : 1);
+                           w.unp, w.tr, w.zba_quirk, w.learned ? 0 : 1, w.filter ? w.fd.cap : -1);
     if (e != cudaSuccess) return e;
   }
   return cudaGetLastError();
@@ -2021,8 +2139,16 @@ template <typename T>
 static cudaError_t step_t(Workspace &w, T *A, T *U, T *Z, int n_2, cudaStream_t s)
 {
   const int n = w.n;
-  cudaError_t e = weights_t(w, (const T *)A, s);
+  cudaError_t e = trig_t(w, (const T *)A, s);
   if (e != cudaSuccess) return e;
+  const bool hyp = w.n_plus > 0 && w.n_minus > 0;
+  if (w.filter && hyp) {
+    // the filtered weights, the lists, the exact weights of what is ambiguous in them
+    if ((e = launch_filter(w, A, s)) != cudaSuccess) return e;
+    if ((e = colsort<1>(w, s)) != cudaSuccess) return e;
+    if ((e = launch_exact(w, A, s)) != cudaSuccess) return e;
+  }
+  if ((e = weights_t(w, (const T *)A, s)) != cudaSuccess) return e;
   // a learned solve: the scorer ranks the scanned hyperbolic pairs (the exact scan kernels
   // above return at once in its learned steps)
   if (w.learned && (e = launch_learned_weights(w, A, s)) != cudaSuccess) return e;
@@ -2179,7 +2305,7 @@ cudaError_t launch_weights_noalloc(int n, const double *A, const int *J, double 
   const int *dj = (const int *)(d + kScratchState), *dp = dj + kNoallocMaxN, *dm = dp + kNoallocMaxN;
   dim3 bt(32, 8), gt((n + 31) / 32, (n + 7) / 8);
   k_weights_trig<double><<<gt, bt, 0, s>>>(st, A, dj, W, n);
-  if (np > 0 && nm > 0) hyp_small_launch(st, A, dp, dm, np, nm, W, n, s);
+  if (np > 0 && nm > 0) hyp_small_launch(st, A, dp, dm, np, nm, W, n, 0, s);
   return cudaGetLastError();
 }
 

@@ -116,22 +116,8 @@ __device__ __forceinline__ void scan_rows_cplx_mag(const double2 *xs, const doub
 // hyp_setup for a complex pair (ZMAGF2H, src/Z/zstep.F90:43-74)
 __device__ __forceinline__ bool zhyp_setup(double2 app, double2 aqp, double2 apq, double2 aqq, int jp, double &w, double &d, ZRot &t)
 {
-  w = nan_w();
-  if (!may_transform(app, aqp, apq, aqq)) return false;
-  double2 A2[4] = { app, aqp, apq, aqq }, U2[4], Z2[4];
-  int info = 0;
-  zhsvd2(A2, jp, -jp, U2, Z2, JK_TH1FIX, info);
-  if (info < 0) return false;
-  if (!(info & 1)) { w = 0.0; return false; }
-  if (!(info & 4)) { w = dasum4(aqp.x, aqp.y, apq.x, apq.y); return false; }
-  // the four off-diagonal terms that start ABODNZF2
-  const double2 a1 = (info & 8) ? A2[M21] : make_double2(0.0, 0.0);
-  const double2 a2 = (info & 8) ? A2[M12] : make_double2(0.0, 0.0);
-  d = 0.0;
-  d = fma(__dsub_rn(aqp.x, a1.x), __dadd_rn(aqp.x, a1.x), d);
-  d = fma(__dsub_rn(aqp.y, a1.y), __dadd_rn(aqp.y, a1.y), d);
-  d = fma(__dsub_rn(apq.x, a2.x), __dadd_rn(apq.x, a2.x), d);
-  d = fma(__dsub_rn(apq.y, a2.y), __dadd_rn(apq.y, a2.y), d);
+  double2 Z2[4];
+  if (!zhyp_setup_z(app, aqp, apq, aqq, jp, w, d, Z2)) return false;
   t = zrot_ab(Z2);
   return true;
 }

@@ -167,7 +167,7 @@ template <int C>
 __global__ void __launch_bounds__(256)
 k_colnorm(const State *st, const double *__restrict__ A, int n, double *__restrict__ cn)
 {
-  if (st->stop || !st->learned_step) return;
+  if (st->stop || st->halt || !(st->learned_step || st->filter)) return;
   const int lane = threadIdx.x & 31;
   for (int j = blockIdx.x * 8 + (threadIdx.x >> 5); j < n; j += gridDim.x * 8) {
     const double *c = A + (long long)j * C * n;
@@ -305,7 +305,7 @@ __global__ void __launch_bounds__(128)
 k_gram(const State *st, const double *__restrict__ A, const int *__restrict__ plus, const int *__restrict__ minus,
        int n_plus, int n_minus, int n, double *__restrict__ G)
 {
-  if (st->stop || !st->learned_step) return;
+  if (st->stop || st->halt || !(st->learned_step || st->filter)) return;
   if (C == 2 && blockIdx.z) gram_tile<C, true>(A, plus, minus, n_plus, n_minus, n, G + (long long)n_plus * n_minus);
   else gram_tile<C, false>(A, plus, minus, n_plus, n_minus, n, G);
 }
@@ -740,17 +740,30 @@ __global__ void k_mlp_pack(const float *__restrict__ P, unsigned short *w, float
 // ---------------------------------------------------------------------------
 // host launchers
 // ---------------------------------------------------------------------------
+// the column norms and the Gram products of a scored or filtered step
+template <int C>
+static cudaError_t gram_t(Workspace &w, const double *A, cudaStream_t s)
+{
+  const int n = w.n;
+  k_colnorm<C><<<(n + 7) / 8 < 1184 ? (n + 7) / 8 : 1184, 256, 0, s>>>(w.st, A, n, w.cn);
+  dim3 g((w.n_plus + GT - 1) / GT, (w.n_minus + GT - 1) / GT, C);
+  k_gram<C><<<g, 128, 2 * kGramOperand, s>>>(w.st, A, w.plus, w.minus, w.n_plus, w.n_minus, n, w.gram);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_gram(Workspace &w, const void *A, cudaStream_t s)
+{
+  return w.cplx ? gram_t<2>(w, (const double *)A, s) : gram_t<1>(w, (const double *)A, s);
+}
+
 template <typename T>
 static cudaError_t learned_weights_t(Workspace &w, const T *A, cudaStream_t s)
 {
-  constexpr int C = sizeof(T) / sizeof(double);
   if (w.n_plus > 0 && w.n_minus > 0) {
-    const int n = w.n;
-    k_colnorm<C><<<(n + 7) / 8 < 1184 ? (n + 7) / 8 : 1184, 256, 0, s>>>(w.st, (const double *)A, n, w.cn);
-    dim3 g((w.n_plus + GT - 1) / GT, (w.n_minus + GT - 1) / GT, C);
-    k_gram<C><<<g, 128, 2 * kGramOperand, s>>>(w.st, (const double *)A, w.plus, w.minus, w.n_plus, w.n_minus, n, w.gram);
+    const cudaError_t e = launch_gram(w, A, s);
+    if (e != cudaSuccess) return e;
     const long long np = (long long)w.n_plus * w.n_minus;
-    k_hyp_gram<T><<<(unsigned)((np + 255) / 256), 256, 0, s>>>(w.st, A, w.plus, w.minus, w.n_plus, w.n_minus, n,
+    k_hyp_gram<T><<<(unsigned)((np + 255) / 256), 256, 0, s>>>(w.st, A, w.plus, w.minus, w.n_plus, w.n_minus, w.n,
                                                               w.gram, w.cn, w.Wm, w.sc);
   }
   return cudaGetLastError();
