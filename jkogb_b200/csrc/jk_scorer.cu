@@ -59,16 +59,20 @@ __device__ __forceinline__ float lg64(double x)
 // ---------------------------------------------------------------------------
 // the network
 // ---------------------------------------------------------------------------
-// one block's copy of the inference parameters (shared memory)
+// one block's copy of the inference parameters (shared memory).  The rows of W2 are padded by 16
+// bytes: the eight rows that a B fragment's lanes read lay 128 bytes apart, in the same four banks.
+constexpr int HP2 = H + 8;
 struct TNet {
-  unsigned short w1[H * NF], w2[H * H];
+  alignas(16) unsigned short w1[H * NF];
+  alignas(16) unsigned short w2[H * HP2];
   float w3[H], b1[H], b2[H], b3;
 };
 
 __device__ void load_tnet(TNet &s, const unsigned short *w, const float *b)
 {
-  for (int k = threadIdx.x; k < H * NF; k += blockDim.x) s.w1[k] = w[PW_W1 + k];
-  for (int k = threadIdx.x; k < H * H; k += blockDim.x) s.w2[k] = w[PW_W2 + k];
+  for (int k = threadIdx.x; k < H * NF / 8; k += blockDim.x) ((uint4 *)s.w1)[k] = ((const uint4 *)(w + PW_W1))[k];
+  for (int k = threadIdx.x; k < H * H / 8; k += blockDim.x)
+    *(uint4 *)&s.w2[(k / (H / 8)) * HP2 + 8 * (k % (H / 8))] = ((const uint4 *)(w + PW_W2))[k];
   for (int k = threadIdx.x; k < H; k += blockDim.x) {
     s.w3[k] = bf16_load(w[PW_W3 + k]);
     s.b1[k] = b[k];
@@ -76,6 +80,7 @@ __device__ void load_tnet(TNet &s, const unsigned short *w, const float *b)
   }
   if (threadIdx.x == 0) s.b3 = b[2 * H];
 }
+static_assert(PW_W2 % 8 == 0, "16-byte loads of the packed weights");
 
 __device__ __forceinline__ void mma_bf16(float (&c)[4], const unsigned (&a)[4], unsigned b0, unsigned b1)
 {
@@ -122,7 +127,7 @@ __device__ __forceinline__ void mlp16(const TNet &s, const float (*xs)[NF], floa
     a2[3] = pack_bf16(fmaxf(h1[2 * kt + 1][2], 0.0f), fmaxf(h1[2 * kt + 1][3], 0.0f));
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
-      const unsigned short *row = &s.w2[(8 * j + g) * H + 16 * kt + 2 * t];
+      const unsigned short *row = &s.w2[(8 * j + g) * HP2 + 16 * kt + 2 * t];
       mma_bf16(h2[j], a2, *(const unsigned *)row, *(const unsigned *)(row + 8));
     }
   }
@@ -419,7 +424,9 @@ __device__ __forceinline__ GPair gram_pair(const double2 *__restrict__ A, int n,
 __device__ __forceinline__ double corrected(double w, float y) { return w * exp2((double)fminf(fmaxf(y, -1.0f), 1.0f) * 0.125); }
 
 // the weights of the hyperbolic pairs in a scored step (one thread per pair, (+, -) order);
-// with a network, every warp scores its 32 pairs as two tiles of 16 on the tensor cores
+// with a network, every warp scores its 32 pairs as two tiles of 16 on the tensor cores.  A block
+// loads the network once for all its pairs (grid-stride: with one block per 256 pairs the loads, and
+// the bank conflicts of W2's fragments, took 182 us at N = 2048; 153 us now).
 template <typename T>
 __global__ void __launch_bounds__(256)
 k_hyp_gram(const State *st, const T *__restrict__ A, const int *__restrict__ plus, const int *__restrict__ minus,
@@ -433,35 +440,37 @@ k_hyp_gram(const State *st, const T *__restrict__ A, const int *__restrict__ plu
   const bool with_net = (sc.nf == NF);
   if (with_net) load_tnet(net, sc.w, sc.b);
   __syncthreads();
-  const long long k = blockIdx.x * 256LL + threadIdx.x;
-  const bool valid = k < (long long)n_plus * n_minus;
+  const long long npm = (long long)n_plus * n_minus;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  int ia = 0, ib = 0;
-  GPair r;
-  r.w = nan_w();
-  r.scan = 0;
-  if (valid) {
-    ia = (int)(k / n_minus);
-    ib = (int)(k % n_minus);
-    r = gram_pair(A, n, plus[ia], minus[ib], (long long)ia * n_minus + ib, (long long)n_plus * n_minus, G, cn,
-                  st->steps);
-  }
-  if (with_net && __any_sync(0xFFFFFFFFu, r.scan)) {
+  for (long long k0 = blockIdx.x * 256LL; k0 < npm; k0 += gridDim.x * 256LL) {
+    const long long k = k0 + threadIdx.x;
+    const bool valid = k < npm;
+    int a = 0, b = 0;
+    GPair r;
+    r.w = nan_w();
+    r.scan = 0;
+    if (valid) {
+      const int ia = (int)(k / n_minus), ib = (int)(k % n_minus);
+      a = plus[ia];
+      b = minus[ib];
+      r = gram_pair(A, n, a, b, k, npm, G, cn, st->steps);
+    }
+    if (with_net && __any_sync(0xFFFFFFFFu, r.scan)) {
 #pragma unroll
-    for (int f = 0; f < NF; ++f) xs[warp][lane][f] = r.scan ? r.x[f] : 0.0f;
-    __syncwarp();
-    mlp16(net, xs[warp], ys[warp]);
-    mlp16(net, xs[warp] + 16, ys[warp] + 16);
-    __syncwarp();
-    if (r.scan) r.w = corrected(r.w, ys[warp][lane]);
+      for (int f = 0; f < NF; ++f) xs[warp][lane][f] = r.scan ? r.x[f] : 0.0f;
+      __syncwarp();
+      mlp16(net, xs[warp], ys[warp]);
+      mlp16(net, xs[warp] + 16, ys[warp] + 16);
+      __syncwarp();
+      if (r.scan) r.w = corrected(r.w, ys[warp][lane]);
+      __syncwarp();
+    }
+    if (!valid) continue;
+    double w = r.w;
+    if (w < -JK_HUGE) w = nan_w();
+    Wm[(long long)b * n + a] = w;
+    Wm[(long long)a * n + b] = w;
   }
-  if (!valid) return;
-  double w = r.w;
-  if (w < -JK_HUGE) w = nan_w();
-  const int a = plus[ia], b = minus[ib];
-  const int p = a < b ? a : b, q = a < b ? b : a;
-  Wm[(long long)q * n + p] = w;
-  Wm[(long long)p * n + q] = w;
 }
 
 // training data: the features and w_gram of every hyperbolic pair ((+, -) order); the
@@ -762,9 +771,9 @@ static cudaError_t learned_weights_t(Workspace &w, const T *A, cudaStream_t s)
   if (w.n_plus > 0 && w.n_minus > 0) {
     const cudaError_t e = launch_gram(w, A, s);
     if (e != cudaSuccess) return e;
-    const long long np = (long long)w.n_plus * w.n_minus;
-    k_hyp_gram<T><<<(unsigned)((np + 255) / 256), 256, 0, s>>>(w.st, A, w.plus, w.minus, w.n_plus, w.n_minus, w.n,
-                                                              w.gram, w.cn, w.Wm, w.sc);
+    const long long nb = ((long long)w.n_plus * w.n_minus + 255) / 256, cap = 148LL * 2;  // two blocks fit an SM
+    k_hyp_gram<T><<<(unsigned)(nb < cap ? nb : cap), 256, 0, s>>>(w.st, A, w.plus, w.minus, w.n_plus, w.n_minus, w.n,
+                                                                  w.gram, w.cn, w.Wm, w.sc);
   }
   return cudaGetLastError();
 }
