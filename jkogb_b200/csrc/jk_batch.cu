@@ -25,6 +25,7 @@
 // first), so the launch is persistent and balances itself.
 #include "jk_internal.h"
 #include "jk_device.cuh"
+#include "jk_scan.cuh"
 
 namespace jk {
 
@@ -71,33 +72,6 @@ __device__ __forceinline__ bool rbetter(double w1, unsigned t1, double w2, unsig
 }
 
 __device__ __forceinline__ unsigned rtie(int p, int q) { return ((unsigned)(q - p) << 16) | (unsigned)p; }
-
-// ABODNDF2's sequential sum over the rows i != p, q of the columns xs (p), ys (q)
-// under the AB coefficients t (src/D/dtransf.F90:246-348)
-__device__ __forceinline__ void scan_pair(const double *xs, const double *ys, int n, int p, int q, const Rot &t, double &d)
-{
-  if (t.c1 && t.c2) {
-#pragma unroll 4
-    for (int i = 0; i < n; ++i) {
-      const double x = xs[i], y = ys[i];
-      const double xx = __dmul_rn(fma(y, t.r1, x), t.m1);
-      const double yy = __dmul_rn(fma(x, t.r2, y), t.m2);
-      const double e1 = fma(__dsub_rn(x, xx), __dadd_rn(x, xx), d);
-      const double e2 = fma(__dsub_rn(y, yy), __dadd_rn(y, yy), e1);
-      d = (i != p && i != q) ? e2 : d;
-    }
-  }
-  else {
-    for (int i = 0; i < n; ++i) {
-      double x = xs[i], y = ys[i];
-      const double x0 = x, y0 = y;
-      rot_apply(t, x, y);
-      const double e1 = fma(__dsub_rn(x0, x), __dadd_rn(x0, x), d);
-      const double e2 = fma(__dsub_rn(y0, y), __dadd_rn(y0, y), e1);
-      d = (i != p && i != q) ? e2 : d;
-    }
-  }
-}
 
 // scored: rank the scanned hyperbolic pairs by the Gram form of their weights (squared
 // column norms and the column products without rows p, q; one fma per row instead of the
@@ -239,7 +213,7 @@ __device__ void solve_one(const BatchItem &it, double *__restrict__ gA, double *
         double w, d = 0.0;
         Rot t;
         if (hyp_setup(xs[p], xs[q], ys[p], ys[q], a_is_p ? 1 : -1, w, d, t)) {
-          scan_pair(xs, ys, n, p, q, t, d);
+          scan_rows_real(xs, ys, n, 0, p, q, t, d);
           w = d;
         }
         if (w < -JK_HUGE) w = nan_w();
@@ -277,16 +251,18 @@ __device__ void solve_one(const BatchItem &it, double *__restrict__ gA, double *
             const double x = xs[h][i], y = ys[h][i];
             const double xx = __dmul_rn(fma(y, t[h].r1, x), t[h].m1);
             const double yy = __dmul_rn(fma(x, t[h].r2, y), t[h].m2);
-            const double e1 = fma(__dsub_rn(x, xx), __dadd_rn(x, xx), d[h]);
-            const double e2 = fma(__dsub_rn(y, yy), __dadd_rn(y, yy), e1);
-            d[h] = (i != pp[h] && i != qq[h]) ? e2 : d[h];
+            const double s1 = __dsub_rn(x, xx), a1 = __dadd_rn(x, xx), s2 = __dsub_rn(y, yy), a2 = __dadd_rn(y, yy);
+            if (i != pp[h] && i != qq[h]) {
+              d[h] = fma(s1, a1, d[h]);
+              d[h] = fma(s2, a2, d[h]);
+            }
           }
         }
       }
       else {
 #pragma unroll
         for (int h = 0; h < 2; ++h)
-          if (sc[h]) scan_pair(xs[h], ys[h], n, pp[h], qq[h], t[h], d[h]);
+          if (sc[h]) scan_rows_real(xs[h], ys[h], n, 0, pp[h], qq[h], t[h], d[h]);
       }
 #pragma unroll
       for (int h = 0; h < 2; ++h) {

@@ -94,13 +94,14 @@ __device__ __forceinline__ bool kbetter(unsigned long long k1, unsigned t1, unsi
 // entries app, aqp, apq, aqq and J(p) = jp, J(q) = -jp.  Returns true when the pair
 // needs the column scan of ABODNDF2 (then d holds its two leading terms and t the
 // coefficients of Z2); otherwise w is the weight (NaN: no transformation).
+template <bool FULL = false>
 __device__ __forceinline__ bool hyp_setup(double app, double aqp, double apq, double aqq, int jp, double &w, double &d, Rot &t)
 {
   w = nan_w();
   if (!may_transform(app, aqp, apq, aqq)) return false;
   double A2[4] = { app, aqp, apq, aqq }, U2[4], Z2[4];
   int info = 0;
-  dhsvd2(A2, jp, -jp, U2, Z2, JK_TH1FIX, info);
+  dhsvd2<FULL>(A2, jp, -jp, U2, Z2, JK_TH1FIX, info);
   if (info < 0) return false;
   if (!(info & 1)) { w = 0.0; return false; }
   if (!(info & 4)) { w = dasum2(aqp, apq); return false; }
@@ -121,7 +122,7 @@ __device__ __forceinline__ bool hyp_setup_z(double app, double aqp, double apq, 
   if (!may_transform(app, aqp, apq, aqq)) return false;
   double A2[4] = { app, aqp, apq, aqq }, U2[4];
   int info = 0;
-  dhsvd2(A2, jp, -jp, U2, Z2, JK_TH1FIX, info);
+  dhsvd2<false>(A2, jp, -jp, U2, Z2, JK_TH1FIX, info);
   if (info < 0) return false;
   if (!(info & 1)) { w = 0.0; return false; }
   if (!(info & 4)) { w = dasum2(aqp, apq); return false; }
@@ -153,7 +154,7 @@ __device__ __forceinline__ bool zhyp_setup_z(double2 app, double2 aqp, double2 a
   if (!may_transform(app, aqp, apq, aqq)) return false;
   double2 A2[4] = { app, aqp, apq, aqq }, U2[4];
   int info = 0;
-  zhsvd2(A2, jp, -jp, U2, Z2, JK_TH1FIX, info);
+  zhsvd2<false>(A2, jp, -jp, U2, Z2, JK_TH1FIX, info);
   if (info < 0) return false;
   if (!(info & 1)) { w = 0.0; return false; }
   if (!(info & 4)) { w = dasum4(aqp.x, aqp.y, apq.x, apq.y); return false; }

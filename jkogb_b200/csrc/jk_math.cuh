@@ -532,7 +532,9 @@ struct NearK {
 // KHSVD2, src/shared/ktransf.F90:15-217, on a nonnegative triangle scaled by 2^s.  An upper one
 // [a, b; 0, c] takes T (equal signs) or U, a lower one [c, 0; b, a] (unequal signs) L.  One straight line:
 // ok is cleared for KHSVD2's argument errors, for INFO -10 and -11 and for operands that the
-// straight-line forms do not take (a vanishing denominator, a new diagonal below 2^-1000).
+// straight-line forms do not take (a vanishing denominator, a new diagonal below 2^-1000).  Without FULL,
+// the new diagonal is left out.
+template <bool FULL>
 __device__ __forceinline__ void khsvd2_near(const double A[4], const bool tg, int s, double th1, int &info, NearK &k, bool &ok)
 {
   const bool upper = (A[M21] == 0.0);
@@ -559,17 +561,19 @@ __device__ __forceinline__ void khsvd2_near(const double A[4], const bool tg, in
   info += cut ? 8 : 0;
   const double cz = root(fma(tg ? tz : -tz, tz, 1.0));
   const double yu = recip(cu), yz = recip(cz);
-  const double w = quot(tg ? cz : cu, tg ? cu : cz, tg ? yu : yz);
-  const double m = __dmul_rn(tg ? as : cs, w), dv = quot(tg ? cs : as, w, recip(w));
-  // the original multiplies or divides and scales with one rounding; so does this while the results
-  // are normal
-  const int em = bexp(m), ed = bexp(dv);
-  ok = ok && (cut || ((m == 0.0 || (em >= 123 && em + 600 - s >= 23)) && (dv == 0.0 || (ed >= 123 && ed + 600 - s >= 23))));
-  const double f1 = pow2(600 - s), m1 = __dmul_rn(m, f1), dv1 = __dmul_rn(dv, f1);
-  // T: G = (a w, c / w); U: (a / w, c w); L (a = A22, c = A11): (c w, a / w)
-  const bool mf = tg || !upper;
-  k.g0 = mf ? m1 : dv1;
-  k.g1 = mf ? dv1 : m1;
+  if constexpr (FULL) {
+    const double w = quot(tg ? cz : cu, tg ? cu : cz, tg ? yu : yz);
+    const double m = __dmul_rn(tg ? as : cs, w), dv = quot(tg ? cs : as, w, recip(w));
+    // the original multiplies or divides and scales with one rounding; so does this while the results
+    // are normal
+    const int em = bexp(m), ed = bexp(dv);
+    ok = ok && (cut || ((m == 0.0 || (em >= 123 && em + 600 - s >= 23)) && (dv == 0.0 || (ed >= 123 && ed + 600 - s >= 23))));
+    const double f1 = pow2(600 - s), m1 = __dmul_rn(m, f1), dv1 = __dmul_rn(dv, f1);
+    // T: G = (a w, c / w); U: (a / w, c w); L (a = A22, c = A11): (c w, a / w)
+    const bool mf = tg || !upper;
+    k.g0 = mf ? m1 : dv1;
+    k.g1 = mf ? dv1 : m1;
+  }
   k.tu = tu; k.tz = tz; k.c12 = tg ? -tz : tz; k.cu = cu; k.cz = cz; k.yu = yu; k.yz = yz;
 }
 
@@ -612,7 +616,10 @@ __device__ __forceinline__ double cneg(bool c, double a) { return c ? -a : a; }
 // square root and magnitude and with selects for the swaps and sign changes.  Off-diagonal entries
 // shrink to zero through the whole exponent range before a loop ends (in a quarter of all blocks of a
 // solve they are below 2^-200 of the diagonal); the forms hold down to about 2^-1000 of it.
-// Returns false, with nothing written, when the block does not allow it.
+// Returns false, with nothing written, when the block does not allow it.  Without FULL (the weights:
+// Z, INFO's bits 0, 2, 3 and, where bit 3 is set, the remaining off-diagonal entries) U and the new
+// diagonal are left out.
+template <bool FULL>
 __device__ __forceinline__ bool dhsvd2_near(double Ain[4], const int J0, const int J1, double Uo[4], double Zo[4], double th1, int &info_o)
 {
   const int hi = max(max(bexp(Ain[0]), bexp(Ain[1])), max(bexp(Ain[2]), bexp(Ain[3])));
@@ -641,12 +648,14 @@ __device__ __forceinline__ bool dhsvd2_near(double Ain[4], const int J0, const i
   {
     const double t = quot_scaled(A[M21], A[M11], recip(down600(A[M11])), ok);
     const double q = root(fma(t, t, 1.0)), y = recip(q);
-    double V[4] = { U[0], U[1], U[2], U[3] };
-    c2a_near(t, q, y, V, ok);
+    if constexpr (FULL) {
+      double V[4] = { U[0], U[1], U[2], U[3] };
+      c2a_near(t, q, y, V, ok);
+#pragma unroll
+      for (int k = 0; k < 4; ++k) U[k] = d ? U[k] : V[k];
+    }
     double v[2] = { fma(t, A[M22], A[M12]), fma(-t, A[M12], A[M22]) };  // C1A
     quots<2>(v, q, y, ok);
-#pragma unroll
-    for (int k = 0; k < 4; ++k) U[k] = d ? U[k] : V[k];
     A[M12] = d ? A[M12] : v[0];
     A[M22] = d ? A[M22] : v[1];
   }
@@ -671,10 +680,12 @@ __device__ __forceinline__ bool dhsvd2_near(double Ain[4], const int J0, const i
   if (d) { A[M11] = scale(A[M11], -s); A[M22] = scale(A[M22], -s); }
   else {
     NearK k;
-    khsvd2_near(A, tg, s, th1, info, k, ok);
-    c2a_near(k.tu, k.cu, k.yu, U, ok);
+    khsvd2_near<FULL>(A, tg, s, th1, info, k, ok);
+    if constexpr (FULL) c2a_near(k.tu, k.cu, k.yu, U, ok);
     a2c_near(Z, k.tz, k.c12, k.cz, k.yz, ok);
-    if (!(info & 8)) { A[M11] = k.g0; A[M22] = k.g1; }
+    if (!(info & 8)) {
+      if constexpr (FULL) { A[M11] = k.g0; A[M22] = k.g1; }
+    }
     else {
 #pragma unroll
       for (int i = 0; i < 4; ++i) A[i] = scale(A[i], -s);
@@ -690,10 +701,11 @@ __device__ __forceinline__ bool dhsvd2_near(double Ain[4], const int J0, const i
   return true;
 }
 
-// DHSVD2, src/D/dtransf.F90:614-683
+// DHSVD2, src/D/dtransf.F90:614-683; without FULL what dhsvd2_near leaves out is undefined
+template <bool FULL = true>
 __device__ __forceinline__ void dhsvd2(double A[4], const int J0, const int J1, double U[4], double Z[4], double th1, int &info)
 {
-  if (!dhsvd2_near(A, J0, J1, U, Z, th1, info)) {
+  if (!dhsvd2_near<FULL>(A, J0, J1, U, Z, th1, info)) {
     // copies, so that the caller's arrays stay in registers beside the call
     double a[4] = { A[0], A[1], A[2], A[3] }, u[4] = { 0.0, 0.0, 0.0, 0.0 }, z[4] = { 0.0, 0.0, 0.0, 0.0 };
     int inf = 0;

@@ -341,7 +341,7 @@ __device__ __forceinline__ GPair gram_pair(const double *__restrict__ A, int n, 
   double A2[4] = { app, aqp, apq, aqq }, U2[4], Z2[4];
   int info = 0;
   const int jp = a_is_p ? 1 : -1;
-  dhsvd2(A2, jp, -jp, U2, Z2, JK_TH1FIX, info);
+  dhsvd2<false>(A2, jp, -jp, U2, Z2, JK_TH1FIX, info);
   if (info < 0) return r;
   if (!(info & 1)) { r.w = 0.0; return r; }
   if (!(info & 4)) { r.w = dasum2(aqp, apq); return r; }
@@ -388,7 +388,7 @@ __device__ __forceinline__ GPair gram_pair(const double2 *__restrict__ A, int n,
   double2 A2[4] = { app, aqp, apq, aqq }, U2[4], Z2[4];
   int info = 0;
   const int jp = a_is_p ? 1 : -1;
-  zhsvd2(A2, jp, -jp, U2, Z2, JK_TH1FIX, info);
+  zhsvd2<false>(A2, jp, -jp, U2, Z2, JK_TH1FIX, info);
   if (info < 0) return r;
   if (!(info & 1)) { r.w = 0.0; return r; }
   if (!(info & 4)) { r.w = dasum4(aqp.x, aqp.y, apq.x, apq.y); return r; }

@@ -282,7 +282,8 @@ __device__ __forceinline__ double2 zcmul(bool c, double2 a, double2 v) { return 
 
 // ZHSVD2 for a block without a zero column whose largest part lies in 2^(+-300): the operations
 // of zhsvd2_any in the same order, as dhsvd2_near.  Returns false, with nothing written, when the
-// block does not allow it.
+// block does not allow it.  Without FULL, U and the new diagonal are left out.
+template <bool FULL>
 __device__ __forceinline__ bool zhsvd2_near(double2 Ain[4], const int J0, const int J1, double2 Uo[4], double2 Zo[4], double th1, int &info_o)
 {
   int hi = 0;
@@ -324,12 +325,14 @@ __device__ __forceinline__ bool zhsvd2_near(double2 Ain[4], const int J0, const 
     ok = ok && (d || A[M11].x > 0.0);
     const double t = quot_scaled(A[M21].x, A[M11].x, recip(down600(A[M11].x)), ok);
     const double q = root(fma(t, t, 1.0)), y = recip(q);
-    double2 V[4] = { U[0], U[1], U[2], U[3] };
-    zc2a_near(t, q, y, V, ok);
+    if constexpr (FULL) {
+      double2 V[4] = { U[0], U[1], U[2], U[3] };
+      zc2a_near(t, q, y, V, ok);
+#pragma unroll
+      for (int k = 0; k < 4; ++k) U[k] = zsel(d, U[k], V[k]);
+    }
     double2 v[2] = { zdfma(t, A[M22], A[M12]), zdfma(-t, A[M12], A[M22]) };  // C1A
     zquots<2>(v, q, y, ok);
-#pragma unroll
-    for (int k = 0; k < 4; ++k) U[k] = zsel(d, U[k], V[k]);
     A[M12] = zsel(d, A[M12], v[0]);
     A[M22] = zsel(d, A[M22], v[1]);
   }
@@ -363,11 +366,11 @@ __device__ __forceinline__ bool zhsvd2_near(double2 Ain[4], const int J0, const 
   else {
     const double W[4] = { A[M11].x, A[M21].x, A[M12].x, A[M22].x };
     NearK k;
-    khsvd2_near(W, tg, sc, th1, info, k, ok);
-    zc2a_near(k.tu, k.cu, k.yu, U, ok);
+    khsvd2_near<FULL>(W, tg, sc, th1, info, k, ok);
+    if constexpr (FULL) zc2a_near(k.tu, k.cu, k.yu, U, ok);
     za2c_near(Z, k.tz, k.c12, k.cz, k.yz, ok);
-    w11 = k.g0;
-    w22 = k.g1;
+    w11 = FULL ? k.g0 : 0.0;
+    w22 = FULL ? k.g1 : 0.0;
     if (info & 8) {
 #pragma unroll
       for (int i = 0; i < 4; ++i) A[i] = zc(scale(A[i].x, -sc), scale(A[i].y, -sc));
@@ -384,10 +387,11 @@ __device__ __forceinline__ bool zhsvd2_near(double2 Ain[4], const int J0, const 
   return true;
 }
 
-// ZHSVD2, src/Z/ztransf.F90:925-1009
+// ZHSVD2, src/Z/ztransf.F90:925-1009; without FULL what zhsvd2_near leaves out is undefined
+template <bool FULL = true>
 __device__ __forceinline__ void zhsvd2(double2 A[4], const int J0, const int J1, double2 U[4], double2 Z[4], double th1, int &info)
 {
-  if (!zhsvd2_near(A, J0, J1, U, Z, th1, info)) {
+  if (!zhsvd2_near<FULL>(A, J0, J1, U, Z, th1, info)) {
     double2 a[4] = { A[0], A[1], A[2], A[3] }, u[4] = {}, z[4] = {};
     int inf = 0;
     zhsvd2_any(a, J0, J1, u, z, th1, inf);
