@@ -314,6 +314,10 @@ int solver_make(jk_solver *v, int cplx, int n, const int *J, int n_2, int id_ncp
     CK(g.alloc(&f.list, ((size_t)f.cap + 1) * sizeof(int)));
     CK(g.alloc(&f.dirty, n * sizeof(int)));
     CK(g.alloc(&f.cls, n * sizeof(int)));
+    CK(g.alloc(&f.mate, n * sizeof(int)));
+    CK(g.alloc(&f.mlo, n * sizeof(double)));
+    CK(g.alloc(&f.mtie, n * sizeof(unsigned)));
+    f.n_minus = w.n_minus;
     CK(g.alloc(&w.gram, ((size_t)(cplx ? 2 : 1) * npm + 1) * sizeof(double)));
     CK(g.alloc(&w.cn, (size_t)n * sizeof(double)));
     std::vector<int> cls(n);
@@ -345,8 +349,8 @@ int solver_make(jk_solver *v, int cplx, int n, const int *J, int n_2, int id_ncp
 long long step_launches(const Workspace &w)
 {
   const bool hyp = (w.n_plus > 0 && w.n_minus > 0);
-  // norms, Gram, weights; the off-norm (learned) or the exact weights and a second ranking (filtered)
-  const int learned = w.learned ? (hyp ? 4 : 1) : w.filter ? 5 : 0;
+  // norms, Gram, weights; the off-norm (learned) or two rankings, matchings and checks and the exact weights (filtered)
+  const int learned = w.learned ? (hyp ? 4 : 1) : w.filter ? 10 : 0;
   return kStepLaunches - (hyp ? 0 : 1) + ((w.cplx && hyp) ? 1 : 0) + learned;
 }
 

@@ -4,6 +4,7 @@
 // 2x2 part of the hyperbolic pair weight.
 #pragma once
 
+#include "jk_internal.h"
 #include "jk_math.cuh"
 #include "jk_zmath.cuh"
 
@@ -83,6 +84,28 @@ __device__ __forceinline__ unsigned tkey(int u, int v)
 {
   const int p = (u < v) ? u : v, b = (u < v) ? (v - u) : (u - v);
   return ((unsigned)b << 16) | (unsigned)p;
+}
+
+// the interval of pair (u, v)'s filtered weight w (jk_filter.cu); exact: whether it is w itself
+__device__ __forceinline__ void weight_interval(const FilterDev &f, int u, int v, double w, double &lo, double &hi, bool &exact, int &k)
+{
+  const int cu = f.cls[u], cv = f.cls[v];
+  lo = hi = w;
+  exact = true;
+  k = -1;
+  if ((cu < 0) == (cv < 0)) return;
+  k = ((cu < 0) ? cv : cu) * f.n_minus + ~((cu < 0) ? cu : cv);
+  const short c = f.code[k];
+  if (c == kBoundExact) return;
+  exact = false;
+  if (c == kBoundNone) {
+    hi = __longlong_as_double(0x7FF0000000000000LL);
+    lo = -hi;
+    return;
+  }
+  const double r = (c >= -1022) ? pow2(c) : __longlong_as_double(1LL << (c + 1074));
+  lo = __dsub_rd(w, r);
+  hi = __dadd_ru(w, r);
 }
 
 __device__ __forceinline__ bool kbetter(unsigned long long k1, unsigned t1, unsigned long long k2, unsigned t2)

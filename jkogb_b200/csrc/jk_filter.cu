@@ -6,10 +6,13 @@
 // step uses the weights only to rank every vertex's partners.  So they are filtered, as
 // geometric predicates are: every scanned pair gets its weight from the Gram products of the columns
 // (k_gram, FP64 tensor pipe; the formula of the scored ranking) with a bound on how far the sequential
-// sum can lie from it, every vertex's partners are ranked by it, and only the pairs whose interval
-// meets a neighbour's in some list are summed exactly and their lists ranked again.  The lists, and
-// with them the pivots, are those of the exact weights.  Where too many pairs are ambiguous (weights
-// at the level of their own rounding) the full scan runs, and for the next kDirectSteps steps at once.
+// sum can lie from it, and the step's greedy matching is built from these weights.  A matching is
+// the greedy one of the exact weights if and only if every pair outside it is worse than the matched
+// pair of one of its two vertices; k_verify checks that with the intervals.  The pairs for which it is not
+// certain, and the matched pairs that they meet, are then summed exactly, their vertices' lists
+// ranked and the matching built again, and checked again.  What still fails, or leaves more pairs than
+// the list holds, takes the full scan, and so do the next steps (1, 2, 4, ... up to kDirectSteps, doubled with
+// each failure in a row).
 //
 // The bound.  Let u = 2^-53, x, y the columns without rows p, q, (z11, z21), (z12, z22) the right
 // transformation's columns, S = |x|^2 + |y|^2 <= cn[p] + cn[q], zm = max(z11^2 + z12^2, z21^2 + z22^2),
@@ -32,8 +35,7 @@
 // formed from parts: 1.1 u ((150 zm + 60) S + k S (7 n + 64) + (2 n + 16) |d|).  Bounds are kept as
 // powers of two (two bytes a pair), at least 2^-1000 (complex) or 2^-1056 (real: 4 n roundings
 // below the normal numbers), which covers underflow; a pair whose numbers leave [0, 1e300] is summed
-// exactly.  On the graded inputs a bound is about 1e-12 of its weight, and no pair of a step's million is
-// ambiguous in the first fifth of a solve.
+// exactly.  On the graded inputs a bound is about 1e-12 of its weight.
 #include "jk_internal.h"
 #include "jk_device.cuh"
 #include "jk_scan.cuh"
@@ -129,6 +131,58 @@ k_hyp_filter(State *st, const T *__restrict__ A, const int *__restrict__ plus, c
   if ((threadIdx.x & 31) == 0 && k < npm) f.claim[k >> 5] = m;
 }
 
+// Round 1: the pairs outside the matching of which it is not certain that the matched pair of one of their
+// vertices is better, and those matched pairs, go to the list of pairs to be summed (a claim bit each),
+// their vertices are marked to be ranked again.  Round 2, after that: any such pair fails the step.
+// A block per vertex: its pairs with the later vertices of its own class, and, for a "+" vertex, those with all "-"
+// vertices.
+__global__ void __launch_bounds__(256)
+k_verify(State *st, const double *__restrict__ Wm, int n, FilterDev f, int round)
+{
+  if (st->stop || st->halt || !st->filter) return;
+  if (round == 2 && (st->namb == 0 || st->namb > f.cap)) return;
+  const int v = blockIdx.x, cv = f.cls[v];
+  const double ml = f.mlo[v];
+  const unsigned mt = f.mtie[v];
+  const double *row = Wm + (long long)v * n;
+  for (int u = threadIdx.x; u < n; u += 256) {
+    const bool same = (f.cls[u] < 0) == (cv < 0);
+    if (u == v || (same ? u < v : cv < 0)) continue;
+    const double w = row[u];
+    double lo, hi;
+    bool exact;
+    int k;
+    weight_interval(f, u, v, w, lo, hi, exact, k);
+    if (exact && w != w) continue;  // no record
+    const double mu = f.mlo[u];
+    const unsigned ut = f.mtie[u];
+    if (ml > hi || mu > hi) continue;
+    const unsigned t = tkey(u, v);
+    // equal exact weights: the tie decides (and the pair itself may be the matched one)
+    if (exact && ((mt && ml == w && mt >= t) || (ut && mu == w && ut >= t))) continue;
+    if (f.mate[v] == u) continue;
+    if (round == 2) { st->bad = 1; continue; }
+    auto claim = [&](int a, int b, int kk) {
+      f.dirty[a] = 1;
+      f.dirty[b] = 1;
+      if (!((atomicOr(&f.claim[kk >> 5], 1u << (kk & 31)) >> (kk & 31)) & 1u)) {
+        const int x = atomicAdd(&st->namb, 1);
+        if (x < f.cap) f.list[x] = kk;
+      }
+    };
+    if (!exact) claim(u, v, k);
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int a = h ? u : v, b = f.mate[a];
+      if (b < 0) continue;
+      const int ca = f.cls[a], cb = f.cls[b];
+      if ((ca < 0) == (cb < 0)) continue;
+      const int kk = ((ca < 0) ? cb : ca) * f.n_minus + ~((ca < 0) ? ca : cb);
+      if (f.code[kk] != kBoundExact) claim(a, b, kk);
+    }
+  }
+}
+
 // one row's terms of the sequential sum: d = fma(s1, a1, d), d = fma(s2, a2, d)
 struct Terms { double s1, a1, s2, a2; };
 
@@ -161,7 +215,7 @@ __global__ void __launch_bounds__(256)
 k_exact_pairs(const State *st, const T *__restrict__ A, const int *__restrict__ plus, const int *__restrict__ minus,
               int n_minus, int n, double *__restrict__ Wm, FilterDev f)
 {
-  if (st->stop || st->halt || !st->filter || st->namb > f.cap) return;
+  if (st->stop || st->halt || !st->filter || st->namb == 0 || st->namb > f.cap) return;
   __shared__ Terms sh[8][2][32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, cnt = st->namb;
   for (int i = blockIdx.x * 8 + warp; i < cnt; i += gridDim.x * 8) {
@@ -196,6 +250,7 @@ k_exact_pairs(const State *st, const T *__restrict__ A, const int *__restrict__ 
       if (w < -JK_HUGE) w = nan_w();
       Wm[(long long)q * n + p] = w;
       Wm[(long long)p * n + q] = w;
+      f.code[k] = kBoundExact;
     }
   }
 }
@@ -216,6 +271,12 @@ cudaError_t filter_t(Workspace &w, const T *A, cudaStream_t s)
 cudaError_t launch_filter(Workspace &w, const void *A, cudaStream_t s)
 {
   return w.cplx ? filter_t(w, (const double2 *)A, s) : filter_t(w, (const double *)A, s);
+}
+
+cudaError_t launch_verify(Workspace &w, int round, cudaStream_t s)
+{
+  k_verify<<<w.n, 256, 0, s>>>(w.st, w.Wm, w.n, w.fd, round);
+  return cudaGetLastError();
 }
 
 cudaError_t launch_exact(Workspace &w, const void *A, cudaStream_t s)

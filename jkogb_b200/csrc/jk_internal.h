@@ -39,7 +39,9 @@ struct State {
   // the filtered exact ranking (jk_filter.cu)
   int filter;        // this step ranks by the filter (0: the full scan)
   int namb;          // pairs of this step that have to be summed exactly
-  int direct;        // steps left that take the full scan at once
+  int bad;           // the filtered matching could not be verified: the step takes the full scan
+  int np;            // matched pairs of the filtered selection
+  int direct, fails; // steps left that take the full scan at once; such failures in a row
 };
 
 // Per-step trace on the device (optional).
@@ -85,13 +87,17 @@ struct ScorerDev {
 // the filter's buffers; a pair's bound is 2^code
 constexpr short kBoundExact = -32768, kBoundNone = 32767;
 constexpr long long kHypTileMin = 512LL * 148 * 2;  // real hyperbolic pairs from which the scan takes its large tiles
-constexpr int kDirectSteps = 64;  // full scans after a step with too many ambiguous pairs
+constexpr int kDirectSteps = 64;  // most full scans in a row before the filter is tried again
 struct FilterDev {
   short *code;       // n_plus x n_minus bounds
   unsigned *claim;   // a bit per pair that is in the list
   int *list;         // the pairs to be summed exactly
   int *dirty;        // per vertex: its list has to be ranked again
   int *cls;          // per vertex: its index in its sign class (+), or the complement of it (-)
+  int *mate;         // per vertex: its partner in the filtered matching (-1: none)
+  double *mlo;       // per vertex: the lower end of its matched pair's weight (-infinity: not matched)
+  unsigned *mtie;    // per vertex: its matched pair's tie key where the weight is exact, else 0
+  int n_minus;
   int cap;           // capacity of the list; with more pairs the step takes the full scan
 };
 
@@ -172,6 +178,7 @@ cudaError_t launch_learned_weights(Workspace &w, const void *A, cudaStream_t s);
 cudaError_t launch_gram(Workspace &w, const void *A, cudaStream_t s);  // column norms, Gram products
 // the filtered exact ranking (jk_filter.cu)
 cudaError_t launch_filter(Workspace &w, const void *A, cudaStream_t s);
+cudaError_t launch_verify(Workspace &w, int round, cudaStream_t s);
 cudaError_t launch_exact(Workspace &w, const void *A, cudaStream_t s);
 cudaError_t prepare_gram();
 constexpr int kOffBlocks = 296;  // fixed grid of the off-norm reduction (a fixed summation order)

@@ -147,10 +147,10 @@ __global__ void k_jztj(T *Z, const int *J, int n)
 }
 
 // Whether a step leaves out the column scans: at the loop's end, in a learned step (the scorer
-// ranks the pairs) and in a filtered one without more than cap ambiguous pairs.
+// ranks the pairs) and in a filtered one whose matching is verified.
 __device__ __forceinline__ bool scan_off(const State *st, int cap)
 {
-  return st->stop || st->halt || st->learned_step || (st->filter && st->namb <= cap);
+  return st->stop || st->halt || st->learned_step || (st->filter && st->namb <= cap && !st->bad);
 }
 
 // ---------------------------------------------------------------------------
@@ -1018,104 +1018,22 @@ __device__ __forceinline__ void block_sort_desc(unsigned long long (&k)[E], unsi
   }
 }
 
-// The pairs of a list (sk, sorted by the filtered weights) whose order is not certain.  Position i is
-// cut from i + 1 where every interval up to i lies above every one from i + 1 on; an
-// approximate weight without a cut on either side is ambiguous.  (Exact weights among
-// themselves are in order.)
+// mode 0: all lists.  Filtered steps: 1 the lists of the filtered weights, 2 those again whose
+// vertices had pairs summed, 3 all lists after a full scan.
 template <int E>
-__device__ __forceinline__ void mark_ambiguous(State *st, const double *col, int v, int cnt, unsigned long long *sk, unsigned short *slo,
-                                               const FilterDev &f, int n_minus)
-{
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  __shared__ double s_lo[SORT_THREADS / 32], s_hi[SORT_THREADS / 32];
-  const double inf = __longlong_as_double(0x7FF0000000000000LL);
-  const int cv = f.cls[v];
-  double lo[E], hi[E];
-  int pair[E];
-#pragma unroll
-  for (int e = 0; e < E; ++e) {
-    const int i = tid * E + e;
-    lo[e] = inf;
-    hi[e] = -inf;
-    pair[e] = -1;
-    if (i < cnt) {
-      const int u = ckey_u(sk[i], v), cu = f.cls[u];
-      const double w = col[u];
-      lo[e] = hi[e] = w;
-      if ((cv < 0) != (cu < 0)) {
-        const int k = ((cv < 0) ? cu : cv) * n_minus + ~((cv < 0) ? cv : cu);
-        const short c = f.code[k];
-        // (a pair without a bound is summed anyway, and its lists are ranked again)
-        if (c != kBoundExact && c != kBoundNone) {
-          const double r = (c >= -1022) ? pow2(c) : __longlong_as_double(1LL << (c + 1074));
-          pair[e] = k;
-          lo[e] = __dsub_rd(w, r);
-          hi[e] = __dadd_ru(w, r);
-        }
-      }
-    }
-  }
-  __syncthreads();
-  // the least lower end up to each position, the greatest upper end from each position on
-#pragma unroll
-  for (int e = 1; e < E; ++e) lo[e] = fmin(lo[e], lo[e - 1]);
-#pragma unroll
-  for (int e = E - 2; e >= 0; --e) hi[e] = fmax(hi[e], hi[e + 1]);
-  double a = lo[E - 1], b = hi[0];
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const double x = __shfl_up_sync(0xFFFFFFFFu, a, o), y = __shfl_down_sync(0xFFFFFFFFu, b, o);
-    if (lane >= o) a = fmin(a, x);
-    if (lane + o < 32) b = fmax(b, y);
-  }
-  if (lane == 31) s_lo[warp] = a;
-  if (lane == 0) s_hi[warp] = b;
-  const double al = __shfl_up_sync(0xFFFFFFFFu, a, 1), bl = __shfl_down_sync(0xFFFFFFFFu, b, 1);
-  __syncthreads();
-  double pl = lane > 0 ? al : inf, sh = lane < 31 ? bl : -inf;
-#pragma unroll
-  for (int k = 0; k < SORT_THREADS / 32; ++k) {
-    if (k < warp) pl = fmin(pl, s_lo[k]);
-    if (k > warp) sh = fmax(sh, s_hi[k]);
-  }
-  double *S = (double *)sk;
-#pragma unroll
-  for (int e = 0; e < E; ++e) S[tid * E + e] = fmax(hi[e], sh);
-  __syncthreads();
-#pragma unroll
-  for (int e = 0; e < E; ++e) {
-    const int i = tid * E + e;
-    slo[i] = (i >= cnt - 1 || fmin(lo[e], pl) > S[i + 1]) ? 1 : 0;  // cut after i
-  }
-  __syncthreads();
-#pragma unroll
-  for (int e = 0; e < E; ++e) {
-    const int i = tid * E + e;
-    if (pair[e] >= 0 && !(slo[i] && (i == 0 || slo[i - 1]))) {
-      f.dirty[v] = 1;
-      if (!((atomicOr(&f.claim[pair[e] >> 5], 1u << (pair[e] & 31)) >> (pair[e] & 31)) & 1u)) {
-        const int x = atomicAdd(&st->namb, 1);
-        if (x < f.cap) f.list[x] = pair[e];
-      }
-    }
-  }
-}
-
-// MODE 0: the lists of the exact weights.  MODE 1: the lists of the filtered weights; the pairs
-// whose interval meets that of a neighbour go to the list of pairs to be summed exactly, and the
-// vertex is marked to be ranked again.  MODE 2: those vertices again, or all after a full scan.
-template <int E, int MODE>
 __global__ void __launch_bounds__(SORT_THREADS)
-k_colsort(State *st, const double *__restrict__ Wm, int n, unsigned short *list, int *len, FilterDev f, int n_minus)
+k_colsort(const State *st, const double *__restrict__ Wm, int n, unsigned short *list, int *len, FilterDev f, int mode)
 {
   if (st->stop || st->halt) return;
-  if (MODE == 1 && !st->filter) return;
-  if (MODE == 2) {
+  if (mode == 1 && !st->filter) return;
+  if (mode == 2) {
+    if (!st->filter || st->namb == 0) return;
     const int d = f.dirty[blockIdx.x];
-    if (st->filter && st->namb <= f.cap && !d) return;
     __syncthreads();
     if (threadIdx.x == 0 && d) f.dirty[blockIdx.x] = 0;
+    if (st->namb > f.cap || !d) return;
   }
+  if (mode == 3 && st->filter && st->namb <= f.cap && !st->bad) return;
   __shared__ unsigned long long sk[SORT_THREADS * E];
   __shared__ unsigned short slo[SORT_THREADS * E];  // low 16 bits of the sorted keys' weight keys
   __shared__ int s_cnt, s_warp[SORT_THREADS / 32];
@@ -1199,7 +1117,6 @@ k_colsort(State *st, const double *__restrict__ Wm, int n, unsigned short *list,
   for (int r = tid; r < cnt; r += blockDim.x) {
     lv[r] = (unsigned short)ckey_u(sk[r], v);
   }
-  if constexpr (MODE == 1) mark_ambiguous<E>(st, col, v, cnt, sk, slo, f, n_minus);
   // the last group of 8 is read whole
   if (tid < 8 && cnt + tid < ((cnt + 7) & ~7)) lv[cnt + tid] = 0;
   if (tid == 0) len[v] = cnt;
@@ -1360,11 +1277,52 @@ struct SelLayout {
   }
 };
 
+// the end of a selection, by one block: the columns outside the pivots (those without a bit in
+// `taken`), the step's scalars, how the next step ranks, the loop test
+template <typename T>
+__device__ void select_end(State *st, const int *J, int n, int sl, int rounds, const unsigned *taken, const Piv<T> *piv, int *unp,
+                           int *s_nunp, Trace &tr, int early, const FilterDev &f, int mode)
+{
+  const int tid = threadIdx.x;
+  for (int v = tid; v < n; v += blockDim.x)
+    if (!((taken[v >> 5] >> (v & 31)) & 1u)) unp[atomicAdd(s_nunp, 1)] = v;
+  __syncthreads();
+  if (tid == 0) {
+    st->sl = sl;
+    st->nunp = *s_nunp;
+    st->rounds = rounds;
+    if (mode == 3) {
+      if (!st->filter) { if (--st->direct <= 0) st->filter = 1; }
+      else if (st->namb > f.cap || st->bad) {
+        st->direct = min(1 << min(st->fails, 16), kDirectSteps);
+        st->fails += 1;
+        st->filter = 0;
+      }
+      else st->fails = 0;
+      st->namb = 0;
+      st->bad = 0;
+    }
+    if (sl <= 0) {
+      // DSTEP_EXEC returns with SL = 0: the loop ends with INFO = S (src/D/dstep.F90:421, 575-582)
+      st->info = st->steps;
+      st->stop = 1;
+      if (st->trace_on && st->trace_steps < st->trace_cap_steps) {
+        const int s = st->trace_steps++;
+        tr.sl[s] = 0; tr.nl[s] = -1; tr.tw[s] = -0.0; tr.trig[s] = 0; tr.hyp[s] = 0; tr.rounds[s] = rounds;
+      }
+    }
+    else {
+      st->pending = 1;
+      if (early) end_of_step<T>(st, piv, J, tr, &st->halt);
+    }
+  }
+}
+
 template <typename T>
 __global__ void __launch_bounds__(kSelThreads, 1)
 k_select(State *st, const double *__restrict__ Wm, const int *__restrict__ J, int n, int n_2,
          const unsigned short *__restrict__ list, const int *__restrict__ len, const T *__restrict__ A, Piv<T> *piv,
-         RowRot<T> *rr, int *unp, Trace tr, int quirk, int early, int cap)
+         RowRot<T> *rr, int *unp, Trace tr, int quirk, int early, FilterDev f, int mode)
 {
   cg::cluster_group cluster = cg::this_cluster();
   const int C = (int)cluster.num_blocks(), c = (int)cluster.block_rank();
@@ -1390,7 +1348,32 @@ k_select(State *st, const double *__restrict__ Wm, const int *__restrict__ J, in
   }
   if (*(volatile int *)&st->stop) return;
   if (*(volatile int *)&st->halt) {
-    if (c == 0 && tid == 0) st->stop = st->halt;
+    if (c == 0 && tid == 0 && (mode == 0 || mode == 3)) st->stop = st->halt;
+    return;
+  }
+  // mode 0: the step's selection.  Filtered steps: 1 the matching of the filtered weights, 2 again with
+  // the pairs that were summed, 3 the pivots of the verified matching, or the whole selection after a full scan
+  const bool full = mode == 0 || (mode == 3 && (!st->filter || st->namb > f.cap || st->bad));
+  if (mode == 1 && !st->filter) return;
+  if (mode == 2 && (!st->filter || st->namb == 0 || st->namb > f.cap)) return;
+  if (mode == 3 && !full) {
+    // (nl and err were set to zero when the matching was built)
+    const int np = st->np;
+    for (int r = (warp * C + c) * 32 + lane; r < np; r += kSelThreads * C)
+      pivot_hsvd<T>(st, A, J, n, piv[r].p, piv[r].q, piv[r], rr[r], quirk);
+    if (c == 0) {
+      for (int k = tid; k < (n + 31) / 32; k += kSelThreads) taken[k] = 0u;
+      if (tid == 0) s_nunp = 0;
+      __syncthreads();
+      for (int r = tid; r < np; r += kSelThreads) {
+        atomicOr(&taken[piv[r].p >> 5], 1u << (piv[r].p & 31));
+        atomicOr(&taken[piv[r].q >> 5], 1u << (piv[r].q & 31));
+      }
+    }
+    __threadfence();
+    sync();
+    if (c != 0) return;
+    select_end<T>(st, J, n, np, st->rounds, taken, piv, unp, &s_nunp, tr, early, f, mode);
     return;
   }
   if (tid == 0) { s_cnt = 0; s_nunp = 0; s_got[0] = 0; s_got[1] = 0; }
@@ -1562,6 +1545,36 @@ k_select(State *st, const double *__restrict__ Wm, const int *__restrict__ J, in
     for (int b = 0; b < C; ++b) r += min(s_all[b], i + (b < c ? 1 : 0));
     return r;
   };
+  if (mode == 1 || mode == 2) {
+    // the matching, and what k_verify needs of it per vertex
+    for (int i = tid; i < cnt; i += kSelThreads) {
+      const int r = place(i), p = pairs[i].x, q = pairs[i].y;
+      piv[r].p = p;
+      piv[r].q = q;
+      double lo, hi;
+      bool exact;
+      int k;
+      weight_interval(f, p, q, Wm[(long long)p * n + q], lo, hi, exact, k);
+      f.mate[p] = q;
+      f.mate[q] = p;
+      f.mlo[p] = f.mlo[q] = lo;
+      f.mtie[p] = f.mtie[q] = exact ? tkey(p, q) : 0u;
+    }
+    if (c == 0) {
+      for (int v = tid; v < n; v += kSelThreads)
+        if (!((taken[v >> 5] >> (v & 31)) & 1u)) {
+          f.mate[v] = -1;
+          f.mlo[v] = -__longlong_as_double(0x7FF0000000000000LL);
+          f.mtie[v] = 0u;
+        }
+      if (tid == 0) {
+        st->np = np;
+        st->rounds = rounds;
+      }
+    }
+    sync();  // (the counts of other blocks have been read)
+    return;
+  }
   const int sl = (np < n_2) ? np : n_2;
   const bool ranked = (np > n_2) || st->trace_on || !A;
   if (ranked) {
@@ -1613,35 +1626,7 @@ k_select(State *st, const double *__restrict__ Wm, const int *__restrict__ J, in
     __threadfence();
     sync();  // every pivot is counted
   }
-  if (c != 0) return;
-  // the columns outside the pivots
-  for (int v = tid; v < n; v += kSelThreads)
-    if (!((taken[v >> 5] >> (v & 31)) & 1u)) unp[atomicAdd(&s_nunp, 1)] = v;
-  __syncthreads();
-  if (tid == 0) {
-    st->sl = sl;
-    st->nunp = s_nunp;
-    st->rounds = rounds;
-    if (cap >= 0) {
-      // how the next step ranks
-      if (!st->filter) { if (--st->direct <= 0) st->filter = 1; }
-      else if (st->namb > cap) { st->filter = 0; st->direct = kDirectSteps; }
-      st->namb = 0;
-    }
-    if (sl <= 0) {
-      // DSTEP_EXEC returns with SL = 0: the loop ends with INFO = S (src/D/dstep.F90:421, 575-582)
-      st->info = st->steps;
-      st->stop = 1;
-      if (st->trace_on && st->trace_steps < st->trace_cap_steps) {
-        const int s = st->trace_steps++;
-        tr.sl[s] = 0; tr.nl[s] = -1; tr.tw[s] = -0.0; tr.trig[s] = 0; tr.hyp[s] = 0; tr.rounds[s] = rounds;
-      }
-    }
-    else {
-      st->pending = 1;
-      if (early) end_of_step<T>(st, piv, J, tr, &st->halt);
-    }
-  }
+  if (c == 0) select_end<T>(st, J, n, sl, rounds, taken, piv, unp, &s_nunp, tr, early, f, mode);
 }
 
 // ---------------------------------------------------------------------------
@@ -2089,19 +2074,39 @@ cudaError_t launch_weights(Workspace &w, const void *A, cudaStream_t s)
   return w.cplx ? weights_t(w, (const double2 *)A, s) : weights_t(w, (const double *)A, s);
 }
 
-template <int MODE>
-static cudaError_t colsort(Workspace &w, cudaStream_t s)
+static cudaError_t colsort(Workspace &w, int mode, cudaStream_t s)
 {
   const int n = w.n;
   switch (colsort_e(n)) {
-  case 1: k_colsort<1, MODE><<<n, SORT_THREADS, 0, s>>>(w.st, w.Wm, n, w.list, w.len, w.fd, w.n_minus); break;
-  case 2: k_colsort<2, MODE><<<n, SORT_THREADS, 0, s>>>(w.st, w.Wm, n, w.list, w.len, w.fd, w.n_minus); break;
-  case 4: k_colsort<4, MODE><<<n, SORT_THREADS, 0, s>>>(w.st, w.Wm, n, w.list, w.len, w.fd, w.n_minus); break;
-  case 8: k_colsort<8, MODE><<<n, SORT_THREADS, 0, s>>>(w.st, w.Wm, n, w.list, w.len, w.fd, w.n_minus); break;
-  case 16: k_colsort<16, MODE><<<n, SORT_THREADS, 0, s>>>(w.st, w.Wm, n, w.list, w.len, w.fd, w.n_minus); break;
+  case 1: k_colsort<1><<<n, SORT_THREADS, 0, s>>>(w.st, w.Wm, n, w.list, w.len, w.fd, mode); break;
+  case 2: k_colsort<2><<<n, SORT_THREADS, 0, s>>>(w.st, w.Wm, n, w.list, w.len, w.fd, mode); break;
+  case 4: k_colsort<4><<<n, SORT_THREADS, 0, s>>>(w.st, w.Wm, n, w.list, w.len, w.fd, mode); break;
+  case 8: k_colsort<8><<<n, SORT_THREADS, 0, s>>>(w.st, w.Wm, n, w.list, w.len, w.fd, mode); break;
+  case 16: k_colsort<16><<<n, SORT_THREADS, 0, s>>>(w.st, w.Wm, n, w.list, w.len, w.fd, mode); break;
   default: return cudaErrorInvalidValue;
   }
   return cudaGetLastError();
+}
+
+template <typename T>
+static cudaError_t match_t(Workspace &w, const T *A, int n_2, int mode, cudaStream_t s)
+{
+  const int n = w.n;
+  const int C = select_cluster(n);
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = (unsigned)C;
+  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  cfg.gridDim = dim3((unsigned)C);
+  cfg.blockDim = dim3(kSelThreads);
+  cfg.dynamicSmemBytes = SelLayout(n, C).total;
+  cfg.stream = s;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, k_select<T>, w.st, (const double *)w.Wm, (const int *)w.J, n, n_2,
+                         (const unsigned short *)w.list, (const int *)w.len, A, (Piv<T> *)w.piv, (RowRot<T> *)w.rowrot,
+                         w.unp, w.tr, w.zba_quirk, w.learned ? 0 : 1, w.fd, mode);
 }
 
 template <typename T>
@@ -2124,24 +2129,8 @@ static cudaError_t select_t(Workspace &w, const T *A, int n_2, cudaStream_t s)
     }
   }
   else {
-    e = w.filter ? colsort<2>(w, s) : colsort<0>(w, s);
-    if (e != cudaSuccess) return e;
-    const int C = select_cluster(n);
-    cudaLaunchConfig_t cfg = {};
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = (unsigned)C;
-    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
-    cfg.gridDim = dim3((unsigned)C);
-    cfg.blockDim = dim3(kSelThreads);
-    cfg.dynamicSmemBytes = SelLayout(n, C).total;
-    cfg.stream = s;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    e = cudaLaunchKernelEx(&cfg, k_select<T>, w.st, (const double *)w.Wm, (const int *)w.J, n, n_2,
-                           (const unsigned short *)w.list, (const int *)w.len, A, (Piv<T> *)w.piv, (RowRot<T> *)w.rowrot,
-                           w.unp, w.tr, w.zba_quirk, w.learned ? 0 : 1, w.filter ? w.fd.cap : -1);
-    if (e != cudaSuccess) return e;
+    if ((e = colsort(w, w.filter ? 3 : 0, s)) != cudaSuccess) return e;
+    if ((e = match_t<T>(w, A, n_2, w.filter ? 3 : 0, s)) != cudaSuccess) return e;
   }
   return cudaGetLastError();
 }
@@ -2159,10 +2148,14 @@ static cudaError_t step_t(Workspace &w, T *A, T *U, T *Z, int n_2, cudaStream_t 
   if (e != cudaSuccess) return e;
   const bool hyp = w.n_plus > 0 && w.n_minus > 0;
   if (w.filter && hyp) {
-    // the filtered weights, the lists, the exact weights of what is ambiguous in them
+    // the filtered weights and their matching; what it leaves uncertain summed, and the matching again
     if ((e = launch_filter(w, A, s)) != cudaSuccess) return e;
-    if ((e = colsort<1>(w, s)) != cudaSuccess) return e;
-    if ((e = launch_exact(w, A, s)) != cudaSuccess) return e;
+    for (int round = 1; round <= 2; ++round) {
+      if ((e = colsort(w, round, s)) != cudaSuccess) return e;
+      if ((e = match_t<T>(w, (const T *)A, n_2, round, s)) != cudaSuccess) return e;
+      if ((e = launch_verify(w, round, s)) != cudaSuccess) return e;
+      if (round == 1 && (e = launch_exact(w, A, s)) != cudaSuccess) return e;
+    }
   }
   if ((e = weights_t(w, (const T *)A, s)) != cudaSuccess) return e;
   // a learned solve: the scorer ranks the scanned hyperbolic pairs (the exact scan kernels
