@@ -911,7 +911,6 @@ k_weights_hyp(const State *st, const double *__restrict__ A, const int *__restri
 // in registers, shuffles and shared memory), so a round only moves each free
 // vertex's list pointer past partners matched meanwhile (k_select, one block).
 // ---------------------------------------------------------------------------
-#define SORT_THREADS 256
 
 // descending bitonic sort of s2 (a power of two) records (k, t, i) in shared memory
 __device__ __forceinline__ void bitonic_desc(unsigned long long *k, unsigned *t, int *ix, int s2)
@@ -945,13 +944,19 @@ __host__ __device__ __forceinline__ int pow2ceil(int x)
 __host__ __device__ __forceinline__ int list_ld(int n) { return (n + 7) & ~7; }
 
 // rank the partners of vertex v = blockIdx.x: list[v][r] = r-th best partner,
-// len[v] = number of partners.
-// One 64-bit key per partner: the top 48 bits of the weight key, then the 16-bit
-// tie code (band << 1 | (u > v)), which orders the partners of v as (band, p) do
-// and also names u.  Partners whose keys agree in the top 48 bits are re-ordered by
-// the full key afterwards.  E keys per thread in registers (position tid*E + e);
+// len[v] = number of partners.  E keys per thread in registers (position tid*E + e);
 // stages with partner distance < E run in registers, < 32E by warp shuffles, the
 // rest in shared memory.
+// The sort is bound by its comparisons, so above 256 vertices the keys are short: a minimum and a maximum
+// of 32 bits against a compare and four selects of 64 (133 -> 61 us at N = 2048 with 8 keys a thread, 610 -> 302 us
+// at N = 4096, where 512 threads with 8 keys also replace 256 with 16, which left 2 blocks to an SM).
+// Sixty-four bits before, with the threads' keys unpadded in shared memory (a 16- to 32-way bank conflict) and read a
+// column piece per thread: 174 and 1060 us.
+//
+// The 64-bit key: the top 48 bits of the weight key, then the 16-bit
+// tie code (band << 1 | (u > v)), which orders the partners of v as (band, p) do
+// and also names u.  Partners whose keys agree in the top 48 bits are re-ordered by
+// the full key afterwards.
 __device__ __forceinline__ unsigned long long ckey(double w, int u, int v)
 {
   const unsigned long long k = wkey(w);
@@ -966,13 +971,18 @@ __device__ __forceinline__ int ckey_u(unsigned long long c, int v)
   return (t & 1) ? v + (t >> 1) : v - (t >> 1);
 }
 
-// descending bitonic sort of the SORT_THREADS * E keys a block holds E per thread
+// where position i of a sort lies in shared memory: a thread's E positions are followed by a free one (8-byte
+// keys) or two (16-bit values), so that the warp's threads, E positions apart, meet different banks
+template <int E> __device__ __forceinline__ int pad8(int i) { return i + i / E; }
+template <int E> __device__ __forceinline__ int pad2(int i) { return i + 2 * (i / E); }
+
+// descending bitonic sort of the NT * E keys a block holds E per thread
 // (position tid * E + e): stages with partner distance < E in registers, < 32 E by warp
-// shuffles, the rest through shared memory (sk, SORT_THREADS * E entries)
-template <int E>
+// shuffles, the rest through shared memory (sk, NT * (E + 1) entries)
+template <int E, int NT>
 __device__ __forceinline__ void block_sort_desc(unsigned long long (&k)[E], unsigned long long *sk)
 {
-  const int tid = threadIdx.x, s2 = SORT_THREADS * E;
+  const int tid = threadIdx.x, s2 = NT * E;
   for (int kk = 2; kk <= s2; kk <<= 1) {
     for (int j = kk >> 1; j >= E; j >>= 1) {
       if (j < 32 * E) {
@@ -990,12 +1000,12 @@ __device__ __forceinline__ void block_sort_desc(unsigned long long (&k)[E], unsi
       else {
         __syncthreads();
 #pragma unroll
-        for (int e = 0; e < E; ++e) sk[tid * E + e] = k[e];
+        for (int e = 0; e < E; ++e) sk[pad8<E>(tid * E + e)] = k[e];
         __syncthreads();
 #pragma unroll
         for (int e = 0; e < E; ++e) {
           const int i = tid * E + e, l = i ^ j;
-          const unsigned long long ok = sk[l];
+          const unsigned long long ok = sk[pad8<E>(l)];
           const bool desc = ((i & kk) == 0), lower = (i < l);
           const unsigned long long hi = (ok > k[e]) ? ok : k[e], lo = (ok > k[e]) ? k[e] : ok;
           k[e] = (desc == lower) ? hi : lo;
@@ -1018,64 +1028,54 @@ __device__ __forceinline__ void block_sort_desc(unsigned long long (&k)[E], unsi
   }
 }
 
-// mode 0: all lists.  Filtered steps: 1 the lists of the filtered weights, 2 those again whose
-// vertices had pairs summed, 3 all lists after a full scan.
-template <int E>
-__global__ void __launch_bounds__(SORT_THREADS)
-k_colsort(const State *st, const double *__restrict__ Wm, int n, unsigned short *list, int *len, FilterDev f, int mode)
+// the ranked partners of vertex v by their 64-bit keys, into sk (s_cnt partners, in shared memory)
+template <int E, int NT>
+__device__ __forceinline__ void rank_by_key(const double *__restrict__ col, int n, int v, const int &s_cnt, unsigned long long *sk,
+                                            unsigned short *slo, int *s_warp)
 {
-  if (st->stop || st->halt) return;
-  if (mode == 1 && !st->filter) return;
-  if (mode == 2) {
-    if (!st->filter || st->namb == 0) return;
-    const int d = f.dirty[blockIdx.x];
-    __syncthreads();
-    if (threadIdx.x == 0 && d) f.dirty[blockIdx.x] = 0;
-    if (st->namb > f.cap || !d) return;
-  }
-  if (mode == 3 && st->filter && st->namb <= f.cap && !st->bad) return;
-  __shared__ unsigned long long sk[SORT_THREADS * E];
-  __shared__ unsigned short slo[SORT_THREADS * E];  // low 16 bits of the sorted keys' weight keys
-  __shared__ int s_cnt, s_warp[SORT_THREADS / 32];
-  const int v = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const double *col = Wm + (long long)v * n;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   unsigned long long k[E];
-  int valid = 0;
 #pragma unroll
   for (int e = 0; e < E; ++e) {
-    const int i = tid * E + e;
+    const int i = e * NT + tid;  // (in any order)
     k[e] = (i < n && i != v) ? ckey(col[i], i, v) : 0ULL;
-    valid += k[e] ? 1 : 0;
   }
-  if (tid == 0) s_cnt = 0;
-  __syncthreads();
-  atomicAdd(&s_cnt, valid);
-  block_sort_desc<E>(k, sk);
+  block_sort_desc<E, NT>(k, sk);
   __syncthreads();
   const int cnt = s_cnt;
   // The sort saw the top 48 bits of each weight key: keys that agree there but differ in
-  // the low 16 bits are in tie-code order and must be reordered by the full key.  The low
-  // bits of every sorted key show whether any run of equal top bits needs it (near
+  // the low 16 bits are in tie-code order and must be reordered by the full key.  Where there are
+  // such runs of equal top bits, the low bits of every sorted key show whether any of them needs it (near
   // convergence many weights are exactly equal, zeros above all: such runs are already in
   // the record order).
+#pragma unroll
+  for (int e = 0; e < E; ++e) sk[pad8<E>(tid * E + e)] = k[e];
+  __syncthreads();
+  int bad = 0, starts = 0, runs = 0;
+  bool start[E];
   unsigned lo[E];
 #pragma unroll
   for (int e = 0; e < E; ++e) {
     const int i = tid * E + e;
-    sk[i] = k[e];
-    lo[e] = (i < cnt) ? (unsigned)(wkey(col[ckey_u(k[e], v)]) & 0xFFFFu) : 0u;
-    slo[i] = (unsigned short)lo[e];
-  }
-  __syncthreads();
-  int bad = 0, starts = 0;
-  bool start[E];
-#pragma unroll
-  for (int e = 0; e < E; ++e) {
-    const int i = tid * E + e;
-    const bool same = (i > 0) && (i < cnt) && ((sk[i - 1] >> 16) == (k[e] >> 16));
+    const unsigned long long before = (e > 0) ? k[e - 1] : (tid > 0) ? sk[pad8<E>(i - 1)] : 0ULL;
+    const bool same = (i > 0) && (i < cnt) && ((before >> 16) == (k[e] >> 16));
     start[e] = (i < cnt) && !same;
     starts += start[e] ? 1 : 0;
-    if (same && slo[i - 1] != (unsigned short)lo[e]) bad = 1;
+    runs |= same ? 1 : 0;
+  }
+  if (__syncthreads_or(runs)) {
+#pragma unroll
+    for (int e = 0; e < E; ++e) {
+      const int i = tid * E + e;
+      lo[e] = (i < cnt) ? (unsigned)(wkey(col[ckey_u(k[e], v)]) & 0xFFFFu) : 0u;
+      slo[pad2<E>(i)] = (unsigned short)lo[e];
+    }
+    __syncthreads();
+#pragma unroll
+    for (int e = 0; e < E; ++e) {
+      const int i = tid * E + e;
+      if (i > 0 && i < cnt && !start[e] && slo[pad2<E>(i - 1)] != (unsigned short)lo[e]) bad = 1;
+    }
   }
   if (__syncthreads_or(bad)) {
     // order every run by (low bits, tie code): a second sort on (run index, low 16 bits,
@@ -1089,13 +1089,13 @@ k_colsort(const State *st, const double *__restrict__ Wm, int n, unsigned short 
     if (lane == 31) s_warp[warp] = c;
     __syncthreads();
     if (warp == 0) {
-      int x = (lane < SORT_THREADS / 32) ? s_warp[lane] : 0;
+      int x = (lane < NT / 32) ? s_warp[lane] : 0;
 #pragma unroll
       for (int o = 1; o < 32; o <<= 1) {
         const int t = __shfl_up_sync(0xFFFFFFFFu, x, o);
         if (lane >= o) x += t;
       }
-      if (lane < SORT_THREADS / 32) s_warp[lane] = x;
+      if (lane < NT / 32) s_warp[lane] = x;
     }
     __syncthreads();
     int run = c - starts + (warp > 0 ? s_warp[warp - 1] : 0) - 1;  // the run before my first key
@@ -1107,16 +1107,265 @@ k_colsort(const State *st, const double *__restrict__ Wm, int n, unsigned short 
                           (k[e] & 0xFFFFull))
                        : 0ULL;
     }
-    block_sort_desc<E>(k, sk);  // the low 16 bits (the tie code, which names the partner) are kept
+    block_sort_desc<E, NT>(k, sk);  // the low 16 bits (the tie code, which names the partner) are kept
     __syncthreads();
 #pragma unroll
-    for (int e = 0; e < E; ++e) sk[tid * E + e] = k[e];
+    for (int e = 0; e < E; ++e) sk[pad8<E>(tid * E + e)] = k[e];
     __syncthreads();
   }
-  unsigned short *lv = list + (long long)v * list_ld(n);
-  for (int r = tid; r < cnt; r += blockDim.x) {
-    lv[r] = (unsigned short)ckey_u(sk[r], v);
+}
+
+// A short key of each partner: its weight in the first bits, its tie code in the last log2(E NT).
+// The weight is taken by a monotone map to a fixed-point number over the list's own range: the bits of |w| above those
+// of the least |w| that is not zero, negative weights mirrored.  Partners that share those bits form a group,
+// which is put in order by the full weights afterwards; a group of more than kGroup members with different weights
+// leaves the list to the 64-bit sort.
+constexpr int kGroup = 32;
+
+__host__ __device__ constexpr int tie_bits(int keys) { return keys > 1 ? 1 + tie_bits(keys / 2) : 0; }
+
+// the partners of v in the order (band, u > v), counted without gaps, and back
+__device__ __forceinline__ unsigned tie_code(int u, int v, int m)
+{
+  const int b = (u < v) ? v - u : u - v;
+  return (unsigned)((b <= m) ? 2 * (b - 1) + (u > v ? 1 : 0) : m + b - 1);
+}
+
+__device__ __forceinline__ int tie_partner(unsigned c, int v, int n, int m)
+{
+  if ((int)c < 2 * m) return (c & 1) ? v + (int)(c >> 1) + 1 : v - (int)(c >> 1) - 1;
+  const int b = (int)c - m + 1;
+  return (v < n - 1 - v) ? v + b : v - b;
+}
+
+// descending bitonic sort of 32-bit keys, as block_sort_desc; the keys of an ascending run are held complemented,
+// so that every exchange of a thread's own keys is a minimum and a maximum
+template <int E, int NT>
+__device__ __forceinline__ void block_sort_desc32(unsigned (&k)[E], unsigned *sk)
+{
+  const int tid = threadIdx.x, s2 = NT * E;
+#pragma unroll
+  for (int kk = 2; kk <= E; kk <<= 1)
+#pragma unroll
+    for (int j = kk >> 1; j > 0; j >>= 1)
+#pragma unroll
+      for (int e = 0; e < E; ++e) {
+        const int f = e ^ j;
+        if (f > e) {
+          const bool desc = (kk < E) ? ((e & kk) == 0) : ((tid & 1) == 0);
+          const unsigned hi = max(k[e], k[f]), lo = min(k[e], k[f]);
+          k[e] = desc ? hi : lo;
+          k[f] = desc ? lo : hi;
+        }
+      }
+  for (int kk = 2 * E; kk <= s2; kk <<= 1) {
+    const unsigned flip = ((tid * E) & kk) ? 0xFFFFFFFFu : 0u;
+#pragma unroll
+    for (int e = 0; e < E; ++e) k[e] ^= flip;
+    for (int j = kk >> 1; j >= 32 * E; j >>= 1) {
+      // (a pair's threads are in the same run)
+      const int m = j / E;
+      __syncthreads();
+#pragma unroll
+      for (int e = 0; e < E; ++e) sk[pad8<E>(tid * E + e)] = k[e];
+      __syncthreads();
+      const bool lower = ((tid & m) == 0);
+#pragma unroll
+      for (int e = 0; e < E; ++e) {
+        const unsigned o = sk[pad8<E>((tid ^ m) * E + e)];
+        k[e] = lower ? max(k[e], o) : min(k[e], o);
+      }
+    }
+    for (int m = min(kk / (2 * E), 16); m > 0; m >>= 1) {
+      const bool lower = ((tid & m) == 0);
+#pragma unroll
+      for (int e = 0; e < E; ++e) {
+        const unsigned o = __shfl_xor_sync(0xFFFFFFFFu, k[e], m);
+        k[e] = lower ? max(k[e], o) : min(k[e], o);
+      }
+    }
+#pragma unroll
+    for (int j = E / 2; j > 0; j >>= 1)
+#pragma unroll
+      for (int e = 0; e < E; ++e) {
+        const int f = e ^ j;
+        if (f > e) {
+          const unsigned hi = max(k[e], k[f]), lo = min(k[e], k[f]);
+          k[e] = hi;
+          k[f] = lo;
+        }
+      }
+#pragma unroll
+    for (int e = 0; e < E; ++e) k[e] ^= flip;
   }
+}
+
+// The list of vertex v by short keys; false: a group was too long.  s32: the sorted keys, NT (E + 1);
+// slot: as many bytes, the positions of the members of groups; flag: NT E bytes.
+template <int E, int NT>
+__device__ __forceinline__ bool rank_by_short_key(const double (&w)[E], const double *__restrict__ col, int n, int v, int cnt, unsigned low,
+                                                  unsigned top, bool negs, unsigned *s32, unsigned short *slot, unsigned char *flag,
+                                                  int *s_m, unsigned short *lv)
+{
+  constexpr int TB = tie_bits(E * NT), QB = 32 - TB;
+  const int tid = threadIdx.x, m = min(v, n - 1 - v);
+  const unsigned long long F = (unsigned long long)low << 32, R = (unsigned long long)(top - low + 1) << 32, C = negs ? R : 0ULL;
+  const unsigned long long most = (negs ? 2 * R : R) - 1;
+  int sh = 64 - __clzll((long long)most) - QB;
+  sh = max(sh, 0);
+  if ((most >> sh) >= (1ULL << QB) - 1) ++sh;
+  unsigned k[E];
+#pragma unroll
+  for (int e = 0; e < E; ++e) {
+    const int i = e * NT + tid;
+    k[e] = 0u;
+    if (w[e] == w[e]) {
+      const unsigned long long b = (unsigned long long)__double_as_longlong(w[e]), a = b & 0x7FFFFFFFFFFFFFFFULL;
+      const unsigned long long t = a ? a - F : 0ULL, y = (b >> 63) ? C - t : C + t;
+      k[e] = (((unsigned)(y >> sh) + 1u) << TB) | tie_code(i, v, m);
+    }
+  }
+  block_sort_desc32<E, NT>(k, s32);
+  __syncthreads();
+#pragma unroll
+  for (int e = 0; e < E; ++e) s32[pad8<E>(tid * E + e)] = k[e];
+  __syncthreads();
+  auto same = [&](unsigned x, unsigned y) { return (x >> TB) == (y >> TB); };
+  auto partner = [&](unsigned key) { return tie_partner(key & ((1u << TB) - 1), v, n, m); };
+  auto weight = [&](unsigned key) { return wkey(col[partner(key)]); };
+  // (no partner's key is 0)
+  const unsigned before = tid ? s32[pad8<E>(tid * E - 1)] : 0u, after = (tid < NT - 1) ? s32[pad8<E>(tid * E + E)] : 0u;
+#pragma unroll
+  for (int e = 0; e < E; ++e) {
+    const unsigned kb = e ? k[e - 1] : before, ka = (e < E - 1) ? k[e + 1] : after;
+    if (k[e] && (same(kb, k[e]) || same(ka, k[e]))) slot[atomicAdd(s_m, 1)] = (unsigned short)(tid * E + e);
+  }
+  __syncthreads();
+  const int members = *s_m;
+  // where a member's weight differs from the one before
+  int differ = 0;
+  for (int x = tid; x < members; x += NT) {
+    const int i = slot[x];
+    const unsigned key = s32[pad8<E>(i)], kb = i ? s32[pad8<E>(i - 1)] : 0u;
+    const unsigned char d = (same(kb, key) && weight(kb) != weight(key)) ? 1 : 0;
+    flag[i] = d;
+    differ |= d;
+  }
+  differ = __syncthreads_or(differ);
+  // (the limits are the group's ends, or kGroup + 1 positions away)
+  auto ends = [&](int i, unsigned key, int &a, int &b) {
+    a = b = i;
+    while (a > 0 && i - a <= kGroup && same(s32[pad8<E>(a - 1)], key)) --a;
+    while (b + 1 < cnt && b - i <= kGroup && same(s32[pad8<E>(b + 1)], key)) ++b;
+  };
+  if (differ) {
+    int bad = 0;
+    for (int x = tid; x < members; x += NT) {
+      const int i = slot[x];
+      if (flag[i]) {
+        int a, b;
+        ends(i, s32[pad8<E>(i)], a, b);
+        if (b - a + 1 > kGroup) bad = 1;
+      }
+    }
+    if (__syncthreads_or(bad)) return false;
+  }
+  for (int r = tid; r < cnt; r += NT) lv[r] = (unsigned short)partner(s32[pad8<E>(r)]);
+  if (differ) {
+    __syncthreads();
+    // a member's place: its group's first and those that go before it
+    for (int x = tid; x < members; x += NT) {
+      const int i = slot[x];
+      const unsigned key = s32[pad8<E>(i)];
+      int a, b, any = 0;
+      ends(i, key, a, b);
+      if (b - a + 1 <= kGroup)
+        for (int j = a + 1; j <= b; ++j) any |= flag[j];
+      if (any) {
+        const unsigned long long me = weight(key);
+        int r = a;
+        for (int j = a; j <= b; ++j)
+          if (j != i) {
+            const unsigned long long o = weight(s32[pad8<E>(j)]);
+            r += (o > me || (o == me && j < i)) ? 1 : 0;
+          }
+        lv[r] = (unsigned short)partner(key);
+      }
+    }
+  }
+  return true;
+}
+
+// mode 0: all lists.  Filtered steps: 1 the lists of the filtered weights, 2 those again whose
+// vertices had pairs summed, 3 all lists after a full scan.
+template <int E, int NT>
+__global__ void __launch_bounds__(NT)
+k_colsort(const State *st, const double *__restrict__ Wm, int n, unsigned short *list, int *len, FilterDev f, int mode)
+{
+  if (st->stop || st->halt) return;
+  if (mode == 1 && !st->filter) return;
+  if (mode == 2) {
+    if (!st->filter || st->namb == 0) return;
+    const int d = f.dirty[blockIdx.x];
+    __syncthreads();
+    if (threadIdx.x == 0 && d) f.dirty[blockIdx.x] = 0;
+    if (st->namb > f.cap || !d) return;
+  }
+  if (mode == 3 && st->filter && st->namb <= f.cap && !st->bad) return;
+  __shared__ unsigned long long sk[NT * (E + 1)];
+  __shared__ unsigned short slo[NT * (E + 2)];  // low 16 bits of the sorted keys' weight keys
+  __shared__ int s_cnt, s_neg, s_m, s_warp[NT / 32];
+  __shared__ unsigned s_low, s_top;
+  // (one launch's blocks all run at once at n <= 256, and the short keys' extra barriers cost 1 us of 4.3)
+  constexpr bool kShort = E * NT > 256;
+  const int v = blockIdx.x, tid = threadIdx.x;
+  const double *col = Wm + (long long)v * n;
+  unsigned short *lv = list + (long long)v * list_ld(n);
+  if (tid == 0) { s_cnt = 0; s_neg = 0; s_m = 0; s_low = 0x7FFFFFFFu; s_top = 0u; }
+  double w[E];
+  int valid = 0, neg_w = 0;
+  unsigned low = 0x7FFFFFFFu, top = 0u;
+#pragma unroll
+  for (int e = 0; e < E; ++e) {
+    const int i = e * NT + tid;  // (in any order)
+    w[e] = (i < n && i != v) ? col[i] : nan_w();
+  }
+#pragma unroll
+  for (int e = 0; e < E; ++e)
+    if (w[e] == w[e]) {
+      ++valid;
+      if (kShort && w[e] != 0.0) {
+        const unsigned h = (unsigned)__double2hiint(fabs(w[e]));
+        low = min(low, h);
+        top = max(top, h);
+        neg_w |= (w[e] < 0.0) ? 1 : 0;
+      }
+    }
+  valid = __reduce_add_sync(0xFFFFFFFFu, valid);
+  if constexpr (kShort) {
+    low = __reduce_min_sync(0xFFFFFFFFu, low);
+    top = __reduce_max_sync(0xFFFFFFFFu, top);
+    neg_w = __any_sync(0xFFFFFFFFu, neg_w);
+  }
+  __syncthreads();
+  if ((tid & 31) == 0) {
+    atomicAdd(&s_cnt, valid);
+    if (kShort && valid) { atomicMin(&s_low, low); atomicMax(&s_top, top); }
+    if (neg_w) s_neg = 1;
+  }
+  bool done = false;
+  if constexpr (kShort) {
+    __syncthreads();
+    unsigned *s32 = (unsigned *)sk;
+    done = rank_by_short_key<E, NT>(w, col, n, v, s_cnt, min(s_low, s_top), s_top, s_neg != 0, s32,
+                                    (unsigned short *)(s32 + NT * (E + 1)), (unsigned char *)slo, &s_m, lv);
+    if (!done) __syncthreads();
+  }
+  if (!done) {
+    rank_by_key<E, NT>(col, n, v, s_cnt, sk, slo, s_warp);
+    for (int r = tid; r < s_cnt; r += NT) lv[r] = (unsigned short)ckey_u(sk[pad8<E>(r)], v);
+  }
+  const int cnt = s_cnt;
   // the last group of 8 is read whole
   if (tid < 8 && cnt + tid < ((cnt + 7) & ~7)) lv[cnt + tid] = 0;
   if (tid == 0) len[v] = cnt;
@@ -1824,12 +2073,13 @@ k_ncp3_pick(State *st, const int *__restrict__ itp, const int *__restrict__ sort
   }
 }
 
-// k_colsort instantiations: records per thread E = pow2ceil(n) / SORT_THREADS
+// k_colsort instantiations: keys per 256 threads (16: 512 threads with 8 each)
 int colsort_e(int n)
 {
   const int s2 = pow2ceil(n);
-  return s2 <= SORT_THREADS ? 1 : s2 / SORT_THREADS;
+  return s2 <= 256 ? 1 : s2 / 256;
 }
+
 // ---------------------------------------------------------------------------
 // the fused transformations of one step (src/D/dstep.F90:301-346).
 // Block b < SL owns pivot b's column pair (p, q); the other blocks own two
@@ -2078,11 +2328,11 @@ static cudaError_t colsort(Workspace &w, int mode, cudaStream_t s)
 {
   const int n = w.n;
   switch (colsort_e(n)) {
-  case 1: k_colsort<1><<<n, SORT_THREADS, 0, s>>>(w.st, w.Wm, n, w.list, w.len, w.fd, mode); break;
-  case 2: k_colsort<2><<<n, SORT_THREADS, 0, s>>>(w.st, w.Wm, n, w.list, w.len, w.fd, mode); break;
-  case 4: k_colsort<4><<<n, SORT_THREADS, 0, s>>>(w.st, w.Wm, n, w.list, w.len, w.fd, mode); break;
-  case 8: k_colsort<8><<<n, SORT_THREADS, 0, s>>>(w.st, w.Wm, n, w.list, w.len, w.fd, mode); break;
-  case 16: k_colsort<16><<<n, SORT_THREADS, 0, s>>>(w.st, w.Wm, n, w.list, w.len, w.fd, mode); break;
+  case 1: k_colsort<1, 256><<<n, 256, 0, s>>>(w.st, w.Wm, n, w.list, w.len, w.fd, mode); break;
+  case 2: k_colsort<2, 256><<<n, 256, 0, s>>>(w.st, w.Wm, n, w.list, w.len, w.fd, mode); break;
+  case 4: k_colsort<4, 256><<<n, 256, 0, s>>>(w.st, w.Wm, n, w.list, w.len, w.fd, mode); break;
+  case 8: k_colsort<8, 256><<<n, 256, 0, s>>>(w.st, w.Wm, n, w.list, w.len, w.fd, mode); break;
+  case 16: k_colsort<8, 512><<<n, 512, 0, s>>>(w.st, w.Wm, n, w.list, w.len, w.fd, mode); break;
   default: return cudaErrorInvalidValue;
   }
   return cudaGetLastError();
