@@ -263,15 +263,14 @@ struct jk_solver {
 
 namespace {
 
-// Where the filter pays: it adds the Gram products, a bound per pair and five launches to a step (60 us
-// at the smallest orders) and takes the column scans away.  Measured over the first steps, filter
-// against scan: real N = 512 graded 176 to 173 us a step, 701 258 to 247, 800 (where the scan takes its
-// large tiles) 199 to 302, 2048 graded 0.80 to 2.11 ms, 4096 3.9 to 14.3 ms; complex N = 100 103 to 118 us,
-// 200 128 to 178, 1024 0.37 to 3.18 ms.
+// Where the filter pays: it adds the Gram products, a bound per pair and ten launches to a step (40 us
+// at the smallest orders) and takes the column scans away.  Measured, filter against scan: whole real
+// solves N = 256 256 to 244 ms, 384 452 to 474, 512 725 to 847, 640 1.17 to 1.55 s, complex N = 100 119 to 141 ms, 200
+// 343 to 479; the first steps, complex N = 90, 17.9 to 22.1 ms for 200, real 256 33.8 to 32.4 and 384 34.8 to 36.2 for 300.
 bool filter_pays(int cplx, int n, int np, int nm)
 {
   const long long nh = (long long)np * nm;
-  return cplx ? nh * n >= 250000 : nh >= kHypTileMin;
+  return cplx ? nh * n >= 100000 : nh >= 32768;
 }
 
 int solver_make(jk_solver *v, int cplx, int n, const int *J, int n_2, int id_ncp, const jk_opts *opts,

@@ -86,7 +86,6 @@ struct ScorerDev {
 
 // the filter's buffers; a pair's bound is 2^code
 constexpr short kBoundExact = -32768, kBoundNone = 32767;
-constexpr long long kHypTileMin = 512LL * 148 * 2;  // real hyperbolic pairs from which the scan takes its large tiles
 constexpr int kDirectSteps = 64;  // most full scans in a row before the filter is tried again
 struct FilterDev {
   short *code;       // n_plus x n_minus bounds

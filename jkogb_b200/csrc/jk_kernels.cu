@@ -2288,6 +2288,8 @@ static cudaError_t trig_t(Workspace &w, const T *A, cudaStream_t s)
   return cudaGetLastError();
 }
 
+constexpr long long kHypTileMin = 512LL * 148 * 2;  // real hyperbolic pairs from which the scan takes its large tiles
+
 template <typename T>
 static cudaError_t weights_t(Workspace &w, const T *A, cudaStream_t s)
 {

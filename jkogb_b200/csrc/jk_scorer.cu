@@ -185,14 +185,16 @@ k_colnorm(const State *st, const double *__restrict__ A, int n, double *__restri
   }
 }
 
-// G[a][b] = sum_i A0(i, plus[a]) A0(i, minus[b]) with A0 = A minus its diagonal:
-// a 64 x 64 tile per block of 4 warps (32 x 32 each, 4 x 4 DMMA m8n8k4 tiles), row
-// chunks of 32 staged with cp.async in two buffers; the diagonal entries are masked
-// when the fragments are read.
-#define GT 64
+// G[a][b] = sum_i A0(i, plus[a]) A0(i, minus[b]) with A0 = A minus its diagonal, by DMMA m8n8k4: tiles of
+// T x T, row chunks of GK staged with cp.async in two buffers with one barrier each; the diagonal entries are masked
+// when the fragments are read, in the chunks that hold a tile's diagonal entries.
+// Bound by the FP64 tensor pipe (37.1 TFLOP/s of m8n8k4 in a loop of nothing else) and, within a chunk, by the latency
+// between a fragment's load and its product: eight warps of 32 x 16 on a 64 x 64 tile reach 30.3 TFLOP/s at N = 4096
+// (1111 us), four of 32 x 32 reached 27.6 (1221 us).  Smaller orders have too few tiles: four warps of 16 x 16 on
+// 32 x 32 take 40 us at N = 1024 (64 x 64: 61, before 81), complex 107 us (120, 161).
 #define GK 32
 #define GKP 36  // padded chunk row: the 8 x 4 fragment reads hit distinct banks
-constexpr size_t kGramOperand = 2 * GT * GKP * sizeof(double);  // one operand's two buffers
+constexpr size_t gram_smem(int tile) { return (size_t)2 * 2 * tile * GKP * sizeof(double); }
 
 __device__ __forceinline__ void dmma_8x8x4(double (&c)[2], double a, double b)
 {
@@ -201,101 +203,116 @@ __device__ __forceinline__ void dmma_8x8x4(double (&c)[2], double a, double b)
                : "d"(a), "d"(b));
 }
 
-__device__ __forceinline__ void cp_async16g(void *smem, const void *gmem, bool full)
+__device__ __forceinline__ void cp_async16g(void *smem, const void *gmem)
 {
   const unsigned sa = (unsigned)__cvta_generic_to_shared(smem);
-  const int sz = full ? 16 : 0;  // 0: the 16 bytes are zero-filled
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(sa), "l"(gmem), "r"(sz));
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(sa), "l"(gmem));
+}
+
+__device__ __forceinline__ void cp_async8g(void *smem, const void *gmem)
+{
+  const unsigned sa = (unsigned)__cvta_generic_to_shared(smem);
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(sa), "l"(gmem));
 }
 
 // C = 1: real A; C = 2: complex A, read as 2 n interleaved reals per column, so that the
 // real product of two columns is Re(x^H y); IM: the B operand's (re, im) pairs are read as
 // (im, -re), which makes the product Im(x^H y)
-template <int C, bool IM>
+template <int C, bool IM, int T, int WM, int WN>
 __device__ __forceinline__ void gram_tile(const double *__restrict__ A, const int *__restrict__ plus,
                                           const int *__restrict__ minus, int n_plus, int n_minus, int n,
                                           double *__restrict__ G)
 {
+  constexpr int NTH = (T / WM) * (T / WN) * 32, FM = WM / 8, FN = WN / 8;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  double (*xs)[GT][GKP] = (double (*)[GT][GKP])smem_raw;            // [2][GT][GKP]
-  double (*ys)[GT][GKP] = (double (*)[GT][GKP])(smem_raw + kGramOperand);
-  __shared__ int cx[GT], cy[GT];
+  double (*sm)[2 * T][GKP] = (double (*)[2 * T][GKP])smem_raw;  // [2]: the "+" columns, the "-" columns
+  __shared__ int cols[2 * T];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int a0 = blockIdx.x * GT, b0 = blockIdx.y * GT;
+  const int a0 = blockIdx.x * T, b0 = blockIdx.y * T;
   const int nd = C * n;  // reals per column
-  if (tid < GT) {
-    cx[tid] = (a0 + tid < n_plus) ? plus[a0 + tid] : -1;
-    cy[tid] = (b0 + tid < n_minus) ? minus[b0 + tid] : -1;
-  }
+  for (int k = tid; k < 2 * T; k += NTH)
+    cols[k] = (k < T) ? ((a0 + k < n_plus) ? plus[a0 + k] : -1) : ((b0 + k - T < n_minus) ? minus[b0 + k - T] : -1);
   __syncthreads();
   const int nk = (nd + GK - 1) / GK;
-  // staging: 2 operands x 64 columns x 16 pieces of 16 bytes (two reals each) = 2048
-  // copies, 16 per thread; a piece that is not 16-byte aligned in A or runs past the
-  // column's end is loaded by plain loads (zeros past the end)
   auto stage = [&](int c) {
     if (c < nk) {
-      const int k0 = c * GK, buf = c & 1;
+      const int k0 = c * GK, buf = c & 1, piece = tid & 15, r = k0 + 2 * piece;
 #pragma unroll
-      for (int t = 0; t < 16; ++t) {
-        const int idx = tid + 128 * t;        // 0 .. 2047
-        const int op = idx >> 10, col = (idx >> 4) & 63, piece = idx & 15;
-        const int g = op ? cy[col] : cx[col];
-        const int r = k0 + 2 * piece;
-        double *dst = op ? &ys[buf][col][2 * piece] : &xs[buf][col][2 * piece];
+      for (int t = 0; t < (2 * T) * 16 / NTH; ++t) {
+        const int col = (tid >> 4) + t * (NTH / 16), g = cols[col];
+        double *dst = &sm[buf][col][2 * piece];
         const long long e = (long long)g * nd + r;
-        if (g >= 0 && r + 1 < nd && !(e & 1)) cp_async16g(dst, A + e, true);  // 16-byte aligned piece
+        if (g >= 0 && r + 1 < nd) {
+          // (every other column of an odd order starts between two pieces of 16 bytes)
+          if (!((size_t)(A + e) & 15)) cp_async16g(dst, A + e);
+          else {
+            cp_async8g(dst, A + e);
+            cp_async8g(dst + 1, A + e + 1);
+          }
+        }
         else {
           dst[0] = (g >= 0 && r < nd) ? A[e] : 0.0;
-          dst[1] = (g >= 0 && r + 1 < nd) ? A[e + 1] : 0.0;
+          dst[1] = 0.0;
         }
       }
     }
     asm volatile("cp.async.commit_group;\n" ::);
   };
-  double acc[4][4][2];
+  double acc[FM][FN][2];
 #pragma unroll
-  for (int i = 0; i < 4; ++i)
+  for (int i = 0; i < FM; ++i)
 #pragma unroll
-    for (int j = 0; j < 4; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
-  const int wm = (warp & 1) * 32, wn = (warp >> 1) * 32;  // the warp's 32 x 32 sub-tile
-  const int fr = lane >> 2, fk = lane & 3;                   // fragment row / k of this lane
-  int gxa[4], gyb[4];
+    for (int j = 0; j < FN; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
+  const int wm = (warp % (T / WM)) * WM, wn = (warp / (T / WM)) * WN;  // the warp's sub-tile
+  const int fr = lane >> 2, fk = lane & 3;                               // fragment row / k of this lane
+  int gxa[FM], gyb[FN];
 #pragma unroll
-  for (int i = 0; i < 4; ++i) { gxa[i] = cx[wm + 8 * i + fr]; gyb[i] = cy[wn + 8 * i + fr]; }
-  stage(0);
-  for (int c = 0; c < nk; ++c) {
-    stage(c + 1);
-    asm volatile("cp.async.wait_group 1;\n" ::);
-    __syncthreads();
+  for (int i = 0; i < FM; ++i) gxa[i] = cols[wm + 8 * i + fr];
+#pragma unroll
+  for (int i = 0; i < FN; ++i) gyb[i] = cols[T + wn + 8 * i + fr];
+  // the rows of the tile's diagonal entries (the columns are in ascending order)
+  const int alo = cols[0], ahi = plus[min(a0 + T, n_plus) - 1], blo = cols[T], bhi = minus[min(b0 + T, n_minus) - 1];
+  auto chunk = [&](int c, auto masked) {
+    constexpr bool M = decltype(masked)::value;
     const int buf = c & 1, k0 = c * GK;
 #pragma unroll
     for (int kk = 0; kk < GK; kk += 4) {
-      const int kr = kk + fk;             // this lane's real index in the chunk
-      const int row = (k0 + kr) / C;      // the matrix row it belongs to
-      double fa[4], fb[4];
+      const int kr = kk + fk;         // this lane's real index in the chunk
+      const int row = (k0 + kr) / C;  // the matrix row it belongs to
+      double fa[FM], fb[FN];
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        fa[i] = (row == gxa[i]) ? 0.0 : xs[buf][wm + 8 * i + fr][kr];
-        double b;
-        if constexpr (IM) b = (kr & 1) ? -ys[buf][wn + 8 * i + fr][kr - 1] : ys[buf][wn + 8 * i + fr][kr + 1];
-        else b = ys[buf][wn + 8 * i + fr][kr];
-        fb[i] = (row == gyb[i]) ? 0.0 : b;
+      for (int i = 0; i < FM; ++i) {
+        fa[i] = sm[buf][wm + 8 * i + fr][kr];
+        if (M && row == gxa[i]) fa[i] = 0.0;
       }
 #pragma unroll
-      for (int i = 0; i < 4; ++i)
+      for (int i = 0; i < FN; ++i) {
+        if constexpr (IM) fb[i] = (kr & 1) ? -sm[buf][T + wn + 8 * i + fr][kr - 1] : sm[buf][T + wn + 8 * i + fr][kr + 1];
+        else fb[i] = sm[buf][T + wn + 8 * i + fr][kr];
+        if (M && row == gyb[i]) fb[i] = 0.0;
+      }
 #pragma unroll
-        for (int j = 0; j < 4; ++j) dmma_8x8x4(acc[i][j], fa[i], fb[j]);
+      for (int i = 0; i < FM; ++i)
+#pragma unroll
+        for (int j = 0; j < FN; ++j) dmma_8x8x4(acc[i][j], fa[i], fb[j]);
     }
-    __syncthreads();
+  };
+  stage(0);
+  for (int c = 0; c < nk; ++c) {
+    asm volatile("cp.async.wait_group 0;\n" ::);
+    __syncthreads();  // chunk c has landed, chunk c - 1 has been read
+    stage(c + 1);
+    const int r0 = c * GK / C, r1 = (c * GK + GK - 1) / C;
+    if ((r1 >= alo && r0 <= ahi) || (r1 >= blo && r0 <= bhi)) chunk(c, std::true_type());
+    else chunk(c, std::false_type());
   }
-  asm volatile("cp.async.wait_group 0;\n" ::);
   // C fragment: row fr, columns 2 fk, 2 fk + 1 of each 8 x 8 tile
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
+  for (int i = 0; i < FM; ++i) {
     const int a = a0 + wm + 8 * i + fr;
     if (a >= n_plus) continue;
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
+    for (int j = 0; j < FN; ++j) {
       const int b = b0 + wn + 8 * j + 2 * fk;
       if (b < n_minus) G[(long long)a * n_minus + b] = acc[i][j][0];
       if (b + 1 < n_minus) G[(long long)a * n_minus + b + 1] = acc[i][j][1];
@@ -305,17 +322,16 @@ __device__ __forceinline__ void gram_tile(const double *__restrict__ A, const in
 
 // the Gram products of a scored step: G[a][b] (real A); Re and Im of x_a^H y_b (complex A,
 // blockIdx.z 0 and 1, the imaginary parts n_plus n_minus entries after the real ones)
-template <int C>
-__global__ void __launch_bounds__(128)
+template <int C, int T>
+__global__ void __launch_bounds__(T == 64 ? 256 : 128, T == 64 ? 2 : 5)
 k_gram(const State *st, const double *__restrict__ A, const int *__restrict__ plus, const int *__restrict__ minus,
        int n_plus, int n_minus, int n, double *__restrict__ G)
 {
   if (st->stop || st->halt || !(st->learned_step || st->filter)) return;
-  if (C == 2 && blockIdx.z) gram_tile<C, true>(A, plus, minus, n_plus, n_minus, n, G + (long long)n_plus * n_minus);
-  else gram_tile<C, false>(A, plus, minus, n_plus, n_minus, n, G);
+  constexpr int WM = T / 2, WN = (T == 64) ? T / 4 : T / 2;
+  if (C == 2 && blockIdx.z) gram_tile<C, true, T, WM, WN>(A, plus, minus, n_plus, n_minus, n, G + (long long)n_plus * n_minus);
+  else gram_tile<C, false, T, WM, WN>(A, plus, minus, n_plus, n_minus, n, G);
 }
-
-
 
 // ---------------------------------------------------------------------------
 // a pair of a scored step: the exact 2x2 part of DMAGF2H and, for a pair that needs the
@@ -749,20 +765,24 @@ __global__ void k_mlp_pack(const float *__restrict__ P, unsigned short *w, float
 // ---------------------------------------------------------------------------
 // host launchers
 // ---------------------------------------------------------------------------
-// the column norms and the Gram products of a scored or filtered step
+// the column norms and the Gram products of a scored or filtered step.  The large tiles where every SM has one and
+// some have two (N = 4096: 1111 against 1154 us, 2048: 177 against 183; 1024: 61 against 40, complex 120
+// against 107: the small tiles, which are read from L2 twice as often)
 template <int C>
-static cudaError_t gram_t(Workspace &w, const double *A, cudaStream_t s)
+static cudaError_t gram_t(const State *st, const double *A, const int *plus, const int *minus, int n_plus, int n_minus, int n,
+                          double *G, double *cn, cudaStream_t s)
 {
-  const int n = w.n;
-  k_colnorm<C><<<(n + 7) / 8 < 1184 ? (n + 7) / 8 : 1184, 256, 0, s>>>(w.st, A, n, w.cn);
-  dim3 g((w.n_plus + GT - 1) / GT, (w.n_minus + GT - 1) / GT, C);
-  k_gram<C><<<g, 128, 2 * kGramOperand, s>>>(w.st, A, w.plus, w.minus, w.n_plus, w.n_minus, n, w.gram);
+  k_colnorm<C><<<(n + 7) / 8 < 1184 ? (n + 7) / 8 : 1184, 256, 0, s>>>(st, A, n, cn);
+  if ((long long)((n_plus + 63) / 64) * ((n_minus + 63) / 64) * C > 148)
+    k_gram<C, 64><<<dim3((n_plus + 63) / 64, (n_minus + 63) / 64, C), 256, gram_smem(64), s>>>(st, A, plus, minus, n_plus, n_minus, n, G);
+  else
+    k_gram<C, 32><<<dim3((n_plus + 31) / 32, (n_minus + 31) / 32, C), 128, gram_smem(32), s>>>(st, A, plus, minus, n_plus, n_minus, n, G);
   return cudaGetLastError();
 }
 
 cudaError_t launch_gram(Workspace &w, const void *A, cudaStream_t s)
 {
-  return w.cplx ? gram_t<2>(w, (const double *)A, s) : gram_t<1>(w, (const double *)A, s);
+  return (w.cplx ? gram_t<2> : gram_t<1>)(w.st, (const double *)A, w.plus, w.minus, w.n_plus, w.n_minus, w.n, w.gram, w.cn, s);
 }
 
 template <typename T>
@@ -785,9 +805,10 @@ cudaError_t launch_learned_weights(Workspace &w, const void *A, cudaStream_t s)
 
 cudaError_t prepare_gram()
 {
-  const int sm = (int)(2 * kGramOperand);
-  cudaError_t e = cudaFuncSetAttribute(k_gram<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
-  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_gram<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
+  // (a tile of 32 needs no more than any kernel may take)
+  const int sm = (int)gram_smem(64);
+  cudaError_t e = cudaFuncSetAttribute(k_gram<1, 64>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_gram<2, 64>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
   return e;
 }
 
@@ -804,9 +825,8 @@ static cudaError_t features_t(int n, const T *A, const int *plus, const int *min
 {
   constexpr int C = sizeof(T) / sizeof(double);
   const long long cnt = (long long)n_plus * n_minus;
-  k_colnorm<C><<<(n + 7) / 8 < 1184 ? (n + 7) / 8 : 1184, 256, 0, s>>>(st, (const double *)A, n, cn);
-  dim3 g((n_plus + GT - 1) / GT, (n_minus + GT - 1) / GT, C);
-  k_gram<C><<<g, 128, 2 * kGramOperand, s>>>(st, (const double *)A, plus, minus, n_plus, n_minus, n, G);
+  const cudaError_t e = gram_t<C>(st, (const double *)A, plus, minus, n_plus, n_minus, n, G, cn, s);
+  if (e != cudaSuccess) return e;
   k_gram_features<T><<<(unsigned)((cnt + 255) / 256), 256, 0, s>>>(A, plus, minus, n_plus, n_minus, n, G, cn, step, X,
                                                                     Wg);
   return cudaGetLastError();

@@ -41,6 +41,9 @@ def _input(n, n_plus, cplx, form):
     (800, 400, False, "near", 0, 80), (800, 400, False, "tiny", 0, 12), (801, 400, False, "tied", 0, 10),
     (800, 390, False, "huge", 0, 3), (800, 390, False, "small", 0, 4), (800, 400, False, "gauss", 100, 6),
     (110, 55, True, "gauss", 0, 40), (201, 60, True, "graded", 0, 30), (300, 150, True, "near", 0, 70),
+    (364, 182, False, "gauss", 0, 20), (513, 256, False, "graded", 0, 30), (400, 200, False, "near", 0, 80),
+    (401, 200, False, "tied", 0, 10), (86, 40, True, "graded", 0, 30),
+    (1701, 850, False, "gauss", 0, 4), (1201, 600, True, "graded", 0, 3),  # the large Gram tiles, odd columns
     (203, 100, True, "tiny", 0, 12), (200, 100, True, "tied", 0, 10), (150, 70, True, "huge", 0, 3)])
 def test_filter_equals_scan(n, n_plus, cplx, form, n_2, steps):
     import jkogb_b200 as jk
