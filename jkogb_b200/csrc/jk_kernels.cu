@@ -1567,14 +1567,15 @@ __device__ void select_end(State *st, const int *J, int n, int sl, int rounds, c
   }
 }
 
-template <typename T>
+// (SOLO: the cluster is one block)
+template <typename T, bool SOLO>
 __global__ void __launch_bounds__(kSelThreads, 1)
 k_select(State *st, const double *__restrict__ Wm, const int *__restrict__ J, int n, int n_2,
          const unsigned short *__restrict__ list, const int *__restrict__ len, const T *__restrict__ A, Piv<T> *piv,
          RowRot<T> *rr, int *unp, Trace tr, int quirk, int early, FilterDev f, int mode)
 {
   cg::cluster_group cluster = cg::this_cluster();
-  const int C = (int)cluster.num_blocks(), c = (int)cluster.block_rank();
+  const int C = SOLO ? 1 : (int)cluster.num_blocks(), c = SOLO ? 0 : (int)cluster.block_rank();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const SelLayout L(n, C);
   unsigned *cand = (unsigned *)(smem_raw + L.cand);            // [2][n4]: candidate | (round + 1) << 16
@@ -1586,7 +1587,7 @@ k_select(State *st, const double *__restrict__ Wm, const int *__restrict__ J, in
   unsigned *taken = (unsigned *)(smem_raw + L.taken);          // [(n + 31) / 32]: a bit per vertex
   __shared__ int s_cnt, s_nunp, s_got[2], s_all[16];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, ld = list_ld(n);
-  const bool solo = (C == 1);
+  constexpr bool solo = SOLO;
   auto sync = [&]() { if (solo) __syncthreads(); else cluster.sync(); };
 
   // the end of the previous step, unless its own selection saw to it
@@ -2209,7 +2210,8 @@ cudaError_t prepare_kernels(int n)
   if (e == cudaSuccess) e = cudaFuncSetAttribute(k_rotate<double2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 2 * n * 16);
   if (e == cudaSuccess) e = cudaFuncSetAttribute(k_hyp_z_pm, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kZSmem);
   const int ss = (int)SelLayout(n, select_cluster(n)).total;
-  for (const void *f : { (const void *)k_select<double>, (const void *)k_select<double2> }) {
+  for (const void *f : { (const void *)k_select<double, true>, (const void *)k_select<double, false>, (const void *)k_select<double2, true>,
+                           (const void *)k_select<double2, false> }) {
     if (e == cudaSuccess) e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, ss);
     // clusters of 16
     if (e == cudaSuccess) e = cudaFuncSetAttribute(f, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
@@ -2356,7 +2358,7 @@ static cudaError_t match_t(Workspace &w, const T *A, int n_2, int mode, cudaStre
   cfg.stream = s;
   cfg.attrs = at;
   cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, k_select<T>, w.st, (const double *)w.Wm, (const int *)w.J, n, n_2,
+  return cudaLaunchKernelEx(&cfg, C == 1 ? k_select<T, true> : k_select<T, false>, w.st, (const double *)w.Wm, (const int *)w.J, n, n_2,
                          (const unsigned short *)w.list, (const int *)w.len, A, (Piv<T> *)w.piv, (RowRot<T> *)w.rowrot,
                          w.unp, w.tr, w.zba_quirk, w.learned ? 0 : 1, w.fd, mode);
 }
