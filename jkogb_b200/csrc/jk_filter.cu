@@ -101,7 +101,7 @@ __device__ __forceinline__ double filter_pair(const double2 *__restrict__ A, int
 
 // the weights and bounds of all hyperbolic pairs, one thread each ((+, -) order)
 template <typename T>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, sizeof(T) == sizeof(double) ? 3 : 2)
 k_hyp_filter(State *st, const T *__restrict__ A, const int *__restrict__ plus, const int *__restrict__ minus, int n_plus,
              int n_minus, int n, const double *__restrict__ G, const double *__restrict__ cn, double *__restrict__ Wm,
              FilterDev f)

@@ -1,20 +1,22 @@
 // jk_kernels.cu -- the per-step CUDA kernels of the J-Kogbetliantz HSVD (real and
 // complex), B200 (sm_100a).  One step of DSTEP_EXEC / ZSTEP_EXEC
-// (src/D/dstep.F90:376-443, src/Z/zstep.F90:379-447) is seven launches:
+// (src/D/dstep.F90:376-443, src/Z/zstep.F90:379-447) is five launches:
 //
 //   k_weights_trig  pair weights of the trigonometric pairs      (DMAGF2T / ZMAGF2T)
-//   k_weights_hyp   pair weights of the hyperbolic pairs         (DMAGF2H / ZMAGF2H)
+//   k_hyp_pm, k_weights_hyp (real); k_absmat and k_hyp_z_pm, k_weights_hyp_z (complex)
+//                   pair weights of the hyperbolic pairs         (DMAGF2H / ZMAGF2H)
 //                   = batched 2x2 HSVD + the tiled off-norm scan (ABODNDF2 / ABODNZF2)
 //   k_colsort       every vertex's partners ranked by the records' sort order (AW_CMP)
-//   k_select        one block: the end-of-step test of the previous step
-//                   (SL := MIN(SL, NL)); the greedy non-colliding selection of the
-//                   sorted records (AW_SRT* + AW_NCP1/2) as the greedy matching, in
-//                   rounds of mutual best proposals; the ranking of the matched pairs
-//                   and the first N_2 of them
-//   k_pivots        the 2x2 HSVD of every selected pivot (DHSVD2 / ZHSVD2), INFO, NL
+//   k_select        one cluster: the greedy non-colliding selection of the sorted records
+//                   (AW_SRT* + AW_NCP1/2) as the greedy matching, in rounds of mutual best
+//                   proposals; the 2x2 HSVD of every pivot (DHSVD2 / ZHSVD2), INFO, NL; the loop
+//                   test (SL := MIN(SL, NL))
 //   k_rotate        fused transformations: every block loads a column pair of A,
 //                   applies all row rotations (BA), then its column rotation (AB)
 //                   and the diagonal write-back, and rotates the columns of U and Z
+//
+// Filtered steps (jk_filter.cu) build and verify the matching of bounded weights before the column scans and
+// leave those out; small matrices run their whole loop in one launch (jk_small.cu).
 //
 // Matrices are column-major with leading dimension n; complex entries are double2.
 #include <cooperative_groups.h>
@@ -2088,8 +2090,40 @@ int colsort_e(int n)
 // row rotations of all pivots (BA of phase 1); then, for a pivot block and when no
 // pivot failed, the column rotation AB (phase 2) and the diagonal write-back; store;
 // then rotate the columns p, q of U (by V^T / V^H) and of Z (by W), phase 1.
+// Bound by the latency of its loads (two columns of three matrices, read and written once): W rows
+// of a thread are in flight and, with W > 1, U's and Z's columns are fetched to L2 meanwhile (N = 2048 63 to 51 us,
+// the 201 MB 31 us at the copy's rate; N = 4096 254 to 199 us).
 // ---------------------------------------------------------------------------
+// columns x and y by t, W rows of a thread in flight at a time
+template <typename T, int W>
+__device__ __forceinline__ void rotate_columns(T *x, T *y, int n, const typename Tr<T>::R &t)
+{
+  for (int i0 = threadIdx.x; i0 < n; i0 += W * 256) {
+    T a[W], b[W];
+#pragma unroll
+    for (int k = 0; k < W; ++k)
+      if (i0 + 256 * k < n) { a[k] = x[i0 + 256 * k]; b[k] = y[i0 + 256 * k]; }
+#pragma unroll
+    for (int k = 0; k < W; ++k)
+      if (i0 + 256 * k < n) {
+        Tr<T>::apply_ab(t, a[k], b[k]);
+        x[i0 + 256 * k] = a[k];
+        y[i0 + 256 * k] = b[k];
+      }
+  }
+}
+
 template <typename T>
+__device__ __forceinline__ void prefetch_columns(const T *x, const T *y, int n)
+{
+  constexpr int L = 128 / sizeof(T);
+  for (int i = threadIdx.x * L; i < n; i += 256 * L) {
+    asm volatile("prefetch.global.L2 [%0];\n" ::"l"(x + i));
+    asm volatile("prefetch.global.L2 [%0];\n" ::"l"(y + i));
+  }
+}
+
+template <typename T, int W>
 __global__ void __launch_bounds__(256)
 k_rotate(const State *st, T *__restrict__ A, T *__restrict__ U, T *__restrict__ Z, int n, const Piv<T> *__restrict__ piv,
          const RowRot<T> *__restrict__ rr, const int *__restrict__ unp)
@@ -2107,9 +2141,25 @@ k_rotate(const State *st, T *__restrict__ A, T *__restrict__ U, T *__restrict__ 
     if (j + 1 < nu) c1 = unp[j + 1];
   }
   T *A0 = A + (long long)c0 * n, *A1 = (c1 >= 0) ? (A + (long long)c1 * n) : nullptr;
-  for (int i = threadIdx.x; i < n; i += blockDim.x) {
-    col[i] = A0[i];
-    if (A1) col[n + i] = A1[i];
+  for (int i0 = threadIdx.x; i0 < n; i0 += W * 256) {
+    T a[W], c[W];
+#pragma unroll
+    for (int j = 0; j < W; ++j)
+      if (i0 + 256 * j < n) {
+        a[j] = A0[i0 + 256 * j];
+        if (A1) c[j] = A1[i0 + 256 * j];
+      }
+#pragma unroll
+    for (int j = 0; j < W; ++j)
+      if (i0 + 256 * j < n) {
+        col[i0 + 256 * j] = a[j];
+        if (A1) col[n + i0 + 256 * j] = c[j];
+      }
+  }
+  if (W > 1 && k >= 0) {
+    // (U's and Z's columns come while A's are rotated)
+    prefetch_columns<T>(U + (long long)c0 * n, U + (long long)c1 * n, n);
+    prefetch_columns<T>(Z + (long long)c0 * n, Z + (long long)c1 * n, n);
   }
   __syncthreads();
   // phase 1: rows p_m, q_m of every pivot m (BA)
@@ -2153,21 +2203,11 @@ k_rotate(const State *st, T *__restrict__ A, T *__restrict__ U, T *__restrict__ 
   if (info < 0) return;
   if (info & 2) {
     const typename Tr<T>::R t = pv.tu;
-    T *u0 = U + (long long)c0 * n, *u1 = U + (long long)c1 * n;
-    for (int i = threadIdx.x; i < n; i += blockDim.x) {
-      T x = u0[i], y = u1[i];
-      Tr<T>::apply_ab(t, x, y);
-      u0[i] = x; u1[i] = y;
-    }
+    rotate_columns<T, W>(U + (long long)c0 * n, U + (long long)c1 * n, n, t);
   }
   if (info & 4) {
     const typename Tr<T>::R t = pv.tz;
-    T *z0 = Z + (long long)c0 * n, *z1 = Z + (long long)c1 * n;
-    for (int i = threadIdx.x; i < n; i += blockDim.x) {
-      T x = z0[i], y = z1[i];
-      Tr<T>::apply_ab(t, x, y);
-      z0[i] = x; z1[i] = y;
-    }
+    rotate_columns<T, W>(Z + (long long)c0 * n, Z + (long long)c1 * n, n, t);
   }
 }
 
@@ -2204,10 +2244,11 @@ cudaError_t prepare_kernels(int n)
 {
   // dynamic shared memory beyond the default 48 KB: two columns of A per k_rotate
   // block, the ranking and matching state of k_select
-  cudaError_t e = cudaFuncSetAttribute(k_rotate<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, 2 * n * 8);
+  cudaError_t e = cudaFuncSetAttribute(k_rotate<double, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 2 * n * 8);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_rotate<double, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, 2 * n * 8);
   if (e == cudaSuccess)
     e = cudaFuncSetAttribute(k_hyp_pm, cudaFuncAttributeMaxDynamicSharedMemorySize, SCAN_STAGES * (2 * TW) * SCAN_RS * (int)sizeof(double));
-  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_rotate<double2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 2 * n * 16);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_rotate<double2, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 2 * n * 16);
   if (e == cudaSuccess) e = cudaFuncSetAttribute(k_hyp_z_pm, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kZSmem);
   const int ss = (int)SelLayout(n, select_cluster(n)).total;
   for (const void *f : { (const void *)k_select<double, true>, (const void *)k_select<double, false>, (const void *)k_select<double2, true>,
@@ -2417,8 +2458,15 @@ static cudaError_t step_t(Workspace &w, T *A, T *U, T *Z, int n_2, cudaStream_t 
   if (w.learned && (e = launch_learned_weights(w, A, s)) != cudaSuccess) return e;
   e = select_t(w, (const T *)A, n_2, s);
   if (e != cudaSuccess) return e;
-  k_rotate<T><<<(n + 1) / 2, 256, 2 * (size_t)n * sizeof(T), s>>>(w.st, A, U, Z, n, (const Piv<T> *)w.piv,
-                                                                 (const RowRot<T> *)w.rowrot, w.unp);
+  // four rows in flight from N = 512 on (5.8 to 5.6 us; 256: 4.07 to 4.5); complex, where a row takes twice the
+  // registers, one (N = 1024: 14.7 to 18.1)
+  const size_t rs = 2 * (size_t)n * sizeof(T);
+  if constexpr (sizeof(T) == sizeof(double)) {
+    const auto rot = (n >= 512) ? k_rotate<T, 4> : k_rotate<T, 1>;
+    rot<<<(n + 1) / 2, 256, rs, s>>>(w.st, A, U, Z, n, (const Piv<T> *)w.piv, (const RowRot<T> *)w.rowrot, w.unp);
+  }
+  else
+    k_rotate<T, 1><<<(n + 1) / 2, 256, rs, s>>>(w.st, A, U, Z, n, (const Piv<T> *)w.piv, (const RowRot<T> *)w.rowrot, w.unp);
   if (w.learned && (e = cudaGetLastError()) == cudaSuccess) e = launch_offnorm(w, A, s);
   if (e != cudaSuccess) return e;
   return cudaGetLastError();

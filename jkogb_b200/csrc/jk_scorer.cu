@@ -517,13 +517,28 @@ __global__ void __launch_bounds__(256)
 k_offnorm(State *st, const T *__restrict__ A, int n, double *part, int *count)
 {
   if (st->stop || !st->learned) return;
-  __shared__ double red[256];
+  __shared__ double red[256], parts[kOffBlocks];
   __shared__ int last;
-  const long long nn = (long long)n * n;
+  const long long nn = (long long)n * n, step = kOffBlocks * 256LL;
   double acc = 0.0;
-  for (long long k = blockIdx.x * 256LL + threadIdx.x; k < nn; k += (long long)gridDim.x * 256) {
-    const int i = (int)(k % n), j = (int)(k / n);
-    if (i != j) acc = sq_acc(A[k], acc);
+  // element k = i + j n; the walk keeps i and j (a 64-bit division an element took most of the time), several
+  // loads are in flight and the sum stays in k's order (N = 1024 18 to 8.7 us, N = 2048 41 to 21 us)
+  const int di = (int)(step % n), dj = (int)(step / n);
+  long long k = blockIdx.x * 256LL + threadIdx.x;
+  int i = (int)(k % n), j = (int)(k / n);
+  constexpr int W = 8;
+  for (; k < nn; k += W * step) {
+    T x[W];
+#pragma unroll
+    for (int u = 0; u < W; ++u)
+      if (k + u * step < nn) x[u] = A[k + u * step];
+#pragma unroll
+    for (int u = 0; u < W; ++u) {
+      if (k + u * step < nn && i != j) acc = sq_acc(x[u], acc);
+      i += di;
+      j += dj;
+      if (i >= n) { i -= n; ++j; }
+    }
   }
   red[threadIdx.x] = acc;
   __syncthreads();
@@ -537,10 +552,14 @@ k_offnorm(State *st, const T *__restrict__ A, int n, double *part, int *count)
     last = (atomicAdd(count, 1) == (int)gridDim.x - 1);
   }
   __syncthreads();
-  if (!last || threadIdx.x != 0) return;
+  if (!last) return;
   __threadfence();
+  for (int b = threadIdx.x; b < kOffBlocks; b += 256) parts[b] = ((volatile double *)part)[b];
+  __syncthreads();
+  if (threadIdx.x != 0) return;
   double off = 0.0;
-  for (int b = 0; b < (int)gridDim.x; ++b) off += ((volatile double *)part)[b];
+#pragma unroll 8
+  for (int b = 0; b < kOffBlocks; ++b) off += parts[b];
   *count = 0;
   st->off = off;
   const int sl = st->sl, nl = st->nl;
